@@ -191,7 +191,7 @@ merge_numeric_fill_kernel(Operands op, const int32_t *__restrict__ rows, int32_t
     out0 = c_rp[row];
     out_end = c_rp[row + 1];
   }
-  const int32_t m = static_cast<int32_t>(out_end - out0);  // <= 2048 in these classes
+  const int32_t m = static_cast<int32_t>(out_end - out0);  // <= kMergeMaxOps
   const int32_t incl = warp_incl_scan(m);
   const int32_t total = __shfl_sync(kFull, incl, 31);
   const int32_t base = incl - m;

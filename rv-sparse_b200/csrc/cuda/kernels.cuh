@@ -43,7 +43,13 @@ enum RowClass : int {
   kNumClasses
 };
 
-constexpr int kMergeMaxOps = 2048;
+// A thread merges serially, so the longest row of a launch is its time.  On
+// R-MAT matrices (short A rows that select hub B rows) a bound of 2048 kept
+// a few blocks busy for milliseconds after the rest were done: one product at
+// n = 2^16 17.6 ms against 13.7 (512), 13.1 (256) and 13.1 (128, 64), a
+// repeat at 2^15 6.4 ms against 3.1, 2.9, 2.6 and 2.6.  Mesh rows (25
+// products) stay far below any of them.
+constexpr int kMergeMaxOps = 128;
 constexpr int kMergeMaxNnz = 16;
 constexpr int kMergeThreads = 128;
 // The merge classes put one row on one thread; below this many rows the GPU
