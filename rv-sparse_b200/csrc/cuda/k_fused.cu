@@ -44,6 +44,7 @@ compact_large_kernel(const int32_t *__restrict__ big, const int32_t *__restrict_
 // are appended to big[1..] for compact_large_kernel.
 __global__ void __launch_bounds__(kThreads)
 compact_small_kernel(int32_t a_rows, int rows_per_chunk, const int32_t *__restrict__ counts,
+                     const int32_t *__restrict__ cap,
                      const int64_t *__restrict__ off, const int32_t *__restrict__ row_ptr,
                      const int32_t *__restrict__ slab_col,
                      const float *__restrict__ slab_val, int32_t *__restrict__ c_col,
@@ -57,7 +58,11 @@ compact_small_kernel(int32_t a_rows, int rows_per_chunk, const int32_t *__restri
   const int64_t chunks = (int64_t(a_rows) + rows_per_chunk - 1) / rows_per_chunk;
   for (int64_t ch = blockIdx.x; ch < chunks; ch += gridDim.x) {
     const int64_t row = ch * rows_per_chunk + tid;
-    int32_t m = (tid < rows_per_chunk && row < a_rows) ? counts[row] : 0;
+    int32_t m = 0;
+    if (tid < rows_per_chunk && row < a_rows) {
+      m = counts[row];
+      if (m > cap[row]) m = 0;  // not in the slab
+    }
     const bool large = m >= kCompactLarge;
     const unsigned large_mask = __ballot_sync(kFull, large);
     if (large_mask) {
@@ -124,6 +129,15 @@ scatter_list_kernel(const int32_t *__restrict__ list, int32_t n,
   out[class_off[c] + atomicAdd(&class_fill[c], 1)] = list[j];
 }
 
+__global__ void __launch_bounds__(kThreads)
+list_overflow_kernel(const int32_t *__restrict__ rows, int32_t n, FusedOut fo) {
+  const int32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  const int32_t row = row_of(rows, j);
+  fo.counts[row] = -1;
+  fo.ovf_rows[atomicAdd(fo.ovf_count, 1)] = row;
+}
+
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
@@ -149,8 +163,8 @@ values_hash_kernel(const float *__restrict__ v, int64_t n, unsigned long long sa
 
 }  // namespace
 
-void launch_compact(int32_t a_rows, const int32_t *counts, const int64_t *off,
-                    const int32_t *row_ptr, const int32_t *slab_col,
+void launch_compact(int32_t a_rows, const int32_t *counts, const int32_t *cap,
+                    const int64_t *off, const int32_t *row_ptr, const int32_t *slab_col,
                     const float *slab_val, int32_t *c_col, float *c_val,
                     bool with_values, int32_t *big, int num_sms, cudaStream_t s) {
   if (a_rows <= 0) return;
@@ -160,8 +174,8 @@ void launch_compact(int32_t a_rows, const int32_t *counts, const int64_t *off,
   while (rows_per_chunk > 32 && int64_t(a_rows) < int64_t(rows_per_chunk) * blocks)
     rows_per_chunk >>= 1;
   cudaMemsetAsync(big, 0, sizeof(int32_t), s);
-  compact_small_kernel<<<blocks, kThreads, 0, s>>>(a_rows, rows_per_chunk, counts, off,
-                                                   row_ptr, slab_col, slab_val, c_col,
+  compact_small_kernel<<<blocks, kThreads, 0, s>>>(a_rows, rows_per_chunk, counts, cap,
+                                                   off, row_ptr, slab_col, slab_val, c_col,
                                                    c_val, with_values, big);
   compact_large_kernel<<<blocks, kThreads, 0, s>>>(big, counts, off, row_ptr, slab_col,
                                                    slab_val, c_col, c_val, with_values);
@@ -174,6 +188,11 @@ void launch_list_classify(const int32_t *list, int32_t n, const int64_t *ops,
   if (n <= 0) return;
   list_classify_kernel<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(
       list, n, ops, a_rp, counts, b_cols, numeric, cls_out, class_count);
+}
+
+void launch_list_overflow(const int32_t *rows, int32_t n, const FusedOut &fo, cudaStream_t s) {
+  if (n <= 0) return;
+  list_overflow_kernel<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(rows, n, fo);
 }
 
 void launch_scatter_list(const int32_t *list, int32_t n, const uint8_t *cls,

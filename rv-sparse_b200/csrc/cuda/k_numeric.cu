@@ -679,7 +679,7 @@ void launch_numeric_class(int cls, const Operands &op, const int64_t *ops,
                           int32_t dense_slots, int32_t *status, int num_sms,
                           cudaStream_t s, const FusedOut *fo) {
   if (nrows <= 0) return;
-  if ((cls == kB8192 || cls == kDense) && heavy_fits(op.b_cols)) {
+  if (cls >= kB8192 && heavy_fits(op.b_cols)) {  // (B of STRIPE rows is narrow enough)
     launch_heavy_numeric(op, rows, nrows, c_rp, c_col, c_val, fill, status, fo, num_sms, s);
     return;
   }

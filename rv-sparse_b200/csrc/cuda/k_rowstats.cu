@@ -58,7 +58,9 @@ rowstats_kernel(Operands op, int64_t *__restrict__ ops, uint8_t *__restrict__ cl
     } else {
       int64_t s = 0;
       for (int32_t p = p0; p < p1; ++p) s += b_len(op, __ldg(op.a_col + p));
-      c = classify_row(p1 - p0, s, s < op.b_cols ? s : op.b_cols, op.merge_ok);
+      c = with_stripes(
+          classify_row(p1 - p0, s, s < op.b_cols ? s : op.b_cols, op.merge_ok), s,
+          op.stripe_ops);
       ops[i] = s;
       cls[i] = static_cast<uint8_t>(c);
       if (c == kEmpty_) counts[i] = 0;
@@ -90,7 +92,9 @@ rowstats_long_kernel(Operands op, const int32_t *__restrict__ long_rows,
     for (int32_t p = p0 + lane; p < p1; p += 32) s += b_len(op, __ldg(op.a_col + p));
     s = warp_sum64(s);
     if (lane == 0) {
-      const int c = classify_row(p1 - p0, s, s < op.b_cols ? s : op.b_cols, op.merge_ok);
+      const int c = with_stripes(
+          classify_row(p1 - p0, s, s < op.b_cols ? s : op.b_cols, op.merge_ok), s,
+          op.stripe_ops);
       ops[i] = s;
       cls[i] = static_cast<uint8_t>(c);
       if (c == kEmpty_) counts[i] = 0;

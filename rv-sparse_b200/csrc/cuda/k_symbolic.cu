@@ -280,7 +280,7 @@ void launch_symbolic_class(int cls, const Operands &op, const int32_t *rows,
                            int32_t gbitmap_slots, int32_t *status, int num_sms,
                            cudaStream_t s) {
   if (nrows <= 0) return;
-  if ((cls == kB8192 || cls == kDense) && heavy_fits(op.b_cols)) {
+  if (cls >= kB8192 && heavy_fits(op.b_cols)) {  // (B of STRIPE rows is narrow enough)
     launch_heavy_symbolic(op, rows, nrows, counts, num_sms, s);
     return;
   }

@@ -267,6 +267,17 @@ struct rvsp_cuda_plan {
   DevArray<uint16_t> sh_map;
   DevArray<uint32_t> sh_rec;
   TileBuild st;
+  // Stripe rows (k_stripe.cu): B's stripes, and of the rows counted by the
+  // current analysis (sp_ready) their bitmaps, their outputs before each
+  // stripe, their slot by row, and the value items of the numeric STRIPE rows.
+  StripeShape sp;
+  int sp_ready = 0;
+  int64_t sp_cap = 0;
+  DevArray<int32_t> sp_hist, sp_bound, sp_ptr, sp_soff, sp_hslot, sp_cnt;  // cnt: 2, head
+  DevArray<float> sp_share;
+  DevArray<uint8_t> sp_of;
+  DevArray<uint32_t> sp_bits;
+  DevArray<int4> sp_items;
   const int32_t *rmap_col = nullptr;
   int rmap_state = 0;
   int64_t rmap_entries = 0;
@@ -440,6 +451,15 @@ void finish_numeric_bins(rvsp_cuda_plan *p, int32_t a_rows, int32_t b_cols,
                         p->rows_num.p, s);
     ph.launches = 2;
   }
+  if (p->sp_ready && p->num_count[kStripe] > 0) {
+    const bool whole = p->num_whole == kStripe;
+    PhaseScope ph(p, s, RVSP_PHASE_SCAN);
+    launch_stripe_items(p->sp, whole ? nullptr : p->rows_num.p + p->num_off[kStripe],
+                        whole ? a_rows : p->num_count[kStripe], p->ops.p, p->sp_hslot.p,
+                        p->sp_soff.p, p->sp_bound.p, p->sp_share.p, p->sp_items.p, p->sp_cap,
+                        p->sp_cnt.p, s);
+    ph.launches = 1;
+  }
   if (p->num_count[kDense] > 0) {
     p->dense_slots = p->num_count[kDense] < p->num_sms ? p->num_count[kDense] : p->num_sms;
     p->numeric_ws = size_t(p->dense_slots) *
@@ -448,6 +468,44 @@ void finish_numeric_bins(rvsp_cuda_plan *p, int32_t a_rows, int32_t b_cols,
     p->dense_slots = 0;
     p->numeric_ws = 0;
   }
+}
+
+// The exact counts of the nrows STRIPE rows listed at rows (null: every row),
+// with what their columns and values need later.  Sets sp_ready; it stays 0,
+// and nothing was counted, when the row bitmaps (one bit a column) would take
+// more than kStripeBitsMax or a quarter of the free memory.
+constexpr size_t kStripeBitsMax = size_t(2) << 30;
+cudaError_t count_stripe_rows(rvsp_cuda_plan *p, const Operands &op, int32_t b_rows,
+                              const int32_t *rows, int32_t nrows, cudaStream_t s) {
+  const StripeShape &g = p->sp;
+  const size_t n = static_cast<size_t>(nrows), stops = static_cast<size_t>(g.ns_max) + 1;
+  const size_t words = static_cast<size_t>(g.words);
+  const size_t need = n * words * sizeof(uint32_t);
+  if (need > kStripeBitsMax) return cudaSuccess;
+  if (n * words > p->sp_bits.cap) {
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return cudaGetLastError();
+    if (need > free_b / 4) return cudaSuccess;
+  }
+  p->sp_cap = int64_t(nrows) * g.ns_max;
+  if (p->sp_bits.reserve(n * words) != cudaSuccess ||
+      p->sp_soff.reserve(n * stops) != cudaSuccess ||
+      p->sp_items.reserve(size_t(p->sp_cap)) != cudaSuccess ||
+      p->sp_hslot.reserve(size_t(op.a_rows)) != cudaSuccess ||
+      p->sp_hist.reserve(words) != cudaSuccess || p->sp_of.reserve(words) != cudaSuccess ||
+      p->sp_bound.reserve(stops) != cudaSuccess || p->sp_share.reserve(stops) != cudaSuccess ||
+      p->sp_cnt.reserve(3) != cudaSuccess ||
+      p->sp_ptr.reserve(size_t(b_rows) * stops) != cudaSuccess) {
+    cudaGetLastError();  // out of memory: the rows keep the block-per-row kernels
+    return cudaSuccess;
+  }
+  launch_stripe_table(g, b_rows, op.b_rp, op.b_col, p->sp_hist.p, p->sp_bound.p, p->sp_share.p,
+                      p->sp_of.p, p->sp_ptr.p, p->num_sms, s);
+  cudaMemsetAsync(p->sp_hslot.p, 0xff, size_t(op.a_rows) * sizeof(int32_t), s);
+  launch_stripe_count(g, op, rows, nrows, p->sp_bound.p, p->counts.p, p->sp_hslot.p,
+                      p->sp_bits.p, p->sp_soff.p, p->sp_cnt.p + 2, p->num_sms, s);
+  p->sp_ready = 1;
+  return cudaGetLastError();
 }
 
 // Reserves (and zeroes when grown) the global bitmaps dense symbolic rows use
@@ -559,6 +617,12 @@ void rvsp_cuda_plan_destroy(rvsp_cuda_plan_t p) {
   p->sh_pat_off.release();
   p->sh_map.release();
   p->sh_rec.release();
+  for (auto *a : {&p->sp_hist, &p->sp_bound, &p->sp_ptr, &p->sp_soff, &p->sp_hslot, &p->sp_cnt})
+    a->release();
+  p->sp_share.release();
+  p->sp_of.release();
+  p->sp_bits.release();
+  p->sp_items.release();
   p->ops.release();
   p->cls.release();
   p->cls_spec.release();
@@ -641,8 +705,9 @@ rvsp_status_t symbolic_impl(rvsp_cuda_plan_t p, cudaStream_t s, int32_t a_rows,
                             const int32_t *b_col_idx, int32_t *c_row_ptr,
                             int64_t *c_nnz_out, const PreCheck *chk);
 cudaError_t symbolic_rest(rvsp_cuda_plan *p, cudaStream_t s, const Operands &op,
-                          int32_t a_rows, int32_t b_cols, const int32_t *a_row_ptr,
-                          int32_t *c_row_ptr, const int32_t *sym_off, bool merge_done);
+                          int32_t a_rows, int32_t b_rows, int32_t b_cols,
+                          const int32_t *a_row_ptr, int32_t *c_row_ptr,
+                          const int32_t *sym_off, bool merge_done);
 
 }  // namespace
 
@@ -694,6 +759,8 @@ rvsp_status_t symbolic_impl(rvsp_cuda_plan_t p, cudaStream_t s, int32_t a_rows,
   p->analysed = 0;
   p->rmap_state = 0;
   p->rmap_col = nullptr;
+  p->sp = stripe_shape(b_rows, b_cols);
+  p->sp_ready = 0;
   const size_t n = static_cast<size_t>(a_rows);
 
   cudaError_t e = p->ops.reserve(n);
@@ -713,6 +780,7 @@ rvsp_status_t symbolic_impl(rvsp_cuda_plan_t p, cudaStream_t s, int32_t a_rows,
   Operands op{a_rows, b_cols, a_row_ptr, a_col_idx, nullptr,
               b_row_ptr, b_col_idx, nullptr,
               merge_allowed(p->merge_policy, a_rows)};
+  op.stripe_ops = p->sp.min_ops;
   if (chk) {
     // Checks of A (and B) run first; the row statistics after them are
     // bounded (they read nothing outside A's entries and B's row pointers),
@@ -830,7 +898,7 @@ rvsp_status_t symbolic_impl(rvsp_cuda_plan_t p, cudaStream_t s, int32_t a_rows,
     if (c != kEmpty_ && !is_merge_class(c) && p->sym_count[c] > 0) rest = true;
   }
   if (rest) {
-    e = symbolic_rest(p, s, op, a_rows, b_cols, a_row_ptr, c_row_ptr, sym_off, spec);
+    e = symbolic_rest(p, s, op, a_rows, b_rows, b_cols, a_row_ptr, c_row_ptr, sym_off, spec);
     if (e != cudaSuccess) return map_cuda(e);
   } else {
     std::swap(p->cls, p->cls_spec);  // the early scan's numeric classes
@@ -860,8 +928,9 @@ rvsp_status_t symbolic_impl(rvsp_cuda_plan_t p, cudaStream_t s, int32_t a_rows,
 // (all rows when merge_done is false), then the scan again, and the host
 // copy of the counters and the total (one more round trip).
 cudaError_t symbolic_rest(rvsp_cuda_plan *p, cudaStream_t s, const Operands &op,
-                          int32_t a_rows, int32_t b_cols, const int32_t *a_row_ptr,
-                          int32_t *c_row_ptr, const int32_t *sym_off, bool merge_done) {
+                          int32_t a_rows, int32_t b_rows, int32_t b_cols,
+                          const int32_t *a_row_ptr, int32_t *c_row_ptr,
+                          const int32_t *sym_off, bool merge_done) {
   int32_t *misc = p->misc.p;
   cudaError_t e = cudaSuccess;
   // Global bitmaps for dense symbolic rows when B is too wide for shared memory.
@@ -883,6 +952,10 @@ cudaError_t symbolic_rest(rvsp_cuda_plan *p, cudaStream_t s, const Operands &op,
     // retry lists live in long_rows (free once the row statistics are done),
     // W1024's from 0, W2048's after it.
     auto launch_class = [&](int c, const int32_t *rows, int32_t nrows) {
+      if (c == kStripe) {
+        if (e == cudaSuccess) e = count_stripe_rows(p, op, b_rows, rows, nrows, s);
+        if (p->sp_ready) return 4;
+      }
       if (symbolic_optimistic_class(c)) {
         const int32_t base = c == kW1024 ? 0 : p->sym_count[kW1024];
         launch_symbolic_optimistic(c, op, rows, nrows, p->counts.p, p->long_rows.p + base,
@@ -910,6 +983,7 @@ cudaError_t symbolic_rest(rvsp_cuda_plan *p, cudaStream_t s, const Operands &op,
       }
     }
   }
+  if (e != cudaSuccess) return e;
   if (merge_done)  // the first scan counted numeric classes already
     cudaMemsetAsync(misc + kNumCount, 0, kNumClasses * sizeof(int32_t), s);
   {
@@ -922,7 +996,7 @@ cudaError_t symbolic_rest(rvsp_cuda_plan *p, cudaStream_t s, const Operands &op,
     launch_scan_and_class(a_rows, p->counts.p, p->ops.p, a_row_ptr, c_row_ptr,
                           p->partials.p,
                           p->total.p, p->cls.p, misc + kNumCount, op.merge_ok, s,
-                          CheckGuard(), skip);
+                          CheckGuard(), skip, p->sp_ready ? p->sp_hslot.p : nullptr);
     ph.launches = skip ? 4 : 3;
   }
   cudaMemcpyAsync(p->h_misc + kNumCount, misc + kNumCount,
@@ -985,9 +1059,12 @@ rvsp_status_t rvsp_cuda_learned_symbolic(
   if (e == cudaSuccess) e = p->partials.reserve(scan_partials_bytes(a_rows) / sizeof(int64_t));
   if (e != cudaSuccess) return map_cuda(e);
 
-  const Operands op{a_rows, b_cols, a_row_ptr, a_col_idx, a_values,
-                    b_row_ptr, b_col_idx, b_values,
-                    merge_allowed(p->merge_policy, a_rows)};
+  Operands op{a_rows, b_cols, a_row_ptr, a_col_idx, a_values,
+              b_row_ptr, b_col_idx, b_values,
+              merge_allowed(p->merge_policy, a_rows)};
+  p->sp = stripe_shape(b_rows, b_cols);
+  p->sp_ready = 0;
+  op.stripe_ops = p->sp.min_ops;
   int32_t *misc = p->misc.p;
   cudaMemsetAsync(misc, 0, kMiscWords * sizeof(int32_t), s);
   // 1. Predict every row's class and capacity; slab offsets = scan of capacities.
@@ -1045,6 +1122,17 @@ rvsp_status_t rvsp_cuda_learned_symbolic(
     for (int c = kEmpty_ + 1; c < kNumClasses; ++c) {
       if (p->sym_count[c] <= 0) continue;
       const bool all = c == whole;
+      if (c == kStripe) {
+        // counted here, written at C by the compute (no slab slot)
+        const int32_t *rows = all ? nullptr : p->rows_sym.p + pred_off[c];
+        e = count_stripe_rows(p, op, b_rows, rows, all ? a_rows : p->sym_count[c], s);
+        if (e != cudaSuccess) return map_cuda(e);
+        // no room for their bitmaps: the plain two-pass path takes them
+        if (!p->sp_ready)
+          launch_list_overflow(rows, all ? a_rows : p->sym_count[c], fo, s);
+        ph.launches += p->sp_ready ? 4 : 1;
+        continue;
+      }
       launch_numeric_class(c, op, p->ops.p, all ? nullptr : p->rows_sym.p + pred_off[c],
                            all ? a_rows : p->sym_count[c], nullptr, p->slab_col.p,
                            p->slab_val.p, true, facc, fbits, fslots, misc + kStatus,
@@ -1058,7 +1146,8 @@ rvsp_status_t rvsp_cuda_learned_symbolic(
     PhaseScope ph(p, s, RVSP_PHASE_SCAN);
     launch_scan_and_class(a_rows, p->counts.p, p->ops.p, a_row_ptr, c_row_ptr,
                           p->partials.p, p->total.p, p->cls.p, misc + kNumCount,
-                            op.merge_ok, s);
+                          op.merge_ok, s, CheckGuard(), nullptr,
+                          p->sp_ready ? p->sp_hslot.p : nullptr, true);
     ph.launches = 3;
   }
   values_fingerprint_launch(p, a_values, a_nnz, b_values, b_nnz, s);
@@ -1113,7 +1202,8 @@ rvsp_status_t rvsp_cuda_learned_symbolic(
       cudaMemsetAsync(misc + kNumCount, 0, kNumClasses * sizeof(int32_t), s);
       launch_scan_and_class(a_rows, p->counts.p, p->ops.p, a_row_ptr, c_row_ptr,
                             p->partials.p, p->total.p, p->cls.p, misc + kNumCount,
-                            op.merge_ok, s);
+                            op.merge_ok, s, CheckGuard(), nullptr,
+                            p->sp_ready ? p->sp_hslot.p : nullptr, true);
       // The overflow rows by numeric class, for the first compute.
       cudaMemsetAsync(misc + kSymCount, 0, 3 * kNumClasses * sizeof(int32_t), s);
       launch_list_classify(p->ovf_rows.p, p->n_ovf, p->ops.p, a_row_ptr, p->counts.p,
@@ -1753,6 +1843,23 @@ int launch_shift_numeric(rvsp_cuda_plan *p, Lanes &ln, const Operands &op,
   return launches;
 }
 
+// The numeric STRIPE rows: columns first when they are to be filled, then
+// the values; returns the launches.
+int launch_stripe_rows(rvsp_cuda_plan *p, const Operands &op, const int32_t *c_rp,
+                       int32_t *c_col, float *c_val, bool fill, cudaStream_t s) {
+  const int32_t nrows = p->num_count[kStripe];
+  if (!p->sp_ready || nrows <= 0) return 0;
+  const int32_t *rows = p->num_whole == kStripe ? nullptr : p->rows_num.p + p->num_off[kStripe];
+  int32_t *status = p->misc.p + kStatus;
+  if (fill)
+    launch_stripe_columns(p->sp, rows, nrows, p->sp_hslot.p, p->sp_bits.p, c_rp, c_col, status,
+                          s);
+  launch_stripe_values(p->sp, op, nrows, p->sp_items.p, p->sp_cap, p->sp_cnt.p,
+                       p->sp_cnt.p + 2, p->sp_bound.p, p->sp_ptr.p, c_rp, c_col, c_val, status,
+                       p->num_sms, s);
+  return fill ? 2 : 1;
+}
+
 cudaError_t build_reuse_map(rvsp_cuda_plan *p, cudaStream_t s, const Operands &op,
                             const int32_t *c_rp, const int32_t *c_col) {
   p->rmap_state = -1;
@@ -1918,10 +2025,10 @@ rvsp_status_t rvsp_cuda_numeric(rvsp_cuda_plan_t p, void *stream,
     // its values: copy them; the overflowed rows take the plain fill.
     {
       PhaseScope ph(p, s, RVSP_PHASE_COMPACT);
-      launch_compact(p->a_rows, p->counts.p, p->slab_off.p, c_row_ptr, p->slab_col.p,
-                     p->slab_val.p, c_col_idx, c_values, true, p->big_rows.p,
-                     p->num_sms, s);
-      ph.launches = 2;
+      launch_compact(p->a_rows, p->counts.p, p->cap.p, p->slab_off.p, c_row_ptr,
+                     p->slab_col.p, p->slab_val.p, c_col_idx, c_values, true,
+                     p->big_rows.p, p->num_sms, s);
+      ph.launches = 2 + launch_stripe_rows(p, op, c_row_ptr, c_col_idx, c_values, true, s);
       for (int c = kEmpty_ + 1; c < kNumClasses && p->n_ovf > 0; ++c) {
         if (p->ovf_num_count[c] <= 0) continue;
         launch_numeric_class(c, op, p->ops.p, p->ovf_sorted.p + p->ovf_num_off[c],
@@ -2021,6 +2128,8 @@ rvsp_status_t rvsp_cuda_numeric(rvsp_cuda_plan_t p, void *stream,
       } else if (use_map && map_class(c))
         launch_map_numeric(c, op, p->ops.p, rows, nrows, c_row_ptr, c_values,
                            p->rmap_off.p, p->rmap.p, p->misc.p + kStatus, ln.next());
+      else if (c == kStripe && p->sp_ready)
+        launch_stripe_rows(p, op, c_row_ptr, c_col_idx, c_values, fill != 0, ln.next());
       else
         launch_numeric_class(c, op, p->ops.p, rows, nrows, c_row_ptr, c_col_idx, c_values,
                              fill != 0, dense_acc, dense_bits, p->dense_slots,
@@ -2144,9 +2253,10 @@ rvsp_status_t rvsp_cuda_plan_class_counts(rvsp_cuda_plan_t p, int32_t *sym_out,
                                           int32_t *num_out, int32_t n) {
   if (!p) return RVSP_ERROR_NULL_POINTER;
   for (int i = 0; i < n; ++i) {
-    const bool in = i < kNumClasses;
-    if (sym_out) sym_out[i] = in ? p->sym_count[i] : 0;
-    if (num_out) num_out[i] = in ? p->num_count[i] : 0;
+    const bool in = i < kStripe;  // (the stripe rows among the dense ones)
+    const bool dense = i == kDense;
+    if (sym_out) sym_out[i] = in ? p->sym_count[i] + (dense ? p->sym_count[kStripe] : 0) : 0;
+    if (num_out) num_out[i] = in ? p->num_count[i] + (dense ? p->num_count[kStripe] : 0) : 0;
   }
   return RVSP_SUCCESS;
 }
