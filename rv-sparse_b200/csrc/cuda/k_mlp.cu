@@ -171,8 +171,8 @@ predict_kernel(Operands op, float b_mean_len, const float *__restrict__ params,
 //   otherwise                            capacity = min(ub, ceil(scale *
 //     (2^y0 - 1)) + kCapPad) with ub = min(ops, b_cols); warp hash with
 //     T >= 2 capacity slots up to 2048, the 8192-slot block hash up to 4096,
-//     else DENSE with capacity ub (never overflows); of the last two, rows of
-//     at least op.stripe_ops products are STRIPE with no slab slot.
+//     else DENSE with capacity ub (never overflows); of the last two, rows
+//     are STRIPE8 or STRIPE with no slab slot when op.stripes.
 // A row whose nnz exceeds its capacity is caught by the fused kernel and
 // redone by the plain two-pass path.
 constexpr int kCapPad = 16;
@@ -207,8 +207,8 @@ learned_plan_kernel(Operands op, float b_mean_len, const float *__restrict__ par
       c = classify_row(nnz, ops, cap, false);
       if (c == kDense) cap = ub;
       // counted exactly by the stripe pass, which needs no slab slot
-      c = with_stripes(c, ops, op.stripe_ops);
-      if (c == kStripe) cap = 0;
+      c = with_stripes(c, op.stripes);
+      if (c >= kStripe8) cap = 0;
     }
     ops_out[row] = ops;
     cls_out[row] = static_cast<uint8_t>(c);

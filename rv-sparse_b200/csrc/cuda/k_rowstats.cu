@@ -59,8 +59,8 @@ rowstats_kernel(Operands op, int64_t *__restrict__ ops, uint8_t *__restrict__ cl
       int64_t s = 0;
       for (int32_t p = p0; p < p1; ++p) s += b_len(op, __ldg(op.a_col + p));
       c = with_stripes(
-          classify_row(p1 - p0, s, s < op.b_cols ? s : op.b_cols, op.merge_ok), s,
-          op.stripe_ops);
+          classify_row(p1 - p0, s, s < op.b_cols ? s : op.b_cols, op.merge_ok),
+          op.stripes);
       ops[i] = s;
       cls[i] = static_cast<uint8_t>(c);
       if (c == kEmpty_) counts[i] = 0;
@@ -93,8 +93,8 @@ rowstats_long_kernel(Operands op, const int32_t *__restrict__ long_rows,
     s = warp_sum64(s);
     if (lane == 0) {
       const int c = with_stripes(
-          classify_row(p1 - p0, s, s < op.b_cols ? s : op.b_cols, op.merge_ok), s,
-          op.stripe_ops);
+          classify_row(p1 - p0, s, s < op.b_cols ? s : op.b_cols, op.merge_ok),
+          op.stripes);
       ops[i] = s;
       cls[i] = static_cast<uint8_t>(c);
       if (c == kEmpty_) counts[i] = 0;

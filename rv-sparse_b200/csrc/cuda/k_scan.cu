@@ -124,7 +124,8 @@ tile_apply_kernel(int32_t n, const int32_t *__restrict__ counts,
       m = counts[i];
       c = (skip && skip[i] >= 0) ? kEmpty_
                                  : classify_row(a_rp[i + 1] - a_rp[i], ops[i], m, merge_ok);
-      if (hslot && (hslot_all || c >= kB8192) && hslot[i] >= 0) c = kStripe;
+      if (hslot && (hslot_all || c >= kB8192) && hslot[i] >= 0)
+        c = c == kDense ? kStripe : kStripe8;
       cls[i] = static_cast<uint8_t>(c);
     }
     s_items[skew(idx)] = m;

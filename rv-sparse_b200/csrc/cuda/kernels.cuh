@@ -27,9 +27,9 @@ const float *mlp_device_params(const rvsp_mlp *m);
 //   W<T>    one warp, shared-memory hash table of T slots (bound <= T/2)
 //   B8192   one 256-thread block, hash table of 8192 slots (bound <= 4096)
 //   DENSE   one 512-thread block, dense accumulator over all of B's columns
-//   STRIPE  B8192 and DENSE rows of enough products (StripeShape::min_ops):
-//           a warp per run of column stripes (k_stripe.cu); reported with the
-//           DENSE rows
+//   STRIPE8, STRIPE  the B8192 and DENSE rows of a product whose B suits
+//           column stripes: a warp per run of stripes (k_stripe.cu); reported
+//           as the classes they come from
 enum RowClass : int {
   kEmpty_ = 0,
   kM4,
@@ -43,6 +43,7 @@ enum RowClass : int {
   kW2048,
   kB8192,
   kDense,
+  kStripe8,
   kStripe,
   kNumClasses
 };
@@ -105,13 +106,12 @@ struct Operands {
   // check has not finished yet (rvsp_cuda_symbolic_checked).
   int32_t a_nnz = -1;
   int32_t b_rows = -1;
-  // Products a B8192 or DENSE row needs for the STRIPE class (0: no stripes).
-  int64_t stripe_ops = 0;
+  // B8192 and DENSE rows take the STRIPE classes.
+  bool stripes = false;
 };
 
-// The class of a row whose products decide between the heavy classes.
-__host__ __device__ inline int with_stripes(int cls, int64_t ops, int64_t stripe_ops) {
-  return stripe_ops > 0 && cls >= kB8192 && ops >= stripe_ops ? kStripe : cls;
+__host__ __device__ inline int with_stripes(int cls, bool stripes) {
+  return !stripes || cls < kB8192 ? cls : cls == kB8192 ? kStripe8 : kStripe;
 }
 
 // The device-side verdict of CSR checks queued earlier on the same stream:
@@ -171,9 +171,9 @@ void launch_scatter_rows(int32_t n, const uint8_t *cls, const int32_t *class_off
 // row_ptr = exclusive scan of counts (n + 1 entries), *total = sum (int64).
 // Also classes every row for the numeric pass (cls, class_count); rows with
 // skip[row] >= 0 (the shift-class members) are classed empty.  With hslot,
-// rows that the stripe count took (hslot[row] >= 0) are classed STRIPE: those
-// of more than 1024 outputs, or all of them (hslot_all).  With a guard that
-// failed, nothing is written but the tile partials.
+// rows that the stripe count took (hslot[row] >= 0) are classed STRIPE8 or
+// STRIPE: those of more than 1024 outputs, or all of them (hslot_all).  With a
+// guard that failed, nothing is written but the tile partials.
 size_t scan_partials_bytes(int32_t n);
 void launch_scan_and_class(int32_t n, const int32_t *counts, const int64_t *ops,
                            const int32_t *a_rp, int32_t *row_ptr,
@@ -256,27 +256,31 @@ void launch_heavy_numeric(const Operands &op, const int32_t *rows, int32_t nrows
 
 // ---- k_stripe.cu -------------------------------------------------------------
 // STRIPE rows, for B of 1025 .. kStripeMaxCols columns whose table of stripe
-// starts stays within 256 MB (min_ops 0 otherwise).
+// starts stays within 256 MB (else off: the block-per-row kernels).
 constexpr int32_t kStripeMaxCols = 1 << 17;
-constexpr int kMaxStripes = 64;
+constexpr int kMaxStripes = 96;
 struct StripeShape {
-  int32_t words = 0;    // 32-column words of B's columns
-  int32_t ns_max = 0;   // stripes at most
-  int64_t min_ops = 0;  // products a heavy row needs to be a STRIPE row
+  bool on = false;
+  int32_t words = 0;   // 32-column words of B's columns
+  int32_t ns_max = 0;  // stripes at most
 };
+__host__ __device__ inline int32_t stripe_groups(int32_t words) { return (words + 31) >> 5; }
 StripeShape stripe_shape(int32_t b_rows, int32_t b_cols);
-// Stripes of B: hist and of_word of words entries, bound of ns_max + 1, share
-// of ns_max, ptr of b_rows * (ns_max + 1).
+// Stripes of B: hist of words entries, bound of ns_max + 1, share of ns_max,
+// ptr of b_rows * (ns_max + 1).
 void launch_stripe_table(const StripeShape &g, int32_t b_rows, const int32_t *b_rp,
                          const int32_t *b_col, int32_t *hist, int32_t *bound, float *share,
-                         uint8_t *of_word, int32_t *ptr, int num_sms, cudaStream_t s);
+                         int32_t *ptr, int num_sms, cudaStream_t s);
 // counts[row] of the listed rows; hslot[row] = the row's place in the list,
-// which indexes its bitmap (words) in bits and its outputs before each stripe
-// (ns_max + 1) in soff.  head: one scratch word.
+// which indexes its bitmap (words) in bits, its outputs before each 32 words of
+// it (stripe_groups) in gpre and before each stripe (ns_max + 1) in soff.
+// Scratch: stripe_tasks(nrows) tasks, three words cnt, nrows words done.
+size_t stripe_tasks(int32_t nrows);
 void launch_stripe_count(const StripeShape &g, const Operands &op, const int32_t *rows,
-                         int32_t nrows, const int32_t *bound, int32_t *counts,
-                         int32_t *hslot, uint32_t *bits, int32_t *soff, int32_t *head,
-                         int num_sms, cudaStream_t s);
+                         int32_t nrows, const int64_t *ops, const int32_t *bound, int2 *tasks,
+                         int32_t *cnt, int32_t *done, int32_t *counts, int32_t *hslot,
+                         uint32_t *bits, int32_t *gpre, int32_t *soff, int num_sms,
+                         cudaStream_t s);
 // The work items of counted rows: items of cap = nrows * ns_max, cnt of two.
 void launch_stripe_items(const StripeShape &g, const int32_t *rows, int32_t nrows,
                          const int64_t *ops, const int32_t *hslot, const int32_t *soff,
@@ -284,14 +288,18 @@ void launch_stripe_items(const StripeShape &g, const int32_t *rows, int32_t nrow
                          int32_t *cnt, cudaStream_t s);
 // Fill: C's columns of counted rows, from their bitmaps.
 void launch_stripe_columns(const StripeShape &g, const int32_t *rows, int32_t nrows,
-                           const int32_t *hslot, const uint32_t *bits, const int32_t *c_rp,
-                           int32_t *c_col, int32_t *status, cudaStream_t s);
-// C's values of the items' rows (columns in C).  nrows: the rows they cover.
+                           const int32_t *hslot, const uint32_t *bits, const int32_t *gpre,
+                           const int32_t *soff, const int32_t *c_rp, int32_t *c_col,
+                           int32_t *status, cudaStream_t s);
+// C's values of the items' rows (columns in C; verify: not written by this
+// plan just now, so they are compared with the bitmaps).  nrows: the rows the
+// items cover.
 void launch_stripe_values(const StripeShape &g, const Operands &op, int32_t nrows,
                           const int4 *items, int64_t cap, const int32_t *cnt, int32_t *head,
-                          const int32_t *bound, const int32_t *ptr, const int32_t *c_rp,
-                          const int32_t *c_col, float *c_val, int32_t *status, int num_sms,
-                          cudaStream_t s);
+                          const int32_t *bound, const float *share, const int32_t *ptr,
+                          const int32_t *hslot, const uint32_t *bits, const int32_t *gpre,
+                          const int32_t *c_rp, const int32_t *c_col, float *c_val, bool verify, int32_t *status,
+                          int num_sms, cudaStream_t s);
 
 // ---- k_reuse.cu ------------------------------------------------------------
 // Reuse map of the W<T> classes: per product, its position in C's row.

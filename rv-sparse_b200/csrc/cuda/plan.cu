@@ -273,9 +273,9 @@ struct rvsp_cuda_plan {
   StripeShape sp;
   int sp_ready = 0;
   int64_t sp_cap = 0;
-  DevArray<int32_t> sp_hist, sp_bound, sp_ptr, sp_soff, sp_hslot, sp_cnt;  // cnt: 2, head
+  DevArray<int32_t> sp_hist, sp_bound, sp_ptr, sp_gpre, sp_soff, sp_hslot, sp_done;
+  DevArray<int32_t> sp_cnt;  // items from the front, from the back, queue head
   DevArray<float> sp_share;
-  DevArray<uint8_t> sp_of;
   DevArray<uint32_t> sp_bits;
   DevArray<int4> sp_items;
   const int32_t *rmap_col = nullptr;
@@ -431,6 +431,16 @@ int whole_matrix_class(const int32_t *count, int32_t a_rows) {
   return (count[kEmpty_] == 0 || merge) ? found : -1;
 }
 
+// The STRIPE8 and STRIPE rows of one census: their lists lie one after the
+// other; one that holds every row needs none.
+struct RowList {
+  const int32_t *rows;
+  int32_t n;
+};
+RowList stripe_rows(const int32_t *count, const int32_t *off, int whole, const int32_t *list) {
+  return {whole >= kStripe8 ? nullptr : list + off[kStripe8], count[kStripe8] + count[kStripe]};
+}
+
 // After the final scan (class counts of the numeric pass in h_misc): host
 // offsets, the row lists (unless one class holds every row) and the dense
 // workspace the numeric pass will need.
@@ -451,13 +461,11 @@ void finish_numeric_bins(rvsp_cuda_plan *p, int32_t a_rows, int32_t b_cols,
                         p->rows_num.p, s);
     ph.launches = 2;
   }
-  if (p->sp_ready && p->num_count[kStripe] > 0) {
-    const bool whole = p->num_whole == kStripe;
+  const RowList sr = stripe_rows(p->num_count, p->num_off, p->num_whole, p->rows_num.p);
+  if (p->sp_ready && sr.n > 0) {
     PhaseScope ph(p, s, RVSP_PHASE_SCAN);
-    launch_stripe_items(p->sp, whole ? nullptr : p->rows_num.p + p->num_off[kStripe],
-                        whole ? a_rows : p->num_count[kStripe], p->ops.p, p->sp_hslot.p,
-                        p->sp_soff.p, p->sp_bound.p, p->sp_share.p, p->sp_items.p, p->sp_cap,
-                        p->sp_cnt.p, s);
+    launch_stripe_items(p->sp, sr.rows, sr.n, p->ops.p, p->sp_hslot.p, p->sp_soff.p,
+                        p->sp_bound.p, p->sp_share.p, p->sp_items.p, p->sp_cap, p->sp_cnt.p, s);
     ph.launches = 1;
   }
   if (p->num_count[kDense] > 0) {
@@ -489,10 +497,12 @@ cudaError_t count_stripe_rows(rvsp_cuda_plan *p, const Operands &op, int32_t b_r
   }
   p->sp_cap = int64_t(nrows) * g.ns_max;
   if (p->sp_bits.reserve(n * words) != cudaSuccess ||
+      p->sp_gpre.reserve(n * size_t(stripe_groups(g.words))) != cudaSuccess ||
       p->sp_soff.reserve(n * stops) != cudaSuccess ||
-      p->sp_items.reserve(size_t(p->sp_cap)) != cudaSuccess ||
+      p->sp_items.reserve(std::max(size_t(p->sp_cap), stripe_tasks(nrows))) != cudaSuccess ||
+      p->sp_done.reserve(n) != cudaSuccess ||
       p->sp_hslot.reserve(size_t(op.a_rows)) != cudaSuccess ||
-      p->sp_hist.reserve(words) != cudaSuccess || p->sp_of.reserve(words) != cudaSuccess ||
+      p->sp_hist.reserve(words) != cudaSuccess ||
       p->sp_bound.reserve(stops) != cudaSuccess || p->sp_share.reserve(stops) != cudaSuccess ||
       p->sp_cnt.reserve(3) != cudaSuccess ||
       p->sp_ptr.reserve(size_t(b_rows) * stops) != cudaSuccess) {
@@ -500,10 +510,13 @@ cudaError_t count_stripe_rows(rvsp_cuda_plan *p, const Operands &op, int32_t b_r
     return cudaSuccess;
   }
   launch_stripe_table(g, b_rows, op.b_rp, op.b_col, p->sp_hist.p, p->sp_bound.p, p->sp_share.p,
-                      p->sp_of.p, p->sp_ptr.p, p->num_sms, s);
+                      p->sp_ptr.p, p->num_sms, s);
   cudaMemsetAsync(p->sp_hslot.p, 0xff, size_t(op.a_rows) * sizeof(int32_t), s);
-  launch_stripe_count(g, op, rows, nrows, p->sp_bound.p, p->counts.p, p->sp_hslot.p,
-                      p->sp_bits.p, p->sp_soff.p, p->sp_cnt.p + 2, p->num_sms, s);
+  // (the items' memory is free until the numeric bins are known)
+  launch_stripe_count(g, op, rows, nrows, p->ops.p, p->sp_bound.p,
+                      reinterpret_cast<int2 *>(p->sp_items.p), p->sp_cnt.p, p->sp_done.p,
+                      p->counts.p, p->sp_hslot.p, p->sp_bits.p, p->sp_gpre.p, p->sp_soff.p,
+                      p->num_sms, s);
   p->sp_ready = 1;
   return cudaGetLastError();
 }
@@ -617,10 +630,10 @@ void rvsp_cuda_plan_destroy(rvsp_cuda_plan_t p) {
   p->sh_pat_off.release();
   p->sh_map.release();
   p->sh_rec.release();
-  for (auto *a : {&p->sp_hist, &p->sp_bound, &p->sp_ptr, &p->sp_soff, &p->sp_hslot, &p->sp_cnt})
+  for (auto *a : {&p->sp_hist, &p->sp_bound, &p->sp_ptr, &p->sp_gpre, &p->sp_soff, &p->sp_hslot,
+                  &p->sp_done, &p->sp_cnt})
     a->release();
   p->sp_share.release();
-  p->sp_of.release();
   p->sp_bits.release();
   p->sp_items.release();
   p->ops.release();
@@ -780,7 +793,7 @@ rvsp_status_t symbolic_impl(rvsp_cuda_plan_t p, cudaStream_t s, int32_t a_rows,
   Operands op{a_rows, b_cols, a_row_ptr, a_col_idx, nullptr,
               b_row_ptr, b_col_idx, nullptr,
               merge_allowed(p->merge_policy, a_rows)};
-  op.stripe_ops = p->sp.min_ops;
+  op.stripes = p->sp.on;
   if (chk) {
     // Checks of A (and B) run first; the row statistics after them are
     // bounded (they read nothing outside A's entries and B's row pointers),
@@ -952,10 +965,6 @@ cudaError_t symbolic_rest(rvsp_cuda_plan *p, cudaStream_t s, const Operands &op,
     // retry lists live in long_rows (free once the row statistics are done),
     // W1024's from 0, W2048's after it.
     auto launch_class = [&](int c, const int32_t *rows, int32_t nrows) {
-      if (c == kStripe) {
-        if (e == cudaSuccess) e = count_stripe_rows(p, op, b_rows, rows, nrows, s);
-        if (p->sp_ready) return 4;
-      }
       if (symbolic_optimistic_class(c)) {
         const int32_t base = c == kW1024 ? 0 : p->sym_count[kW1024];
         launch_symbolic_optimistic(c, op, rows, nrows, p->counts.p, p->long_rows.p + base,
@@ -970,20 +979,28 @@ cudaError_t symbolic_rest(rvsp_cuda_plan *p, cudaStream_t s, const Operands &op,
     // whole >= 0 is never a merge class here when merge_done (a class
     // outside them is non-empty).
     const int whole = p->shift_active ? -1 : whole_matrix_class(p->sym_count, a_rows);
-    if (whole >= 0) {
-      ph.launches = launch_class(whole, nullptr, a_rows);
-    } else {
+    if (whole < 0) {
       launch_class_offsets(misc + kSymCount, misc + kSymOff, s);
       launch_scatter_rows(a_rows, p->cls.p, misc + kSymOff, misc + kSymFill,
                           p->rows_sym.p, s);
       ph.launches = 2;
-      for (int c = kEmpty_ + 1; c < kNumClasses; ++c) {
+    }
+    const RowList sr = stripe_rows(p->sym_count, sym_off, whole, p->rows_sym.p);
+    if (sr.n > 0) {
+      e = count_stripe_rows(p, op, b_rows, sr.rows, sr.n, s);
+      if (e != cudaSuccess) return e;
+      ph.launches += 4;
+    }
+    const int classes = p->sp_ready ? kStripe8 : kNumClasses;
+    if (whole >= 0) {
+      if (whole < classes) ph.launches += launch_class(whole, nullptr, a_rows);
+    } else {
+      for (int c = kEmpty_ + 1; c < classes; ++c) {
         if (p->sym_count[c] <= 0 || (merge_done && is_merge_class(c))) continue;
         ph.launches += launch_class(c, p->rows_sym.p + sym_off[c], p->sym_count[c]);
       }
     }
   }
-  if (e != cudaSuccess) return e;
   if (merge_done)  // the first scan counted numeric classes already
     cudaMemsetAsync(misc + kNumCount, 0, kNumClasses * sizeof(int32_t), s);
   {
@@ -1064,7 +1081,7 @@ rvsp_status_t rvsp_cuda_learned_symbolic(
               merge_allowed(p->merge_policy, a_rows)};
   p->sp = stripe_shape(b_rows, b_cols);
   p->sp_ready = 0;
-  op.stripe_ops = p->sp.min_ops;
+  op.stripes = p->sp.on;
   int32_t *misc = p->misc.p;
   cudaMemsetAsync(misc, 0, kMiscWords * sizeof(int32_t), s);
   // 1. Predict every row's class and capacity; slab offsets = scan of capacities.
@@ -1119,20 +1136,18 @@ rvsp_status_t rvsp_cuda_learned_symbolic(
                           p->rows_sym.p, s);
       ph.launches = 2;
     }
-    for (int c = kEmpty_ + 1; c < kNumClasses; ++c) {
+    const RowList sr = stripe_rows(p->sym_count, pred_off, whole, p->rows_sym.p);
+    if (sr.n > 0) {
+      // counted here, written at C by the compute (no slab slot); without
+      // room for their bitmaps, the plain two-pass path takes them
+      e = count_stripe_rows(p, op, b_rows, sr.rows, sr.n, s);
+      if (e != cudaSuccess) return map_cuda(e);
+      if (!p->sp_ready) launch_list_overflow(sr.rows, sr.n, fo, s);
+      ph.launches += p->sp_ready ? 4 : 1;
+    }
+    for (int c = kEmpty_ + 1; c < kStripe8; ++c) {
       if (p->sym_count[c] <= 0) continue;
       const bool all = c == whole;
-      if (c == kStripe) {
-        // counted here, written at C by the compute (no slab slot)
-        const int32_t *rows = all ? nullptr : p->rows_sym.p + pred_off[c];
-        e = count_stripe_rows(p, op, b_rows, rows, all ? a_rows : p->sym_count[c], s);
-        if (e != cudaSuccess) return map_cuda(e);
-        // no room for their bitmaps: the plain two-pass path takes them
-        if (!p->sp_ready)
-          launch_list_overflow(rows, all ? a_rows : p->sym_count[c], fo, s);
-        ph.launches += p->sp_ready ? 4 : 1;
-        continue;
-      }
       launch_numeric_class(c, op, p->ops.p, all ? nullptr : p->rows_sym.p + pred_off[c],
                            all ? a_rows : p->sym_count[c], nullptr, p->slab_col.p,
                            p->slab_val.p, true, facc, fbits, fslots, misc + kStatus,
@@ -1847,16 +1862,15 @@ int launch_shift_numeric(rvsp_cuda_plan *p, Lanes &ln, const Operands &op,
 // the values; returns the launches.
 int launch_stripe_rows(rvsp_cuda_plan *p, const Operands &op, const int32_t *c_rp,
                        int32_t *c_col, float *c_val, bool fill, cudaStream_t s) {
-  const int32_t nrows = p->num_count[kStripe];
-  if (!p->sp_ready || nrows <= 0) return 0;
-  const int32_t *rows = p->num_whole == kStripe ? nullptr : p->rows_num.p + p->num_off[kStripe];
+  const RowList sr = stripe_rows(p->num_count, p->num_off, p->num_whole, p->rows_num.p);
+  if (!p->sp_ready || sr.n <= 0) return 0;
   int32_t *status = p->misc.p + kStatus;
   if (fill)
-    launch_stripe_columns(p->sp, rows, nrows, p->sp_hslot.p, p->sp_bits.p, c_rp, c_col, status,
-                          s);
-  launch_stripe_values(p->sp, op, nrows, p->sp_items.p, p->sp_cap, p->sp_cnt.p,
-                       p->sp_cnt.p + 2, p->sp_bound.p, p->sp_ptr.p, c_rp, c_col, c_val, status,
-                       p->num_sms, s);
+    launch_stripe_columns(p->sp, sr.rows, sr.n, p->sp_hslot.p, p->sp_bits.p, p->sp_gpre.p,
+                          p->sp_soff.p, c_rp, c_col, status, s);
+  launch_stripe_values(p->sp, op, sr.n, p->sp_items.p, p->sp_cap, p->sp_cnt.p,
+                       p->sp_cnt.p + 2, p->sp_bound.p, p->sp_share.p, p->sp_ptr.p, p->sp_hslot.p, p->sp_bits.p,
+                       p->sp_gpre.p, c_rp, c_col, c_val, !fill, status, p->num_sms, s);
   return fill ? 2 : 1;
 }
 
@@ -2114,7 +2128,8 @@ rvsp_status_t rvsp_cuda_numeric(rvsp_cuda_plan_t p, void *stream,
     } else {
       cudaGetLastError();
     }
-    for (int c = kEmpty_ + 1; c < kNumClasses; ++c) {
+    ph.launches += launch_stripe_rows(p, op, c_row_ptr, c_col_idx, c_values, fill != 0, ln.next());
+    for (int c = kEmpty_ + 1; c < kStripe8; ++c) {
       if (p->num_count[c] <= 0) continue;
       if (persist && persist_class(c)) continue;
       const bool whole = c == p->num_whole;
@@ -2128,8 +2143,6 @@ rvsp_status_t rvsp_cuda_numeric(rvsp_cuda_plan_t p, void *stream,
       } else if (use_map && map_class(c))
         launch_map_numeric(c, op, p->ops.p, rows, nrows, c_row_ptr, c_values,
                            p->rmap_off.p, p->rmap.p, p->misc.p + kStatus, ln.next());
-      else if (c == kStripe && p->sp_ready)
-        launch_stripe_rows(p, op, c_row_ptr, c_col_idx, c_values, fill != 0, ln.next());
       else
         launch_numeric_class(c, op, p->ops.p, rows, nrows, c_row_ptr, c_col_idx, c_values,
                              fill != 0, dense_acc, dense_bits, p->dense_slots,
@@ -2253,10 +2266,12 @@ rvsp_status_t rvsp_cuda_plan_class_counts(rvsp_cuda_plan_t p, int32_t *sym_out,
                                           int32_t *num_out, int32_t n) {
   if (!p) return RVSP_ERROR_NULL_POINTER;
   for (int i = 0; i < n; ++i) {
-    const bool in = i < kStripe;  // (the stripe rows among the dense ones)
-    const bool dense = i == kDense;
-    if (sym_out) sym_out[i] = in ? p->sym_count[i] + (dense ? p->sym_count[kStripe] : 0) : 0;
-    if (num_out) num_out[i] = in ? p->num_count[i] + (dense ? p->num_count[kStripe] : 0) : 0;
+    // the stripe rows as the classes they come from
+    const int from = i == kB8192 ? kStripe8 : i == kDense ? kStripe : -1;
+    if (sym_out)
+      sym_out[i] = i < kStripe8 ? p->sym_count[i] + (from >= 0 ? p->sym_count[from] : 0) : 0;
+    if (num_out)
+      num_out[i] = i < kStripe8 ? p->num_count[i] + (from >= 0 ? p->num_count[from] : 0) : 0;
   }
   return RVSP_SUCCESS;
 }
