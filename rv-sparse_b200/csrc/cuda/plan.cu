@@ -374,43 +374,55 @@ bool side_streams(rvsp_cuda_plan *p, cudaStream_t s) {
   return p->side_state == 1;
 }
 
-// Streams of one numeric-only pass.  Its row groups (pattern kernels, table
-// tiles, leftover rows, class kernels) write disjoint rows of C and only
-// read A, B and the plan's tables, so all but the largest go to the side
-// streams, forked from the caller's stream and joined back into it: the
-// small launches, each bound by the latency of a few long rows, run beside
-// the large one and beside each other instead of after one another.  main()
-// is the caller's stream; next() hands out the side streams in turn
-// (without side streams, the caller's stream).
+// Streams of one pass whose row groups are independent: the numeric pass's
+// (pattern kernels, table tiles, leftover rows, class kernels) write disjoint
+// rows of C and only read A, B and the plan's tables, the symbolic pass's
+// write disjoint counts.  All but the largest go to the side streams, forked
+// from the caller's stream and joined back into it: the small launches, each
+// bound by the latency of a few long rows, run beside the large one and
+// beside each other instead of after one another.  main() is the caller's
+// stream; next() hands out the side streams in turn (without side streams,
+// the caller's stream); a side stream that is not handed out is not waited
+// for.
 struct Lanes {
   rvsp_cuda_plan *pl;
   cudaStream_t s;
   bool forked = false;
+  bool used[rvsp_cuda_plan::kSide] = {};
   int turn = 0;
   Lanes(rvsp_cuda_plan *p, cudaStream_t st, bool want) : pl(p), s(st) {
-    if (!(want && side_streams(p, st) && cudaEventRecord(p->fork_ev, st) == cudaSuccess)) return;
-    bool ok = true;
-    for (int i = 0; i < rvsp_cuda_plan::kSide; ++i)
-      ok = ok && cudaStreamWaitEvent(p->side[i], p->fork_ev, 0) == cudaSuccess;
-    forked = ok;
+    forked = want && side_streams(p, st) && cudaEventRecord(p->fork_ev, st) == cudaSuccess;
   }
   cudaStream_t main() const { return s; }
   cudaStream_t next() {
     if (!forked) return s;
-    const cudaStream_t x = pl->side[turn];
+    const int i = turn;
     turn = (turn + 1) % rvsp_cuda_plan::kSide;
-    return x;
+    if (!used[i]) {
+      if (cudaStreamWaitEvent(pl->side[i], pl->fork_ev, 0) != cudaSuccess) return s;
+      used[i] = true;
+    }
+    return pl->side[i];
   }
   void join() {
     if (!forked) return;
     for (int i = 0; i < rvsp_cuda_plan::kSide; ++i) {
+      if (!used[i]) continue;
       cudaEventRecord(pl->join_ev[i], pl->side[i]);
       cudaStreamWaitEvent(s, pl->join_ev[i], 0);
+      used[i] = false;
     }
     forked = false;
   }
   ~Lanes() { join(); }
 };
+
+// Whether a census has rows in several classes that launch of their own.
+bool several_classes(const int32_t *count) {
+  int n = count[kStripe8] + count[kStripe] > 0;
+  for (int c = kEmpty_ + 1; c < kStripe8; ++c) n += count[c] > 0;
+  return n > 1;
+}
 
 rvsp_status_t device_status_to_rvsp(int32_t st) {
   return st == kDevOk ? RVSP_SUCCESS : RVSP_ERROR_DEVICE;
@@ -964,16 +976,16 @@ cudaError_t symbolic_rest(rvsp_cuda_plan *p, cudaStream_t s, const Operands &op,
     // W1024 / W2048 rows count optimistically in a small table first; their
     // retry lists live in long_rows (free once the row statistics are done),
     // W1024's from 0, W2048's after it.
-    auto launch_class = [&](int c, const int32_t *rows, int32_t nrows) {
+    auto launch_class = [&](int c, const int32_t *rows, int32_t nrows, cudaStream_t cs) {
       if (symbolic_optimistic_class(c)) {
         const int32_t base = c == kW1024 ? 0 : p->sym_count[kW1024];
         launch_symbolic_optimistic(c, op, rows, nrows, p->counts.p, p->long_rows.p + base,
                                    misc + kRetryCount + (c == kW1024 ? 0 : 1),
-                                   misc + kStatus, p->num_sms, s);
+                                   misc + kStatus, p->num_sms, cs);
         return 2;
       }
       launch_symbolic_class(c, op, rows, nrows, p->counts.p, p->sym_bits.p, slots,
-                            misc + kStatus, p->num_sms, s);
+                            misc + kStatus, p->num_sms, cs);
       return 1;
     };
     // whole >= 0 is never a merge class here when merge_done (a class
@@ -985,20 +997,19 @@ cudaError_t symbolic_rest(rvsp_cuda_plan *p, cudaStream_t s, const Operands &op,
                           p->rows_sym.p, s);
       ph.launches = 2;
     }
+    Lanes ln(p, s, several_classes(p->sym_count));
+    for (int c = kEmpty_ + 1; c < kStripe8; ++c) {
+      if (p->sym_count[c] <= 0 || (merge_done && is_merge_class(c))) continue;
+      ph.launches += whole >= 0 ? launch_class(c, nullptr, a_rows, s)
+                                : launch_class(c, p->rows_sym.p + sym_off[c], p->sym_count[c],
+                                               ln.next());
+    }
     const RowList sr = stripe_rows(p->sym_count, sym_off, whole, p->rows_sym.p);
     if (sr.n > 0) {
       e = count_stripe_rows(p, op, b_rows, sr.rows, sr.n, s);
       if (e != cudaSuccess) return e;
-      ph.launches += 4;
-    }
-    const int classes = p->sp_ready ? kStripe8 : kNumClasses;
-    if (whole >= 0) {
-      if (whole < classes) ph.launches += launch_class(whole, nullptr, a_rows);
-    } else {
-      for (int c = kEmpty_ + 1; c < classes; ++c) {
-        if (p->sym_count[c] <= 0 || (merge_done && is_merge_class(c))) continue;
-        ph.launches += launch_class(c, p->rows_sym.p + sym_off[c], p->sym_count[c]);
-      }
+      // without room for their bitmaps they are heavy rows (either class)
+      ph.launches += p->sp_ready ? 5 : launch_class(kStripe8, sr.rows, sr.n, s);
     }
   }
   if (merge_done)  // the first scan counted numeric classes already
@@ -1136,6 +1147,16 @@ rvsp_status_t rvsp_cuda_learned_symbolic(
                           p->rows_sym.p, s);
       ph.launches = 2;
     }
+    Lanes ln(p, s, several_classes(p->sym_count));
+    for (int c = kEmpty_ + 1; c < kStripe8; ++c) {
+      if (p->sym_count[c] <= 0) continue;
+      const bool all = c == whole;
+      launch_numeric_class(c, op, p->ops.p, all ? nullptr : p->rows_sym.p + pred_off[c],
+                           all ? a_rows : p->sym_count[c], nullptr, p->slab_col.p,
+                           p->slab_val.p, true, facc, fbits, fslots, misc + kStatus,
+                           p->num_sms, ln.next(), &fo);
+      ph.launches += 1;
+    }
     const RowList sr = stripe_rows(p->sym_count, pred_off, whole, p->rows_sym.p);
     if (sr.n > 0) {
       // counted here, written at C by the compute (no slab slot); without
@@ -1144,15 +1165,6 @@ rvsp_status_t rvsp_cuda_learned_symbolic(
       if (e != cudaSuccess) return map_cuda(e);
       if (!p->sp_ready) launch_list_overflow(sr.rows, sr.n, fo, s);
       ph.launches += p->sp_ready ? 4 : 1;
-    }
-    for (int c = kEmpty_ + 1; c < kStripe8; ++c) {
-      if (p->sym_count[c] <= 0) continue;
-      const bool all = c == whole;
-      launch_numeric_class(c, op, p->ops.p, all ? nullptr : p->rows_sym.p + pred_off[c],
-                           all ? a_rows : p->sym_count[c], nullptr, p->slab_col.p,
-                           p->slab_val.p, true, facc, fbits, fslots, misc + kStatus,
-                           p->num_sms, s, &fo);
-      ph.launches += 1;
     }
   }
   // 3. Optimistic scan (valid when nothing overflowed) and the fingerprint of
@@ -2070,8 +2082,10 @@ rvsp_status_t rvsp_cuda_numeric(rvsp_cuda_plan_t p, void *stream,
     }
   }
   const bool use_map = fill == 0 && p->rmap_state == 1 && p->rmap_col == c_col_idx;
-  // numeric-only with every table in place: the row groups run side by side
-  Lanes ln(p, s, use_map && (!p->shift_active || p->shift_tables == 1));
+  // numeric-only with every table in place: all row groups run side by side;
+  // else the classes do (the members of shift classes follow, below)
+  const bool all_lanes = use_map && (!p->shift_active || p->shift_tables == 1);
+  Lanes ln(p, s, all_lanes || several_classes(p->num_count));
   bool rt_main = false;  // the largest shared-map pattern kernel, launched last
   {
     PhaseScope ph(p, s, RVSP_PHASE_NUMERIC);
@@ -2128,7 +2142,6 @@ rvsp_status_t rvsp_cuda_numeric(rvsp_cuda_plan_t p, void *stream,
     } else {
       cudaGetLastError();
     }
-    ph.launches += launch_stripe_rows(p, op, c_row_ptr, c_col_idx, c_values, fill != 0, ln.next());
     for (int c = kEmpty_ + 1; c < kStripe8; ++c) {
       if (p->num_count[c] <= 0) continue;
       if (persist && persist_class(c)) continue;
@@ -2149,10 +2162,13 @@ rvsp_status_t rvsp_cuda_numeric(rvsp_cuda_plan_t p, void *stream,
                              p->misc.p + kStatus, p->num_sms, ln.next());
       ph.launches += 1;
     }
+    // the stripe rows, usually the most work, last and on the caller's stream:
+    // their persistent blocks fill the SMs
+    ph.launches += launch_stripe_rows(p, op, c_row_ptr, c_col_idx, c_values, fill != 0, ln.main());
     if (rt_main)
       ph.launches += launch_pattern_kernels(p->rt, op, c_row_ptr, c_values, p->misc.p + kStatus,
                                             ln, true);
-    if (!p->shift_active) ln.join();
+    if (!p->shift_active || !all_lanes) ln.join();
   }
   if (p->shift_active) {
     // Shift-class members: columns by translation of their canonical rows
@@ -2171,7 +2187,10 @@ rvsp_status_t rvsp_cuda_numeric(rvsp_cuda_plan_t p, void *stream,
     }
     if (p->shift_tables != 1) return RVSP_ERROR_DEVICE;
     PhaseScope ph(p, s, RVSP_PHASE_NUMERIC);
-    ph.launches = launch_shift_numeric(p, ln, op, c_row_ptr, c_values);
+    Lanes members(p, s, !ln.forked);
+    ph.launches =
+        launch_shift_numeric(p, ln.forked ? ln : members, op, c_row_ptr, c_values);
+    members.join();
     ln.join();
   }
   return map_cuda(cudaGetLastError());
