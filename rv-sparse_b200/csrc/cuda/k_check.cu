@@ -27,9 +27,11 @@ __device__ __forceinline__ unsigned long long pack(int32_t row, int code) {
 }
 
 // Rows longer than this are checked by a warp each (long_row_check_kernel);
-// one thread walking a power-law hub row of tens of thousands of entries
-// would hold up the whole check.
-constexpr int32_t kCheckLongRow = 256;
+// one thread walking a long row would hold up the whole check.  Either way a
+// row's columns are loaded kCheckUnroll at a time before they are compared:
+// the checks wait on loads, not on bandwidth.
+constexpr int32_t kCheckLongRow = 64;
+constexpr int kCheckUnroll = 8;
 
 // Violation code of column c at a position whose predecessor in the row is
 // last (-1 at the row's start), 0 if none.
@@ -53,23 +55,29 @@ csr_check_kernel(int32_t rows, int32_t cols, const int32_t *__restrict__ row_ptr
   if (hi < lo || lo < 0 || hi > nnz) {
     code = kBadRowPtr;
   } else if (hi - lo > kCheckLongRow) {
-    // rows of more than kCheckLongRow entries (at most nnz / 257 of them)
+    // rows of more than kCheckLongRow entries (at most nnz / (kCheckLongRow + 1))
     const int32_t at = atomicAdd(long_rows, 1);
     if (at < long_cap) long_rows[1 + at] = r;
   } else {
     int32_t last = -1;
-    for (int32_t p = lo; p < hi && !code; ++p) {
-      const int32_t c = col_idx[p];
-      code = col_code(c, last, cols);
-      last = c;
+    const int32_t n = hi - lo;
+    for (int32_t e = 0; e < n && !code; e += kCheckUnroll) {
+      int32_t c[kCheckUnroll];
+#pragma unroll
+      for (int u = 0; u < kCheckUnroll; ++u) c[u] = e + u < n ? __ldg(col_idx + lo + e + u) : 0;
+#pragma unroll
+      for (int u = 0; u < kCheckUnroll; ++u) {
+        if (e + u < n && !code) code = col_code(c[u], last, cols);
+        last = c[u];
+      }
     }
   }
   if (code) atomicMin(result, pack(r, code));
 }
 
 // One warp per listed long row: 32 columns at a time, each compared with its
-// predecessor; the lowest violating position of the first chunk that has one
-// is the row's first violation.
+// predecessor; the lowest violating position of the first 32 that have one is
+// the row's first violation.
 __global__ void __launch_bounds__(kThreads)
 long_row_check_kernel(int32_t cols, const int32_t *__restrict__ row_ptr,
                       const int32_t *__restrict__ col_idx,
@@ -82,19 +90,28 @@ long_row_check_kernel(int32_t cols, const int32_t *__restrict__ row_ptr,
     const int32_t r = long_rows[1 + i];
     const int32_t lo = row_ptr[r], hi = row_ptr[r + 1];
     int32_t prev_last = -1;
-    for (int32_t p0 = lo; p0 < hi; p0 += 32) {
-      const int32_t p = p0 + lane;
-      const int32_t c = p < hi ? col_idx[p] : INT32_MAX;
-      int32_t last = __shfl_up_sync(kFull, c, 1);
-      if (lane == 0) last = prev_last;
-      const int code = p < hi ? col_code(c, last, cols) : 0;
-      const unsigned bad = __ballot_sync(kFull, code != 0);
-      if (bad) {
-        const int first = __ffs(bad) - 1;
-        if (lane == first) atomicMin(result, pack(r, code));
-        break;  // uniform
+    unsigned bad = 0;
+    for (int32_t p0 = lo; p0 < hi && !bad; p0 += 32 * kCheckUnroll) {
+      int32_t c[kCheckUnroll];
+#pragma unroll
+      for (int u = 0; u < kCheckUnroll; ++u) {
+        const int64_t p = int64_t(p0) + 32 * u + lane;
+        c[u] = p < hi ? __ldg(col_idx + p) : INT32_MAX;
       }
-      prev_last = __shfl_sync(kFull, c, 31);
+#pragma unroll
+      for (int u = 0; u < kCheckUnroll; ++u) {
+        const int64_t p = int64_t(p0) + 32 * u + lane;
+        int32_t last = __shfl_up_sync(kFull, c[u], 1);
+        if (lane == 0) last = prev_last;
+        prev_last = __shfl_sync(kFull, c[u], 31);
+        const int code = p < hi ? col_code(c[u], last, cols) : 0;
+        const unsigned now = __ballot_sync(kFull, code != 0);
+        if (now && !bad) {  // (the row's first violation; uniform)
+          bad = now;
+          if (lane == __ffs(now) - 1) atomicMin(result, pack(r, code));
+        }
+      }
+      if (p0 > INT32_MAX - 32 * kCheckUnroll) break;
     }
   }
 }
@@ -118,7 +135,7 @@ void launch_csr_check(int32_t rows, int32_t cols, const int32_t *row_ptr,
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    long_row_check_kernel<<<sms * 2, kThreads, 0, s>>>(cols, row_ptr, col_idx, result,
+    long_row_check_kernel<<<sms * 8, kThreads, 0, s>>>(cols, row_ptr, col_idx, result,
                                                        long_rows, cap);
   }
 }

@@ -264,17 +264,18 @@ learned_plan_kernel(Operands op, float b_mean_len, const float *__restrict__ par
     decide(row, p1 - p0, ops, y0, y1);
   }
   // Longer rows: one warp each (features over the lanes, hidden unit j on
-  // lane j), found 32 rows at a time.
+  // lane j).  Lane l of a warp looks at row base + l * wstride, so the long
+  // rows of one region (the hubs of a power-law matrix) go to different warps.
   const int32_t wstride = tstride >> 5;
   const int lane = lane_id();
-  for (int32_t base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; base < op.a_rows;
-       base += wstride * 32) {
-    const int32_t mine = base + lane;
+  for (int64_t base = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; base < op.a_rows;
+       base += int64_t(wstride) * 32) {
+    const int64_t mine = base + int64_t(lane) * wstride;
     const bool longrow =
         mine < op.a_rows && op.a_rp[mine + 1] - op.a_rp[mine] > kThreadRowNnz;
     unsigned todo = __ballot_sync(kFull, longrow);
     while (todo) {
-      const int32_t row = base + __ffs(todo) - 1;
+      const int32_t row = static_cast<int32_t>(base + int64_t(__ffs(todo) - 1) * wstride);
       todo &= todo - 1u;
       const RowFeat r = warp_row_features(op, row, b_mean_len);
       float x[kMlpIn];

@@ -12,6 +12,7 @@ namespace rvsp {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kStatUnroll = 8;
 
 // Adds one to class_count[c] for every lane with take, one atomic per class
 // per warp.
@@ -56,8 +57,18 @@ rowstats_kernel(Operands op, int64_t *__restrict__ ops, uint8_t *__restrict__ cl
       const int32_t slot = atomicAdd(long_count, 1);
       if (slot < max_long) long_rows[slot] = i;
     } else {
+      // (the loads of kStatUnroll entries are issued together: the walk waits
+      // on them, not on bandwidth)
       int64_t s = 0;
-      for (int32_t p = p0; p < p1; ++p) s += b_len(op, __ldg(op.a_col + p));
+      for (int32_t e = 0; e < p1 - p0; e += kStatUnroll) {
+        int32_t k[kStatUnroll];
+#pragma unroll
+        for (int u = 0; u < kStatUnroll; ++u)
+          k[u] = e + u < p1 - p0 ? __ldg(op.a_col + p0 + e + u) : -1;
+#pragma unroll
+        for (int u = 0; u < kStatUnroll; ++u)
+          if (e + u < p1 - p0) s += b_len(op, k[u]);
+      }
       c = with_stripes(
           classify_row(p1 - p0, s, s < op.b_cols ? s : op.b_cols, op.merge_ok),
           op.stripes);
@@ -89,7 +100,15 @@ rowstats_long_kernel(Operands op, const int32_t *__restrict__ long_rows,
     int32_t p0, p1;
     row_range(op, i, p0, p1);
     long long s = 0;
-    for (int32_t p = p0 + lane; p < p1; p += 32) s += b_len(op, __ldg(op.a_col + p));
+    for (int64_t p = int64_t(p0) + lane; p < p1; p += 32 * kStatUnroll) {
+      int32_t k[kStatUnroll];
+#pragma unroll
+      for (int u = 0; u < kStatUnroll; ++u)
+        k[u] = p + 32 * u < p1 ? __ldg(op.a_col + p + 32 * u) : -1;
+#pragma unroll
+      for (int u = 0; u < kStatUnroll; ++u)
+        if (p + 32 * u < p1) s += b_len(op, k[u]);
+    }
     s = warp_sum64(s);
     if (lane == 0) {
       const int c = with_stripes(
@@ -160,7 +179,7 @@ void launch_rowstats_long(const Operands &op, const int32_t *long_rows,
                           cudaStream_t s) {
   // The kernel reads the number of long rows on the device, so no host
   // round trip is needed; the grid strides over however many there are.
-  const int grid = num_sms * 2;
+  const int grid = num_sms * 8;
   rowstats_long_kernel<<<grid, kThreads, 0, s>>>(op, long_rows, long_count, ops,
                                                  cls, counts, class_count);
 }

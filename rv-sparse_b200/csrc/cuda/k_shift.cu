@@ -51,6 +51,8 @@ constexpr int kShiftMaxA = 32;
 constexpr int kShiftMaxOps = 1024;
 constexpr int kShiftMaxOut = 512;    // C entries of a pattern (the term tables' limit)
 constexpr int kShiftSamples = 2048;  // rows the probe keys
+constexpr int kProbeUnroll = 8;
+constexpr int kLaneMax = 64;         // longest B row one lane walks
 constexpr int kThreads = 256;
 
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
@@ -65,18 +67,23 @@ __device__ __forceinline__ unsigned long long warp_xor64(unsigned long long h) {
   return h;
 }
 
-// Key of B row k (warp-wide; every lane returns it).  Never 0.
+// A B row's key: the XOR of its entries' terms (column offset d at position
+// e), then its length.  Never 0.
+__device__ __forceinline__ unsigned long long brow_term(int32_t e, int32_t d) {
+  return mix64((static_cast<unsigned long long>(e) << 32) | static_cast<uint32_t>(d));
+}
+__device__ __forceinline__ unsigned long long brow_key_of(unsigned long long h, int32_t len) {
+  return mix64(h ^ (static_cast<unsigned long long>(len) * 0x9E3779B97F4A7C15ull)) | 1ull;
+}
+
+// Key of B row k (warp-wide; every lane returns it).
 __device__ __forceinline__ unsigned long long brow_key(const int32_t *__restrict__ b_rp,
                                                        const int32_t *__restrict__ b_col,
                                                        int32_t k, int lane) {
   const int32_t b0 = __ldg(b_rp + k), len = __ldg(b_rp + k + 1) - b0;
   unsigned long long h = 0;
-  for (int32_t e = lane; e < len; e += 32) {
-    const uint32_t off = static_cast<uint32_t>(__ldg(b_col + b0 + e) - k);
-    h ^= mix64((static_cast<unsigned long long>(e) << 32) | off);
-  }
-  h = warp_xor64(h);
-  return mix64(h ^ (static_cast<unsigned long long>(len) * 0x9E3779B97F4A7C15ull)) | 1ull;
+  for (int32_t e = lane; e < len; e += 32) h ^= brow_term(e, __ldg(b_col + b0 + e) - k);
+  return brow_key_of(warp_xor64(h), len);
 }
 
 // A row key's term for A nonzero j at column offset d over a B row whose
@@ -134,22 +141,44 @@ shift_probe_kernel(Operands op, int32_t samples, unsigned long long *__restrict_
     k = __ldg(op.a_col + p0 + lane);
     len = __ldg(op.b_rp + k + 1) - __ldg(op.b_rp + k);
   }
-  unsigned long long mine = 0;
-  for (int32_t j = 0; j < na; ++j) {
-    const int32_t kj = __shfl_sync(kFull, k, j);
-    const unsigned long long bk = brow_key(op.b_rp, op.b_col, kj, lane);
-    if (lane == j) mine = bk;
+  // A row of more products than a pattern takes is not keyed.  A short B row is
+  // keyed by the lane whose A nonzero selects it, all of them side by side (a
+  // warp a B row, one after another, was a chain of na loads; 26 us on a
+  // 27-point stencil, 11 us now), its entries kProbeUnroll at a time; the
+  // whole warp takes the longer ones.
+  const long long ops = warp_sum64(len);
+  unsigned long long key = 0;
+  if (ops <= kShiftMaxOps) {
+    unsigned long long h = 0;
+    const int32_t b0 = lane < na ? __ldg(op.b_rp + k) : 0;
+    const int32_t short_len = len <= kLaneMax ? len : 0;
+    for (int32_t e = 0; e < short_len; e += kProbeUnroll) {
+      int32_t c[kProbeUnroll];
+#pragma unroll
+      for (int u = 0; u < kProbeUnroll; ++u)
+        c[u] = e + u < len ? __ldg(op.b_col + b0 + e + u) : 0;
+#pragma unroll
+      for (int u = 0; u < kProbeUnroll; ++u)
+        if (e + u < len) h ^= brow_term(e + u, c[u] - k);
+    }
+    unsigned long long mine = brow_key_of(h, len);
+    for (unsigned rest = __ballot_sync(kFull, len > kLaneMax); rest; rest &= rest - 1u) {
+      const int j = __ffs(rest) - 1;
+      const unsigned long long bk =
+          brow_key(op.b_rp, op.b_col, __shfl_sync(kFull, k, j), lane);
+      if (lane == j) mine = bk;
+    }
+    key = row_key(na, lane, k - i, mine);
   }
-  const unsigned long long key = row_key(na, lane, k - i, mine);
-  const int32_t ops = warp_sum(len);
   if (lane == 0) {
     keys[w] = key;
     keys[samples + w] = static_cast<unsigned long long>(ops);
   }
 }
 
-// The decision: sorts the probe's keys (one block) and sets *on when at
-// least half of the sampled rows share their key with another sampled row
+// The decision: puts the probe's keys into a shared-memory table (one block;
+// a sort of them took 20 us) and sets *on when at least half of the sampled
+// rows share their key with another sampled row
 // and the sampled rows average at least min_mean_ops products (the caller's
 // bar: rows of few products are cheap on the merge kernels, and the
 // analysis and the tile builds would cost more than they save in a single
@@ -157,7 +186,9 @@ shift_probe_kernel(Operands op, int32_t samples, unsigned long long *__restrict_
 __global__ void __launch_bounds__(1024)
 shift_decide_kernel(const unsigned long long *__restrict__ keys, int32_t samples,
                     int32_t min_mean_ops, int32_t *__restrict__ on, CheckGuard guard) {
-  __shared__ unsigned long long sk[kShiftSamples];
+  constexpr int kSlots = 2 * kShiftSamples;
+  __shared__ unsigned long long sk[kSlots];  // 0: free (no key is 0)
+  __shared__ uint8_t shared_key[kSlots];
   __shared__ int32_t dup;
   __shared__ unsigned long long total_ops;
   const int tid = threadIdx.x;
@@ -174,17 +205,40 @@ shift_decide_kernel(const unsigned long long *__restrict__ keys, int32_t samples
     __syncthreads();
     if (lane_id() == 0 && o) atomicAdd(&total_ops, o);
   }
-  for (int t = tid; t < kShiftSamples; t += blockDim.x)
-    sk[t] = t < samples ? keys[t] : ~0ull;
-  __syncthreads();
-  block_bitonic_sort(sk, kShiftSamples);
-  int mine = 0;
-  for (int t = tid; t < samples; t += blockDim.x) {
-    const unsigned long long v = sk[t];
-    const bool shared = v != 0ull && v != ~0ull &&
-                        ((t > 0 && sk[t - 1] == v) || (t + 1 < samples && sk[t + 1] == v));
-    mine += shared ? 1 : 0;
+  for (int t = tid; t < kSlots; t += blockDim.x) {
+    sk[t] = 0ull;
+    shared_key[t] = 0;
   }
+  __syncthreads();
+  // (at most kShiftSamples keys in twice as many slots: every search ends)
+  constexpr int kPer = kShiftSamples / 1024;
+  int slot[kPer];
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    const int t = tid + q * 1024;
+    const unsigned long long v = t < samples ? keys[t] : 0ull;
+    slot[q] = -1;
+    if (v) {
+      uint32_t h = key_slot(v, kSlots - 1);
+      for (;;) {
+        unsigned long long cur = *reinterpret_cast<volatile unsigned long long *>(&sk[h]);
+        if (cur == 0ull) {
+          cur = atomicCAS(&sk[h], 0ull, v);
+          if (cur == 0ull) break;  // the key's first row
+        }
+        if (cur == v) {
+          shared_key[h] = 1;
+          break;
+        }
+        h = (h + 1) & (kSlots - 1);
+      }
+      slot[q] = static_cast<int>(h);
+    }
+  }
+  __syncthreads();
+  int mine = 0;
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) mine += slot[q] >= 0 && shared_key[slot[q]];
   mine = warp_sum(mine);
   if (lane_id() == 0 && mine) atomicAdd(&dup, mine);
   __syncthreads();
@@ -231,7 +285,6 @@ constexpr int kShiftRows = 4;
 constexpr int kSegCap = 1024;                // column indices one warp stages (4 KB)
 constexpr int kSegVec = kSegCap / 128;       // 16-byte loads a lane issues for it
 constexpr int kBWarps = 8, kAWarps = 4;      // warps per block: B passes, A passes
-constexpr int kLaneMax = 64;                 // longest B row one lane walks
 
 // A warp's 32 rows: this lane's row and bounds, and the staged segment.
 struct SegRows {

@@ -70,7 +70,7 @@ constexpr int kWarpsPerBlock = 4;      // warp-per-row kernels
 // columns (48 Ki words = 192 KiB), else in global scratch.
 constexpr int64_t kSmemBitmapMaxCols = 48 * 1024 * 32;
 // rowstats hands rows with more A nonzeros than this to a warp-per-row pass.
-constexpr int kLongRowNnz = 128;
+constexpr int kLongRowNnz = 64;
 
 // merge_ok: the matrix has at least kMergeMinRows rows.
 __host__ __device__ inline int classify_row(int32_t nnz_a, int64_t ops,
