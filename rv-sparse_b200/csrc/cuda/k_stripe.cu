@@ -54,6 +54,7 @@ constexpr int kStripeShares = 32;    // equal shares of B's entries
 constexpr int kItemOps = 32768;      // products an item aims at
 constexpr int kTaskOps = 1 << 16;    // products of a part of a cut row (count)
 constexpr int kSplitTasks = 1 << 15; // parts of cut rows at most
+constexpr int kPtrThreads = 256;
 constexpr int kItemRows = 64;        // rows a block of the item kernel
 constexpr int kBigRowOps = 1 << 18;  // rows whose items are drawn first
 constexpr size_t kStripeTableMax = size_t(256) << 20;
@@ -169,7 +170,7 @@ stripe_bounds_kernel(int32_t words, int32_t ns_max, const int32_t *__restrict__ 
 // (the row's end for t = ns_max).  A warp per row, a lane per stripe, each a
 // binary search of the row: short rows cost a few cached loads, and a hub row
 // of thousands of entries a dozen.
-__global__ void __launch_bounds__(kCountThreads)
+__global__ void __launch_bounds__(kPtrThreads)
 stripe_ptr_kernel(int32_t b_rows, const int32_t *__restrict__ b_rp,
                   const int32_t *__restrict__ b_col, int32_t ns_max,
                   const int32_t *__restrict__ bound, int32_t *__restrict__ ptr) {
@@ -296,9 +297,10 @@ stripe_tasks_kernel(const int32_t *__restrict__ rows, int32_t nrows,
   if (threadIdx.x == 0) s_n = 0;
   __syncthreads();
   const int32_t r = blockIdx.x * 128 + threadIdx.x;
+  int parts = 0;
   if (r < nrows) {
     const int64_t o = ops[row_of(rows, r)];
-    int parts = static_cast<int>(min((o + kTaskOps - 1) / kTaskOps, int64_t(64)));
+    parts = max(1, static_cast<int>(min((o + kTaskOps - 1) / kTaskOps, int64_t(64))));
     if (parts > 1) {
       const int at = atomicAdd(&cnt[0], parts);
       if (at + parts > kSplitTasks) {
@@ -310,9 +312,14 @@ stripe_tasks_kernel(const int32_t *__restrict__ rows, int32_t nrows,
         done[r] = 0;
       }
     }
-    if (parts <= 1)
-      tasks[kSplitTasks + nrows - 1 - atomicAdd(&cnt[1], 1)] = make_int2(r, 1 << 16);
   }
+  const unsigned whole = __ballot_sync(kFull, parts == 1);
+  int base = 0;
+  if (lane_id() == 0 && whole) base = atomicAdd(&cnt[1], __popc(whole));
+  base = __shfl_sync(kFull, base, 0);
+  if (parts == 1)
+    tasks[kSplitTasks + nrows - 1 - (base + __popc(whole & lanemask_lt()))] =
+        make_int2(r, 1 << 16);
   __syncthreads();
   for (int i = 0; i < s_n; ++i)
     for (int w = threadIdx.x; w < words; w += 128) bits[int64_t(s_cut[i]) * words + w] = 0u;
@@ -489,17 +496,18 @@ stripe_items_kernel(const int32_t *__restrict__ rows, int32_t nrows,
     for (int t = lane_id(); t <= ns_max; t += 32) s_off[r][t] = soff[h * (ns_max + 1) + t];
   }
   __syncthreads();
+  // (every thread stays for the warp's count; one past the rows has no stripes)
   const int32_t i = i0 + threadIdx.x;
-  if (i >= nrows) return;
-  const int32_t row = row_of(rows, i);
+  const bool live = i < nrows;
+  const int32_t row = live ? row_of(rows, i) : 0;
   const int32_t *so = s_off[threadIdx.x];
-  const float work = static_cast<float>(ops[row]);
+  const float work = live ? static_cast<float>(ops[row]) : 0.0f;
   const bool big = work >= float(kBigRowOps);
   int64_t at = 0;
   for (int pass = 0; pass < 2; ++pass) {
     int n = 0;
-    int32_t o = so[0];
-    for (int t0 = 0; t0 < ns_max;) {
+    int32_t o = live ? so[0] : 0;
+    for (int t0 = live ? 0 : ns_max; t0 < ns_max;) {
       const int32_t w0 = s_bound[t0];
       int t1 = t0 + 1;
       float part = s_share[t0];
@@ -522,7 +530,18 @@ stripe_items_kernel(const int32_t *__restrict__ rows, int32_t nrows,
       o = end;
       t0 = t1;
     }
-    if (!pass) at = atomicAdd(&cnt[big ? 0 : 1], n);
+    if (!pass) {
+      // places for all of the warp's items of either kind by one atomic each
+      const int mine = n, bigs = warp_incl_scan(big ? mine : 0), rest = warp_incl_scan(big ? 0 : mine);
+      int base = 0, base_rest = 0;
+      if (lane_id() == 31) {
+        if (bigs) base = atomicAdd(&cnt[0], bigs);
+        if (rest) base_rest = atomicAdd(&cnt[1], rest);
+      }
+      base = __shfl_sync(kFull, base, 31);
+      base_rest = __shfl_sync(kFull, base_rest, 31);
+      at = big ? base + bigs - mine : base_rest + rest - mine;
+    }
   }
 }
 
@@ -901,9 +920,9 @@ void launch_stripe_table(const StripeShape &g, int32_t b_rows, const int32_t *b_
                                                                    hist);
   stripe_bounds_kernel<<<1, 1024, 0, s>>>(g.words, g.ns_max, hist, bound, share);
   int grid = num_sms * 8;
-  const int need = (b_rows + kCountWarps - 1) / kCountWarps;
+  const int need = (b_rows + kPtrThreads / 32 - 1) / (kPtrThreads / 32);
   if (grid > need) grid = need;
-  stripe_ptr_kernel<<<grid, kCountThreads, 0, s>>>(b_rows, b_rp, b_col, g.ns_max, bound, ptr);
+  stripe_ptr_kernel<<<grid, kPtrThreads, 0, s>>>(b_rows, b_rp, b_col, g.ns_max, bound, ptr);
 }
 
 size_t stripe_tasks(int32_t nrows) { return size_t(kSplitTasks) + size_t(nrows); }
