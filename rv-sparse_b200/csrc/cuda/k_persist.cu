@@ -64,11 +64,12 @@ persist_numeric_kernel(Operands op, const int64_t *__restrict__ ops, PersistPlan
                        int32_t *__restrict__ head, const int32_t *__restrict__ c_rp,
                        float *__restrict__ c_val, const int64_t *__restrict__ moff,
                        const uint16_t *__restrict__ map, int32_t *__restrict__ status,
-                       int32_t acc_floats) {
+                       int32_t max_out) {
   extern __shared__ __align__(16) float smem_f32[];
+  __shared__ int4 s_seg[kPersistThreads / 32][32];
   __shared__ int32_t s_item;
   const int tid = threadIdx.x, lane = lane_id(), wid = tid >> 5;
-  float *const acc = smem_f32 + size_t(wid) * acc_floats;
+  float *const acc = smem_f32 + size_t(wid) * map_acc_floats(max_out);
   for (;;) {
     if (tid == 0) s_item = atomicAdd(head, 1);
     __syncthreads();
@@ -90,7 +91,7 @@ persist_numeric_kernel(Operands op, const int64_t *__restrict__ ops, PersistPlan
     } else {
       for (int32_t r = wid; r < cnt; r += kPersistThreads / 32)
         map_numeric_row(op, ops, row_of(g.rows, local + r), c_rp, c_val, moff, map, status,
-                        acc, lane);
+                        acc, max_out, s_seg[wid], lane);
     }
   }
 }
@@ -105,15 +106,15 @@ void launch_persist_numeric(const Operands &op, const int64_t *ops, const Persis
                             int32_t max_map_out, int blocks_per_sm, int num_sms,
                             cudaStream_t s) {
   if (pp.n_items <= 0) return;
-  const int32_t acc_floats = (max_map_out + 3) & ~3;
-  const size_t smem = size_t(kPersistThreads / 32) * size_t(acc_floats) * sizeof(float);
+  const size_t smem =
+      size_t(kPersistThreads / 32) * size_t(map_acc_floats(max_map_out)) * sizeof(float);
   cudaFuncSetAttribute(persist_numeric_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        static_cast<int>(smem));
   cudaMemsetAsync(head, 0, sizeof(int32_t), s);
   int grid = num_sms * (blocks_per_sm > 0 ? blocks_per_sm : 1);
   if (grid > pp.n_items) grid = pp.n_items;
   persist_numeric_kernel<<<grid, kPersistThreads, smem, s>>>(op, ops, pp, head, c_rp, c_val,
-                                                             moff, map, status, acc_floats);
+                                                             moff, map, status, max_map_out);
 }
 
 }  // namespace rvsp

@@ -189,7 +189,7 @@ map_dedup_resolve_kernel(const int32_t *__restrict__ rows, int32_t nrows,
   }
 }
 
-// Shared memory per warp: acc[T/2] f32 = 2 T bytes.
+// Shared memory per warp: map_acc_floats(T/2).
 template <int LOG2T>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 map_numeric_kernel(Operands op, const int64_t *__restrict__ ops,
@@ -199,10 +199,12 @@ map_numeric_kernel(Operands op, const int64_t *__restrict__ ops,
                    int32_t *__restrict__ status) {
   constexpr int H = 1 << (LOG2T - 1);
   extern __shared__ __align__(16) float smem_f32[];
-  float *acc = smem_f32 + size_t(threadIdx.x >> 5) * H;
+  __shared__ int4 s_seg[kWarpsPerBlock][32];
+  const int wb = threadIdx.x >> 5;
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (w >= nrows) return;
-  map_numeric_row(op, ops, row_of(rows, w), c_rp, c_val, moff, map, status, acc, lane_id());
+  map_numeric_row(op, ops, row_of(rows, w), c_rp, c_val, moff, map, status,
+                  smem_f32 + size_t(wb) * map_acc_floats(H), H, s_seg[wb], lane_id());
 }
 
 template <int LOG2T>
@@ -222,7 +224,8 @@ template <int LOG2T>
 void launch_numeric(const Operands &op, const int64_t *ops, const int32_t *rows,
                     int32_t nrows, const int32_t *c_rp, float *c_val, const int64_t *moff,
                     const uint16_t *map, int32_t *status, cudaStream_t s) {
-  const size_t smem = size_t(kWarpsPerBlock) * 2 * (size_t(1) << LOG2T);
+  const size_t smem =
+      size_t(kWarpsPerBlock) * map_acc_floats(1 << (LOG2T - 1)) * sizeof(float);
   const int grid = (nrows + kWarpsPerBlock - 1) / kWarpsPerBlock;
   map_numeric_kernel<LOG2T><<<grid, kWarpsPerBlock * 32, smem, s>>>(
       op, ops, rows, nrows, c_rp, c_val, moff, map, status);
