@@ -50,11 +50,14 @@ __device__ __forceinline__ void map_numeric_row(const Operands &op,
       __syncwarp();
       const int cnt = min(32, p1 - p);
       for (int j = 0; j < cnt; j += kMapUnroll) {  // (past cnt: empty B rows)
-        int pos[kMapUnroll];
-        float val[kMapUnroll];
+        // (shared memory bounds the walk: each entry of seg is read once)
+        int pos[kMapUnroll], len[kMapUnroll];
+        float val[kMapUnroll], a[kMapUnroll];
 #pragma unroll
         for (int u = 0; u < kMapUnroll; ++u) {
           const int4 s = seg[j + u];
+          len[u] = s.y;
+          a[u] = __int_as_float(s.z);
           pos[u] = spare;
           val[u] = 0.0f;
           if (lane < s.y) {
@@ -64,17 +67,16 @@ __device__ __forceinline__ void map_numeric_row(const Operands &op,
         }
 #pragma unroll
         for (int u = 0; u < kMapUnroll; ++u) {
-          const int4 s = seg[j + u];
-          const float a = __int_as_float(s.z);
           if (pos[u] >= m && pos[u] != spare) {  // C is not this product's
             bad = true;
             pos[u] = spare;
           }
-          acc[pos[u]] = __fadd_rn(acc[pos[u]], __fmul_rn(a, val[u]));
-          for (int e = 32 + lane; e - lane < s.y; e += 32) {
-            if (e < s.y) {
+          acc[pos[u]] = __fadd_rn(acc[pos[u]], __fmul_rn(a[u], val[u]));
+          if (len[u] > 32) {
+            const int4 s = seg[j + u];
+            for (int e = 32 + lane; e < s.y; e += 32) {
               const int q = __ldg(mp + s.w + e);
-              const float term = __fmul_rn(a, __ldg(op.b_val + s.x + e));
+              const float term = __fmul_rn(a[u], __ldg(op.b_val + s.x + e));
               if (q < m) acc[q] = __fadd_rn(acc[q], term);
               else bad = true;
             }
