@@ -212,35 +212,14 @@ __device__ __forceinline__ void ordered_apply(float *acc, bool valid, int slot,
   __syncwarp();
 }
 
-// Bitonic sort of n (power of two) 64-bit keys in shared memory by one warp.
-// Pair p of a stage with distance j (a power of two) compares i and i + j,
-// i = (p / j) * 2j + p % j, computed as p + (p & -j) (no division).
-__device__ __forceinline__ void warp_bitonic_sort(unsigned long long *s, int n) {
-  for (int k = 2; k <= n; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int p = lane_id(); p < (n >> 1); p += 32) {
-        const int i = p + (p & -j);
-        const int l = i + j;
-        const unsigned long long x = s[i], y = s[l];
-        const bool up = (i & k) == 0;
-        if ((x > y) == up) {
-          s[i] = y;
-          s[l] = x;
-        }
-      }
-      __syncwarp();
-    }
-  }
-}
-
-// Bitonic sort of 32 R 64-bit keys held in registers by one warp: element
+// Bitonic sort of 32 R keys held in registers by one warp: element
 // e = 32 r + lane is v[r] of that lane.  Stages with distance j < 32 pair
 // lanes (shuffle; the lane with bit j clear holds the lower index and keeps
 // the minimum in an ascending block, the maximum in a descending one);
 // stages with j >= 32 pair registers r and r | j/32 inside a lane.  No
 // shared memory.
-template <int R>
-__device__ __forceinline__ void warp_bitonic_sort_regs(unsigned long long (&v)[R]) {
+template <int R, typename Key>
+__device__ __forceinline__ void warp_bitonic_sort_regs(Key (&v)[R]) {
   constexpr int N = 32 * R;
   const int lane = lane_id();
 #pragma unroll
@@ -253,20 +232,19 @@ __device__ __forceinline__ void warp_bitonic_sort_regs(unsigned long long (&v)[R
         for (int r = 0; r < R; ++r) {
           if (r & jr) continue;  // r holds the pair's lower index
           const bool up = ((r * 32 + lane) & k) == 0;
-          const unsigned long long x = v[r], y = v[r | jr];
-          if ((x > y) == up) {
-            v[r] = y;
-            v[r | jr] = x;
-          }
+          const Key x = v[r], y = v[r | jr];
+          const Key lo = x < y ? x : y, hi = x < y ? y : x;
+          v[r] = up ? lo : hi;
+          v[r | jr] = up ? hi : lo;
         }
       } else {
         const bool lower = (lane & j) == 0;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const bool up = ((r * 32 + lane) & k) == 0;
-          const unsigned long long y = __shfl_xor_sync(kFull, v[r], j);
-          const unsigned long long lo = v[r] < y ? v[r] : y;
-          const unsigned long long hi = v[r] < y ? y : v[r];
+          const Key y = __shfl_xor_sync(kFull, v[r], j);
+          const Key lo = v[r] < y ? v[r] : y;
+          const Key hi = v[r] < y ? y : v[r];
           v[r] = lower == up ? lo : hi;
         }
       }
@@ -274,7 +252,9 @@ __device__ __forceinline__ void warp_bitonic_sort_regs(unsigned long long (&v)[R
   }
 }
 
-// Same, by a whole block (n power of two).
+// Bitonic sort of n (power of two) 64-bit keys in shared memory by a whole
+// block.  Pair p of a stage with distance j (a power of two) compares i and
+// i + j, i = (p / j) * 2j + p % j, computed as p + (p & -j) (no division).
 __device__ __forceinline__ void block_bitonic_sort(unsigned long long *s, int n) {
   for (int k = 2; k <= n; k <<= 1) {
     for (int j = k >> 1; j > 0; j >>= 1) {

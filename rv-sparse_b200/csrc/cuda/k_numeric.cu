@@ -19,9 +19,10 @@
 //           memory that each row leaves zeroed.
 //
 // Fill mode emits columns sorted: hash classes compact their (col, value)
-// pairs and bitonic-sort them (in registers up to 128 pairs a warp, else in
-// shared memory); the dense class walks its column bitmap in order.  Reuse mode (columns already in C) maps column -> position through
-// a hash of C's row and writes the values coalesced.
+// pairs and bitonic-sort them (a warp in registers, a block in shared memory);
+// the dense class walks its column bitmap in order.  Reuse mode (columns
+// already in C) maps column -> position through a hash of C's row and writes
+// the values coalesced.
 #include <climits>
 
 #include "device_common.cuh"
@@ -31,35 +32,55 @@ namespace rvsp {
 
 namespace {
 
-constexpr int kSteppingMinAvgLen = 16;  // avg B row length that favours stepping
+constexpr int kSteppingMinAvgLen = 6;  // avg B row length that favours stepping
+constexpr int kStepsAhead = 4;         // A nonzeros whose B entries are loaded together
 
 // ---- product walkers for warp-per-row classes --------------------------------
 
-// A walker's `stop` functor is called with the warp converged after each A
-// nonzero (stepping) or each tile (tiles); it returns a warp-uniform bool and
+// A walker's `stop` functor is called with the warp converged after every few A
+// nonzeros (stepping) or each tile (tiles); it returns a warp-uniform bool and
 // true ends the walk.  The plain path never stops (NoStop).
 struct NoStop {
   __device__ __forceinline__ bool operator()() const { return false; }
 };
 
 // Stepping: f(col, term) for each entry of A nonzero p's B row, lanes over
-// the B row, __syncwarp after each A nonzero.
+// the B row, __syncwarp after each A nonzero; stop after every kStepsAhead of
+// them.  The walk waits on loads, so the first 32 entries of kStepsAhead B
+// rows are loaded before the first of them is applied.  seg: 32 entries of
+// the warp's own shared memory.
 template <typename F, typename S = NoStop>
 __device__ __forceinline__ void warp_stepping(const Operands &op, int32_t p0,
-                                              int32_t p1, F f, S stop = S()) {
+                                              int32_t p1, int4 *seg, F f, S stop = S()) {
   const int lane = lane_id();
   for (int32_t p = p0; p < p1; p += 32) {
     const AChunk c = load_chunk(op.a_col, op.a_val, op.b_rp, p + lane, p1, true);
+    __syncwarp();  // the chunk before has been read
+    seg[lane] = make_int4(c.bbeg, c.len, __float_as_int(c.a), 0);
+    __syncwarp();
     const int cnt = min(32, p1 - p);
-    for (int jj = 0; jj < cnt; ++jj) {
-      const int len = __shfl_sync(kFull, c.len, jj);
-      const int bbeg = __shfl_sync(kFull, c.bbeg, jj);
-      const float a = __shfl_sync(kFull, c.a, jj);
-      for (int e = lane; e < len; e += 32) {
-        const int32_t col = __ldg(op.b_col + bbeg + e);
-        f(col, __fmul_rn(a, __ldg(op.b_val + bbeg + e)));
+    for (int j = 0; j < cnt; j += kStepsAhead) {  // (past cnt: empty B rows)
+      int len[kStepsAhead], beg[kStepsAhead];
+      int32_t col[kStepsAhead];
+      float a[kStepsAhead], val[kStepsAhead];
+#pragma unroll
+      for (int u = 0; u < kStepsAhead; ++u) {
+        const int4 s = seg[j + u];
+        beg[u] = s.x;
+        len[u] = s.y;
+        a[u] = __int_as_float(s.z);
+        if (lane < s.y) {
+          col[u] = __ldg(op.b_col + s.x + lane);
+          val[u] = __ldg(op.b_val + s.x + lane);
+        }
       }
-      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < kStepsAhead; ++u) {
+        if (lane < len[u]) f(col[u], __fmul_rn(a[u], val[u]));
+        for (int e = 32 + lane; e < len[u]; e += 32)
+          f(__ldg(op.b_col + beg[u] + e), __fmul_rn(a[u], __ldg(op.b_val + beg[u] + e)));
+        __syncwarp();
+      }
       if (stop()) return;
     }
   }
@@ -120,20 +141,44 @@ __device__ __forceinline__ void mark_overflow(const FusedOut &fo, int32_t row) {
   fo.ovf_rows[atomicAdd(fo.ovf_count, 1)] = row;
 }
 
-// Writes a row's kept (column, value) pairs, compacted in sbuf, sorted by
-// column: up to 32 R of them are sorted in registers (no shared-memory
+// Columns of B up to which a row's columns sort as 32-bit keys, column and
+// place among the row's pairs (at most 1024) together: half the shuffles of
+// (column, value) pairs.  Past it they sort as pairs.
+constexpr int kPlaceBits = 10;
+constexpr int32_t kKey32Cols = 1 << (32 - kPlaceBits);
+
+// Writes a row's kept (column, value) pairs, compacted in cols / vals, sorted
+// by column: up to 32 R of them are sorted in registers (no shared-memory
 // traffic, which bounds this kernel) and the first `out` go to C from out0,
 // 32 consecutive entries per store.
 template <int R>
-__device__ __forceinline__ void write_sorted_regs(const unsigned long long *sbuf, int kept,
-                                                  int out, int64_t out0, int32_t *c_col,
-                                                  float *c_val) {
+__device__ __forceinline__ void write_sorted_regs(const int32_t *cols, const float *vals,
+                                                  bool key32, int kept, int out, int64_t out0,
+                                                  int32_t *c_col, float *c_val) {
   const int lane = lane_id();
+  if (key32) {
+    uint32_t v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int e = r * 32 + lane;
+      v[r] = e < kept ? static_cast<uint32_t>(cols[e]) << kPlaceBits | e : ~0u;
+    }
+    warp_bitonic_sort_regs<R>(v);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int e = r * 32 + lane;
+      if (e < out) {
+        c_col[out0 + e] = static_cast<int32_t>(v[r] >> kPlaceBits);
+        c_val[out0 + e] = vals[v[r] & ((1u << kPlaceBits) - 1u)];
+      }
+    }
+    return;
+  }
   unsigned long long v[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int e = r * 32 + lane;
-    v[r] = e < kept ? sbuf[e] : ~0ull;
+    v[r] = e < kept ? pack_col_val(cols[e], vals[e]) : ~0ull;
   }
   warp_bitonic_sort_regs<R>(v);
 #pragma unroll
@@ -146,16 +191,16 @@ __device__ __forceinline__ void write_sorted_regs(const unsigned long long *sbuf
   }
 }
 
-// Blocks per SM the fill kernel asks the compiler to fit: 16 (32 registers)
-// for W64, W128 and non-fused W256 rows, which fit 16 blocks by shared memory
-// too and need no spill at 32 registers; 12 (up to 42) for the others.
-constexpr int fill_min_blocks(int log2t, bool fused) {
-  return log2t <= 7 || (log2t == 8 && !fused) ? 16 : 12;
+// Blocks per SM the fill kernel asks the compiler to fit, by their registers:
+// as many as fit by shared memory (12 T bytes a warp) for the largest tables.
+constexpr int fill_min_blocks(int log2t) {
+  return log2t <= 8 ? 10 : log2t == 9 ? 8 : log2t == 10 ? 4 : 2;
 }
 
-// Shared memory per warp: sbuf[T/2] u64 | keys[T] i32 | vals[T] f32 = 12 T bytes.
+// Shared memory per warp: scol[T/2] i32 | sval[T/2] f32 | keys[T] i32 |
+// vals[T] f32 = 12 T bytes.
 template <int LOG2T, bool kFused>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, fill_min_blocks(LOG2T, kFused))
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, fill_min_blocks(LOG2T))
 num_warp_fill_kernel(Operands op, const int64_t *__restrict__ ops,
                      const int32_t *__restrict__ rows, int32_t nrows,
                      const int32_t *__restrict__ c_rp, int32_t *__restrict__ c_col,
@@ -163,8 +208,11 @@ num_warp_fill_kernel(Operands op, const int64_t *__restrict__ ops,
                      FusedOut fo) {
   constexpr int T = 1 << LOG2T, H = T / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int4 s_seg[kWarpsPerBlock][32];
+  int4 *seg = s_seg[threadIdx.x >> 5];
   unsigned char *base = smem_raw + size_t(threadIdx.x >> 5) * (12 * T);
-  unsigned long long *sbuf = reinterpret_cast<unsigned long long *>(base);
+  int32_t *scol = reinterpret_cast<int32_t *>(base);
+  float *sval = reinterpret_cast<float *>(base + 4 * H);
   int32_t *keys = reinterpret_cast<int32_t *>(base + 4 * T);
   float *vals = reinterpret_cast<float *>(base + 8 * T);
 
@@ -184,7 +232,7 @@ num_warp_fill_kernel(Operands op, const int64_t *__restrict__ ops,
   bool over = false;  // fused: the row outgrew its capacity (warp-uniform)
   if (use_stepping(ops, row, p1 - p0)) {
     warp_stepping(
-        op, p0, p1,
+        op, p0, p1, seg,
         [&](int32_t col, float term) {
           bool created;
           const int s = hash_insert(keys, LOG2T, col, created);
@@ -230,29 +278,28 @@ num_warp_fill_kernel(Operands op, const int64_t *__restrict__ ops,
     const bool occ = key != kEmpty;
     const unsigned msk = __ballot_sync(kFull, occ);
     const int pos = n + __popc(msk & lanemask_lt());
-    if (occ && pos < H) sbuf[pos] = pack_col_val(key, vals[s]);
+    if (occ && pos < H) {
+      scol[pos] = key;
+      sval[pos] = vals[s];
+    }
     n += __popc(msk);
   }
   const int kept = n < H ? n : H;
   const int out = kept < m ? kept : m;
   __syncwarp();
+  const bool key32 = op.b_cols <= kKey32Cols;
   if (kept <= 32) {
-    write_sorted_regs<1>(sbuf, kept, out, out0, c_col, c_val);
+    write_sorted_regs<1>(scol, sval, key32, kept, out, out0, c_col, c_val);
   } else if (H >= 64 && kept <= 64) {
-    write_sorted_regs<2>(sbuf, kept, out, out0, c_col, c_val);
+    write_sorted_regs<2>(scol, sval, key32, kept, out, out0, c_col, c_val);
   } else if (H >= 128 && kept <= 128) {
-    write_sorted_regs<4>(sbuf, kept, out, out0, c_col, c_val);
-  } else {
-    int npow = 1;
-    while (npow < kept) npow <<= 1;
-    for (int e = kept + lane; e < npow; e += 32) sbuf[e] = ~0ull;
-    __syncwarp();
-    warp_bitonic_sort(sbuf, npow);
-    for (int e = lane; e < out; e += 32) {
-      const unsigned long long x = sbuf[e];
-      c_col[out0 + e] = packed_col(x);
-      c_val[out0 + e] = packed_val(x);
-    }
+    write_sorted_regs<4>(scol, sval, key32, kept, out, out0, c_col, c_val);
+  } else if (H >= 256 && kept <= 256) {
+    write_sorted_regs<8>(scol, sval, key32, kept, out, out0, c_col, c_val);
+  } else if (H >= 512 && kept <= 512) {
+    write_sorted_regs<16>(scol, sval, key32, kept, out, out0, c_col, c_val);
+  } else if (H >= 1024) {
+    write_sorted_regs<32>(scol, sval, key32, kept, out, out0, c_col, c_val);
   }
   const bool any_bad = __any_sync(kFull, bad);
   if (lane == 0) {
@@ -281,6 +328,7 @@ num_warp_reuse_kernel(Operands op, const int64_t *__restrict__ ops,
   int32_t *keys = reinterpret_cast<int32_t *>(base);
   int32_t *posv = reinterpret_cast<int32_t *>(base + 4 * T);
   float *acc = reinterpret_cast<float *>(base + 8 * T);
+  __shared__ int4 s_seg[kWarpsPerBlock][32];
 
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (w >= nrows) return;
@@ -302,7 +350,7 @@ num_warp_reuse_kernel(Operands op, const int64_t *__restrict__ ops,
   const int32_t p0 = op.a_rp[row], p1 = op.a_rp[row + 1];
   bool missing = false;
   if (use_stepping(ops, row, p1 - p0)) {
-    warp_stepping(op, p0, p1, [&](int32_t col, float term) {
+    warp_stepping(op, p0, p1, s_seg[threadIdx.x >> 5], [&](int32_t col, float term) {
       const int s = hash_find(keys, LOG2T, col);
       if (s >= 0) {
         const int pos = posv[s];
