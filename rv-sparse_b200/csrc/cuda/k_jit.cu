@@ -17,7 +17,7 @@
 //   the A nonzeros are cut into groups whose B spans overlap (in a stencil
 //   the three x-neighbours of a row read B rows one apart, so the tile's
 //   three spans share all but two rows; the grouping is chosen when the
-//   kernel is built, from the largest union span over the pattern's tiles);
+//   kernel is built, from the largest union spans over the pattern's tiles);
 //   per group, the union of the lanes' B rows is one contiguous range of B
 //   values, copied into shared memory by one bulk copy (cp.async.bulk, the
 //   copy engine; its completion is counted on an mbarrier), one group ahead
@@ -519,210 +519,173 @@ void kernels_for(const std::vector<std::string> &keys, const Source &source,
                       .count();
 }
 
-// Warps per block of the span and record kernels, and the A entries of one
-// tile's segment they stage in shared memory (a longer segment's B row
-// starts are read from global memory instead; 4 KB a warp and at most 64
-// registers keep 32 warps an SM resident, these kernels being bound by load
-// latency).
-constexpr int kBuildWarps = 4;
-constexpr int kBuildSeg = 1024;
+// Warps per block of the record kernel.
+constexpr int kBuildWarps = 8;
 
-// The start of B row a_col[seg0 + i], for every i < seg, into sb[i]: loads
-// of a_col coalesced across the lanes, 512 entries at a time (16 loads a
-// lane in flight, then their 16 gathers of b_rp).
-__device__ __forceinline__ void stage_b_starts(int32_t *sb, int32_t seg0, int32_t seg,
-                                               const int32_t *__restrict__ a_col,
-                                               const int32_t *__restrict__ b_rp, int lane) {
-  for (int32_t i0 = 0; i0 < seg; i0 += 512) {
-    int32_t c[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const int32_t i = i0 + u * 32 + lane;
-      c[u] = i < seg ? __ldg(a_col + seg0 + i) : 0;
-    }
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const int32_t i = i0 + u * 32 + lane;
-      c[u] = i < seg ? __ldg(b_rp + c[u]) : 0;
-    }
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const int32_t i = i0 + u * 32 + lane;
-      if (i < seg) sb[i] = c[u];
-    }
+// The records lie in row order, so that the persistent warps, which take them
+// one after another, work on neighbouring rows at any one time and their B
+// ranges stay in L2 between tiles (in the order the builder's blocks happened
+// to finish, a 128^3 stencil's repeat took 0.565 ms instead of 0.512).  A tile's
+// place: tiles[chunk].w among its block of kRankChunks chunks, and the
+// pattern's tiles before that block, rank[k * blocks + block].
+constexpr int kRankChunks = 1024;
+
+__device__ __forceinline__ int program_of(const TilePrograms &P, int32_t pid) {
+  int k = 0;
+  while (k < P.n && P.p[k].pid != pid) ++k;
+  return pid < 0 ? P.n : k;
+}
+
+__global__ void __launch_bounds__(kRankChunks)
+tile_rank_kernel(int4 *__restrict__ tiles, int32_t nchunks,
+                 const __grid_constant__ TilePrograms P, int32_t *__restrict__ rank) {
+  __shared__ int32_t s_cnt[kJitMaxPatterns][kRankChunks / 32];
+  const int lane = lane_id(), wib = threadIdx.x >> 5;
+  const int32_t i = blockIdx.x * kRankChunks + threadIdx.x;
+  const int k = i < nchunks ? program_of(P, tiles[i].z) : P.n;
+  int mine = 0;
+  for (int q = 0; q < P.n; ++q) {
+    const unsigned b = __ballot_sync(kFull, k == q);
+    if (lane == 0) s_cnt[q][wib] = __popc(b);
+    if (k == q) mine = __popc(b & lanemask_lt());
   }
-  __syncwarp();
+  __syncthreads();
+  if (wib < P.n) {  // warp q: the counts of pattern q
+    const int c = s_cnt[wib][lane], incl = warp_incl_scan(c);
+    s_cnt[wib][lane] = incl - c;
+    if (lane == 31) rank[wib * gridDim.x + blockIdx.x] = incl;
+  }
+  __syncthreads();
+  if (k < P.n) tiles[i].w = s_cnt[k][wib] + mine;
 }
 
-// The start of the B row of segment entry i: staged, or read through a_col.
-__device__ __forceinline__ int32_t b_start(const int32_t *sb, bool staged, int32_t seg0,
-                                           int32_t i, const int32_t *__restrict__ a_col,
-                                           const int32_t *__restrict__ b_rp) {
-  return staged ? sb[i] : __ldg(b_rp + __ldg(a_col + seg0 + i));
+// A warp per pattern: rank's block counts become the tiles before each block.
+__global__ void __launch_bounds__(kJitMaxPatterns * 32)
+tile_rank_scan_kernel(int32_t blocks, int32_t n, int32_t *__restrict__ rank) {
+  const int lane = lane_id(), q = threadIdx.x >> 5;
+  if (q >= n) return;
+  int32_t base = 0;
+  for (int32_t b0 = 0; b0 < blocks; b0 += 32) {
+    const int c = b0 + lane < blocks ? rank[q * blocks + b0 + lane] : 0;
+    const int incl = warp_incl_scan(c);
+    if (b0 + lane < blocks) rank[q * blocks + b0 + lane] = base + incl - c;
+    base += __shfl_sync(kFull, incl, 31);
+  }
 }
 
-// A tile's segment: from the first active row's first A nonzero to the last
-// active row's end.
-__device__ __forceinline__ void tile_segment(const int4 &t, const int32_t *__restrict__ a_rp,
-                                             int32_t *seg0, int32_t *seg) {
+// The tile records of every compiled pattern (see the file comment), a warp
+// per chunk of rows; marks the patterns (desc[pid].w = 1: the table kernel
+// leaves their tiles alone).  kShifted as in the tile builder: a lane's B row
+// starts are then consecutive entries of b_rp, without a look at a_col.
+template <bool kShifted>
+__global__ void __launch_bounds__(kBuildWarps * 32)
+record_kernel(const int4 *__restrict__ tiles, int32_t nchunks,
+              const __grid_constant__ TilePrograms P, const int32_t *__restrict__ rank,
+              int32_t blocks, const uint16_t *__restrict__ lens, const int32_t *__restrict__ offs,
+              const int32_t *__restrict__ a_rp, const int32_t *__restrict__ a_col,
+              const int32_t *__restrict__ b_rp, int4 *__restrict__ desc) {
+  if (blockIdx.x == 0 && threadIdx.x < P.n) desc[P.p[threadIdx.x].pid].w = 1;
+  const int lane = lane_id();
+  const int64_t w = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  if (w >= nchunks) return;
+  const int4 t = tiles[w];
+  const int k = program_of(P, t.z);
+  if (k == P.n) return;
+  const TileProgram &q = P.p[k];
+  const int32_t place = t.w + rank[k * blocks + static_cast<int32_t>(w / kRankChunks)];
+  const int na = q.na, ng = q.ng;
   const uint32_t mask = static_cast<uint32_t>(t.y);
+  const bool active = (mask >> lane) & 1u;
   const int first = __ffs(static_cast<int>(mask)) - 1, last = 31 - __clz(static_cast<int>(mask));
-  *seg0 = a_rp[t.x + first];
-  *seg = a_rp[t.x + last + 1] - *seg0;
+  const int32_t row = t.x + lane;
+  const int32_t seg0 = a_rp[t.x + first], seg = a_rp[t.x + last + 1] - seg0;
+  const int32_t p = active ? a_rp[row] : 0;
+  const int32_t len = lane < na ? lens[size_t(t.z) * 32 + lane] : 0;
+  const int32_t off = lane < na ? offs[size_t(t.z) * 32 + lane] : 0;
+  int32_t *const rec = q.prog + size_t(place) * size_t(q.rw);
+  uint16_t *const aoff = reinterpret_cast<uint16_t *>(rec + 4 + 2 * ng);
+  uint16_t *const d = aoff + 32;
+  // A nonzero `lane`: its group and the range its B rows take over the tile
+  const int gid = lane < na ? q.group[lane] : kNoGroup;
+  int32_t lo = INT_MAX, hi = INT_MIN;
+  if (kShifted) {
+    if (len > 0) {
+      lo = __ldg(b_rp + t.x + first + off);
+      hi = __ldg(b_rp + t.x + last + off) + len;
+    }
+  } else {
+    for (int j = 0; j < na; ++j) {
+      const int32_t r = active ? __ldg(b_rp + __ldg(a_col + p + j)) : 0;
+      const int32_t l = __reduce_min_sync(kFull, active ? r : INT_MAX);
+      const int32_t h = __reduce_max_sync(kFull, active ? r : INT_MIN);
+      if (lane == j && len > 0) {
+        lo = l;
+        hi = h + len;
+      }
+    }
+  }
+  // over the group (runs of at most kJitMaxGroup = 8 lanes)
+  int32_t glo = lo, ghi = hi;
+#pragma unroll
+  for (int i = 1; i < kJitMaxGroup; ++i) {
+    const int32_t l0 = __shfl_up_sync(kFull, lo, i), l1 = __shfl_down_sync(kFull, lo, i);
+    const int32_t h0 = __shfl_up_sync(kFull, hi, i), h1 = __shfl_down_sync(kFull, hi, i);
+    const int g0 = __shfl_up_sync(kFull, gid, i), g1 = __shfl_down_sync(kFull, gid, i);
+    if (lane >= i && g0 == gid) {
+      glo = min(glo, l0);
+      ghi = max(ghi, h0);
+    }
+    if (lane + i < 32 && g1 == gid) {
+      glo = min(glo, l1);
+      ghi = max(ghi, h1);
+    }
+  }
+  const int before = __shfl_up_sync(kFull, gid, 1);
+  if (gid != kNoGroup && (lane == 0 || before != gid)) {
+    rec[4 + 2 * gid] = glo;
+    rec[5 + 2 * gid] = ghi;
+  }
+  // this lane's row: the B row starts of its A nonzeros, as offsets
+  constexpr int kAhead = 9;
+  for (int j0 = 0; j0 < na; j0 += kAhead) {
+    int32_t r[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      const int32_t o = __shfl_sync(kFull, off, (j0 + i) & 31);
+      r[i] = 0;
+      if (active && j0 + i < na)
+        r[i] = kShifted ? __ldg(b_rp + row + o) : __ldg(b_rp + __ldg(a_col + p + j0 + i));
+    }
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      const int32_t l = __shfl_sync(kFull, len, (j0 + i) & 31);
+      const int32_t g = __shfl_sync(kFull, glo, (j0 + i) & 31);
+      if (j0 + i < na)
+        d[(j0 + i) * 32 + lane] = static_cast<uint16_t>(active && l > 0 ? r[i] - g : 0);
+    }
+  }
+  aoff[lane] = static_cast<uint16_t>(active ? p - seg0 : 0);
+  if (lane == 0) {
+    rec[0] = t.x;
+    rec[1] = t.y;
+    rec[2] = seg0;
+    rec[3] = seg;
+    q.arange[place] = make_int2(seg0, seg);
+  }
 }
 
-// Union spans of a sample of a pattern's tiles (every stride-th; warp per
-// tile, grid-stride): for every A nonzero j0 and run length g in
-// [1, kJitMaxGroup], span[j0 * kJitMaxGroup + g - 1] = the largest, over the
-// sample, of (end of the last B value - first B value) that the tile's rows
-// read for A nonzeros j0 .. j0 + g - 1.  A nonzero with an empty B row reads
-// nothing.  The grouping is chosen from these; the tile records then measure
-// every tile's ranges.  span zeroed by the caller.
-__global__ void __launch_bounds__(kBuildWarps * 32, 8)
-span_kernel(const int4 *__restrict__ tiles, int32_t ntiles, int32_t stride,
-            const int4 *__restrict__ desc,
-            const uint16_t *__restrict__ lens, const int32_t *__restrict__ a_rp,
-            const int32_t *__restrict__ a_col, const int32_t *__restrict__ b_rp,
-            int32_t *__restrict__ span) {
-  __shared__ int32_t sseg[kBuildWarps][kBuildSeg];
-  __shared__ int32_t slo[kBuildWarps][32], shi[kBuildWarps][32], slen[32];
-  const int wib = threadIdx.x >> 5, lane = lane_id();
-  const int32_t na = desc->x;  // A nonzeros of the pattern
-  if (na <= 0 || na > 32) return;
-  if (threadIdx.x < 32) slen[threadIdx.x] = threadIdx.x < na ? lens[threadIdx.x] : 0;
-  __syncthreads();
-  int32_t um[kJitMaxGroup];
-#pragma unroll
-  for (int g = 0; g < kJitMaxGroup; ++g) um[g] = 0;
-  for (int64_t w = int64_t(blockIdx.x) * kBuildWarps + wib; w * stride < ntiles;
-       w += int64_t(gridDim.x) * kBuildWarps) {
-    const int4 t = tiles[w * stride];
-    const bool active = ((static_cast<uint32_t>(t.y) >> lane) & 1u) != 0u;
-    int32_t seg0 = 0, seg = 0;
-    tile_segment(t, a_rp, &seg0, &seg);
-    const int32_t p = active ? a_rp[t.x + lane] - seg0 : 0;
-    const bool staged = seg <= kBuildSeg;
-    if (staged) stage_b_starts(sseg[wib], seg0, seg, a_col, b_rp, lane);
-    for (int32_t j = 0; j < na; ++j) {
-      const bool use = active && slen[j] > 0 && p + j < seg;
-      const int32_t r = use ? b_start(sseg[wib], staged, seg0, p + j, a_col, b_rp) : 0;
-      const int32_t lo = __reduce_min_sync(kFull, use ? r : INT_MAX);
-      const int32_t hi = __reduce_max_sync(kFull, use ? r + slen[j] : INT_MIN);
-      if (lane == 0) {
-        slo[wib][j] = lo;
-        shi[wib][j] = hi;
-      }
-    }
-    __syncwarp();
-    if (lane < na) {
-      int32_t lo = INT_MAX, hi = INT_MIN;
-#pragma unroll
-      for (int g = 0; g < kJitMaxGroup; ++g) {
-        if (lane + g < na) {
-          lo = min(lo, slo[wib][lane + g]);
-          hi = max(hi, shi[wib][lane + g]);
-          if (hi > lo) um[g] = max(um[g], hi - lo);
-        }
-      }
-    }
-    __syncwarp();
-  }
-  if (lane < na) {
-#pragma unroll
-    for (int g = 0; g < kJitMaxGroup; ++g)
-      if (um[g] > 0) atomicMax(span + lane * kJitMaxGroup + g, um[g]);
-  }
-}
-
-// Tile records of one pattern (warp per tile, grid-stride), rw words each:
-//   [0] first row of the tile, [1] lane mask, [2] A index of the first active
-//   row's first nonzero, [3] A entries from there to the last active row's
-//   end;  [4 + 2g], [5 + 2g]: the B range [lo, hi) that group g stages;
-//   then 32 uint16 A offsets (lane's first nonzero - [2]) and, per A nonzero
-//   j and lane, the uint16 offset of the lane's B row k_j from its group's
-//   lo (0 for inactive lanes and empty B rows).
-// arange[tile] = ([2], [3]); maxima[0] = the largest [3], maxima[1 + g] =
-// the largest B range of group g.  Structure only: built once per
-// structure, read by every numeric-only repeat.
-__global__ void __launch_bounds__(kBuildWarps * 32, 8)
-program_kernel(const int4 *__restrict__ tiles, int32_t ntiles, int32_t na, int32_t ngroups,
-               const int2 *__restrict__ groups, const uint16_t *__restrict__ lens,
-               const int32_t *__restrict__ a_rp, const int32_t *__restrict__ a_col,
-               const int32_t *__restrict__ b_rp, int32_t rw, int32_t *__restrict__ prog,
-               int2 *__restrict__ arange, int32_t *__restrict__ maxima) {
-  __shared__ int32_t sseg[kBuildWarps][kBuildSeg];
-  __shared__ int32_t slen[32];
-  const int wib = threadIdx.x >> 5, lane = lane_id();
-  if (threadIdx.x < 32) slen[threadIdx.x] = threadIdx.x < na ? lens[threadIdx.x] : 0;
-  __syncthreads();
-  // the warp's maxima over its tiles (the A extent; lane g: group g's B
-  // range), merged into maxima once at the end
-  int32_t mine = 0, segmax = 0;
-  for (int64_t w = int64_t(blockIdx.x) * kBuildWarps + wib; w < ntiles;
-       w += int64_t(gridDim.x) * kBuildWarps) {
-    const int4 t = tiles[w];
-    const bool active = ((static_cast<uint32_t>(t.y) >> lane) & 1u) != 0u;
-    int32_t seg0 = 0, seg = 0;
-    tile_segment(t, a_rp, &seg0, &seg);
-    const int32_t p = active ? a_rp[t.x + lane] - seg0 : 0;
-    const bool staged = seg <= kBuildSeg;
-    if (staged) stage_b_starts(sseg[wib], seg0, seg, a_col, b_rp, lane);
-    int32_t *const rec = prog + w * rw;
-    if (lane == 0) {
-      rec[0] = t.x;
-      rec[1] = t.y;
-      rec[2] = seg0;
-      rec[3] = seg;
-      arange[w] = make_int2(seg0, seg);
-    }
-    segmax = max(segmax, seg);
-    uint16_t *const aoff = reinterpret_cast<uint16_t *>(rec + 4 + 2 * ngroups);
-    uint16_t *const d = aoff + 32;
-    aoff[lane] = static_cast<uint16_t>(p);
-    for (int32_t g = 0; g < ngroups; ++g) {
-      const int2 gr = groups[g];
-      int32_t lo = INT_MAX, hi = INT_MIN;
-      for (int32_t j = gr.x; j < gr.y; ++j) {
-        if (active && slen[j] > 0 && p + j < seg) {
-          const int32_t r = b_start(sseg[wib], staged, seg0, p + j, a_col, b_rp);
-          lo = min(lo, r);
-          hi = max(hi, r + slen[j]);
-        }
-      }
-      lo = __reduce_min_sync(kFull, lo);
-      hi = __reduce_max_sync(kFull, hi);
-      if (lane == 0) {
-        rec[4 + 2 * g] = lo;
-        rec[5 + 2 * g] = hi;
-      }
-      if (lane == g) mine = max(mine, hi - lo);
-      for (int32_t j = gr.x; j < gr.y; ++j) {
-        const bool use = active && slen[j] > 0 && p + j < seg;
-        d[j * 32 + lane] = static_cast<uint16_t>(
-            use ? b_start(sseg[wib], staged, seg0, p + j, a_col, b_rp) - lo : 0);
-      }
-    }
-    __syncwarp();
-  }
-  if (lane == 0 && segmax > 0) atomicMax(maxima, segmax);
-  if (lane < ngroups && mine > 0) atomicMax(maxima + 1 + lane, mine);
-}
-
-// desc[pid].w = 1: the table kernel leaves the pattern's tiles alone.
-__global__ void mark_pattern_kernel(int4 *desc, int32_t pid) { desc[pid].w = 1; }
-
-// The tiles the table kernel keeps (pattern not marked), in order of
+// The tiles the table kernel keeps (of patterns not marked), in order of
 // arrival (count at *n, zeroed by the caller).
 __global__ void __launch_bounds__(256)
-table_tiles_kernel(const int4 *__restrict__ tiles, int32_t ntiles,
+table_tiles_kernel(const int4 *__restrict__ tiles, int32_t nchunks,
                    const int4 *__restrict__ desc, int4 *__restrict__ out,
                    int32_t *__restrict__ n) {
   const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   int4 t = make_int4(0, 0, 0, 0);
   bool take = false;
-  if (i < ntiles) {
+  if (i < nchunks) {
     t = tiles[i];
-    take = desc[t.z].w == 0;
+    take = t.z >= 0 && desc[t.z].w == 0;
   }
   const unsigned b = __ballot_sync(kFull, take);
   if (!b) return;
@@ -809,46 +772,29 @@ std::vector<std::pair<int, int>> jit_groups(int na, const int *len, const int32_
   return groups;
 }
 
-void launch_jit_spans(const int4 *tiles, int32_t ntiles, const int4 *desc, const uint16_t *lens,
-                      const int32_t *a_rp, const int32_t *a_col, const int32_t *b_rp,
-                      int32_t *span, int num_sms, cudaStream_t s) {
-  if (ntiles <= 0) return;
-  // a sample of at most about 1024 tiles spread over the list
-  const int32_t stride = ntiles > 1024 ? ntiles / 1024 : 1;
-  const int64_t sampled = (int64_t(ntiles) + stride - 1) / stride;
-  int64_t grid = (sampled + kBuildWarps - 1) / kBuildWarps;
-  const int64_t cap = int64_t(num_sms > 0 ? num_sms : 148) * 8;
-  if (grid > cap) grid = cap;
-  span_kernel<<<static_cast<unsigned>(grid), kBuildWarps * 32, 0, s>>>(
-      tiles, ntiles, stride, desc, lens, a_rp, a_col, b_rp, span);
-}
-
-void launch_mark_pattern(int4 *desc, int32_t pid, cudaStream_t s) {
-  mark_pattern_kernel<<<1, 1, 0, s>>>(desc, pid);
-}
-
-void launch_table_tiles(const int4 *tiles, int32_t ntiles, const int4 *desc, int4 *out,
+void launch_table_tiles(const int4 *tiles, int32_t nchunks, const int4 *desc, int4 *out,
                         int32_t *n, cudaStream_t s) {
-  if (ntiles <= 0) return;
-  table_tiles_kernel<<<(ntiles + 255) / 256, 256, 0, s>>>(tiles, ntiles, desc, out, n);
+  if (nchunks <= 0) return;
+  table_tiles_kernel<<<(nchunks + 255) / 256, 256, 0, s>>>(tiles, nchunks, desc, out, n);
 }
 
 int32_t jit_record_words(int na, int ngroups) { return record_words(na, ngroups); }
 
-void launch_jit_programs(const int4 *tiles, int32_t ntiles, int32_t na,
-                         const std::vector<std::pair<int, int>> &groups, const int2 *groups_dev,
-                         const uint16_t *lens, const int32_t *a_rp, const int32_t *a_col,
-                         const int32_t *b_rp, int32_t *prog, int2 *arange, int32_t *maxima,
-                         int num_sms, cudaStream_t s) {
-  if (ntiles <= 0) return;
-  const int32_t rw = record_words(na, static_cast<int>(groups.size()));
-  cudaMemsetAsync(prog, 0, size_t(ntiles) * size_t(rw) * sizeof(int32_t), s);
-  int64_t grid = (int64_t(ntiles) + kBuildWarps - 1) / kBuildWarps;
-  const int64_t cap = int64_t(num_sms > 0 ? num_sms : 148) * 8;
-  if (grid > cap) grid = cap;
-  program_kernel<<<static_cast<unsigned>(grid), kBuildWarps * 32, 0, s>>>(
-      tiles, ntiles, na, static_cast<int32_t>(groups.size()), groups_dev, lens, a_rp, a_col,
-      b_rp, rw, prog, arange, maxima);
+size_t tile_rank_words(int32_t nchunks) {
+  return size_t(kJitMaxPatterns) * ((size_t(nchunks) + kRankChunks - 1) / kRankChunks);
+}
+
+void launch_tile_records(int4 *tiles, int32_t nchunks, bool shifted, const TilePrograms &P,
+                         int32_t *rank, const uint16_t *lens, const int32_t *offs,
+                         const int32_t *a_rp, const int32_t *a_col, const int32_t *b_rp,
+                         int4 *desc, cudaStream_t s) {
+  if (nchunks <= 0 || P.n <= 0) return;
+  const int32_t blocks = (nchunks + kRankChunks - 1) / kRankChunks;
+  tile_rank_kernel<<<blocks, kRankChunks, 0, s>>>(tiles, nchunks, P, rank);
+  tile_rank_scan_kernel<<<1, kJitMaxPatterns * 32, 0, s>>>(blocks, P.n, rank);
+  auto kern = shifted ? record_kernel<true> : record_kernel<false>;
+  kern<<<(nchunks + kBuildWarps - 1) / kBuildWarps, kBuildWarps * 32, 0, s>>>(
+      tiles, nchunks, P, rank, blocks, lens, offs, a_rp, a_col, b_rp, desc);
 }
 
 void jit_layout(int32_t rw, int32_t seg_max, int32_t need, int32_t m, int32_t *stage_cap,

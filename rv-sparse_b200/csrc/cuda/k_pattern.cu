@@ -331,6 +331,8 @@ pat_numeric_kernel(const int32_t *__restrict__ a_rp, const int32_t *__restrict__
 
 }  // namespace
 
+int64_t pat_max_records() { return int64_t(2 * ((kPatMaxOps + 31) / 32) + kPatMaxA) * 32; }
+
 void launch_pat_select(const int32_t *rows, int32_t nrows, const int32_t *canon,
                        const int32_t *share_count, int32_t min_share, const int32_t *a_rp,
                        const int32_t *c_rp, const int32_t *mops, int32_t *pat_of,

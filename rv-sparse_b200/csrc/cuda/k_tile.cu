@@ -82,18 +82,21 @@ __device__ __forceinline__ void cp_async_wait() {
 
 // One table per pattern: warp per pattern.  desc[id] = (na, m, ops, 0), or
 // na = -1 when the pattern cannot be tiled (no table, too many outputs).
-// lens[id * 32 + j] = length of the B row of A nonzero j.
+// lens[id * 32 + j] = length of the B row of A nonzero j, offs[id * 32 + j] =
+// its column's distance from the canonical row's index.  *b_nnz = B's entries.
 __global__ void __launch_bounds__(128)
 tile_tab_kernel(int32_t npat, const int32_t *__restrict__ pat_canon,
                 const int32_t *__restrict__ psteps, const int32_t *__restrict__ a_rp,
                 const int32_t *__restrict__ a_col, const int32_t *__restrict__ b_rp,
                 const int32_t *__restrict__ c_rp, const int64_t *__restrict__ moff,
-                const uint16_t *__restrict__ map, int32_t max_out,
+                const uint16_t *__restrict__ map, int32_t max_out, int32_t b_rows,
                 uint16_t *__restrict__ tab, uint16_t *__restrict__ lens,
-                int4 *__restrict__ desc) {
+                int32_t *__restrict__ offs, int4 *__restrict__ desc,
+                int32_t *__restrict__ b_nnz) {
   __shared__ uint32_t seen[4][(kTileMaxOut + 31) / 32];
   const int wib = threadIdx.x >> 5;
   const int32_t id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *b_nnz = b_rp[b_rows];
   if (id >= npat) return;
   const int lane = lane_id();
   const int32_t row = pat_canon[id];
@@ -103,11 +106,13 @@ tile_tab_kernel(int32_t npat, const int32_t *__restrict__ pat_canon,
     if (lane == 0) desc[id] = make_int4(-1, 0, 0, 0);
     return;
   }
-  int32_t len = 0;
+  int32_t len = 0, off = 0;
   if (lane < na) {
     const int32_t k = __ldg(a_col + p0 + lane);
     len = __ldg(b_rp + k + 1) - __ldg(b_rp + k);
+    off = k - row;
   }
+  offs[size_t(id) * 32 + lane] = off;
   lens[size_t(id) * 32 + lane] = static_cast<uint16_t>(lane < na ? len : 0);
   const int32_t r8 = (len + 7) & ~7;
   const int32_t jo = warp_incl_scan(r8) - r8;  // block offset of A nonzero lane
@@ -141,109 +146,172 @@ tile_tab_kernel(int32_t npat, const int32_t *__restrict__ pat_canon,
   if (lane == 0) desc[id] = make_int4(na, m, t0, 0);
 }
 
-// Warps per block of the tile builder, and the A entries of a chunk whose B
-// row starts it stages in shared memory.
-constexpr int kBuildWarps = 4;
-constexpr int kBuildStage = 1024;
+// Warps per block of the tile builder, and the runs of chunks its blocks take
+// in turn.  The words that every tile of the largest pattern raises or counts
+// (its tiles, spans and maxima) are kept in shared memory by a block, whose
+// tiles are mostly of one pattern, and reach global memory once a block: one
+// atomic or one read of them a tile, all on a few words, was most of the
+// builder's 198 us on 40,000 chunks.
+constexpr int kBuildWarps = 16;
 
-// Warp per chunk of 32 consecutive rows (see the file comment).
-__global__ void __launch_bounds__(kBuildWarps * 32, 8)
-tile_build_kernel(int32_t n, const int32_t *__restrict__ pid_of_row,
+// Raises *word to v; most tiles find it there already.
+__device__ __forceinline__ void raise(int32_t *word, int32_t v) {
+  if (v > *reinterpret_cast<volatile int32_t *>(word)) atomicMax(word, v);
+}
+
+// Warp per chunk of 32 consecutive rows (see the file comment): tiles[chunk] =
+// (first row, lane mask, pattern, 0), pattern -1 without a tile; per pattern its tiles (pcount), its longest A segment
+// (pseg) and its largest union spans (spans[pattern * 32 * kJitMaxGroup +
+// j * kJitMaxGroup + g - 1]: end of the last B value minus first B value that
+// a tile's rows read for A nonzeros j .. j + g - 1).  counts: tiles,
+// leftovers, three maxima.  The builder is bound by load latency, so a lane
+// takes an A nonzero: with kShifted every row of a pattern is the canonical
+// row moved, the B row of A nonzero j is row + offs[j], and as B's row
+// pointers ascend a tile's range is its first row's start and its last row's
+// end.
+template <bool kShifted>
+__global__ void __launch_bounds__(kBuildWarps * 32)
+tile_build_kernel(int32_t n, int32_t per_block, const int32_t *__restrict__ pid_of_row,
                   const int4 *__restrict__ desc, const uint16_t *__restrict__ lens,
-                  const int32_t *__restrict__ a_rp, const int32_t *__restrict__ a_col,
-                  const int32_t *__restrict__ b_rp, const int32_t *__restrict__ c_rp,
-                  int4 *__restrict__ tiles, int32_t *__restrict__ ntiles,
-                  int32_t *__restrict__ lo_rows, int32_t *__restrict__ lo_ids,
-                  int32_t *__restrict__ lo_n, int32_t *__restrict__ maxima) {
-  const int64_t chunk = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t row0 = chunk * 32;
-  if (row0 >= n) return;
-  const int lane = lane_id();
-  const int32_t row = static_cast<int32_t>(row0) + lane;
-  const int32_t pid = row < n ? pid_of_row[row] : -1;
-  const unsigned peers = __match_any_sync(kFull, pid);
-  const int cnt = pid >= 0 ? __popc(peers) : 0;
-  const int leader = __ffs(peers) - 1;
-  const int key = cnt > 0 ? (cnt << 5) | (31 - leader) : 0;
-  const int best = __reduce_max_sync(kFull, key);
-  bool ok = (best >> 5) >= kTileMinRows;
-  const int32_t bpid = __shfl_sync(kFull, pid, 31 - (best & 31));
-  const bool in = ok && pid == bpid;
-  int4 d = make_int4(-1, 0, 0, 0);
-  int32_t seg = 0, need = 0;
-  if (ok) {
-    d = desc[bpid];
-    ok = d.x > 0;
+                  const int32_t *__restrict__ offs, const int32_t *__restrict__ a_rp,
+                  const int32_t *__restrict__ a_col, const int32_t *__restrict__ b_rp,
+                  const int32_t *__restrict__ c_rp, int4 *__restrict__ tiles,
+                  int32_t *__restrict__ pcount, int32_t *__restrict__ pseg,
+                  int32_t *__restrict__ spans, int32_t *__restrict__ lo_rows,
+                  int32_t *__restrict__ lo_ids, int32_t *__restrict__ counts) {
+  constexpr int kSpans = 32 * kJitMaxGroup;
+  __shared__ int32_t s_left[kBuildWarps], s_span[kSpans], s_max[3];
+  __shared__ int32_t s_main, s_seg, s_own, s_tiles;
+  const int lane = lane_id(), wib = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < kSpans; i += blockDim.x) s_span[i] = 0;
+  if (threadIdx.x < 3) s_max[threadIdx.x] = 0;
+  if (threadIdx.x == 0) {
+    s_main = -1;
+    s_seg = 0;
+    s_own = 0;
+    s_tiles = 0;
   }
-  if (ok) {
-    const int32_t last = row0 + 32 < n ? static_cast<int32_t>(row0) + 32 : n;
-    seg = a_rp[last] - a_rp[row0];
-    bool fits = seg <= kTileASegMax;
-    if (in) fits = fits && (c_rp[row + 1] - c_rp[row] == d.y) && (a_rp[row + 1] - a_rp[row] == d.x);
-    ok = __all_sync(kFull, fits);
-  }
-  if (ok) {
-    // the chunk's B row starts: a segment of up to kBuildStage entries is
-    // staged in shared memory with coalesced loads of a_col (16 a lane in
-    // flight, then their gathers), a longer one read through a_col (4 KB a
-    // warp and at most 64 registers keep 32 warps an SM resident: this
-    // kernel is bound by load latency)
-    __shared__ int32_t sseg[kBuildWarps][kBuildStage];
-    int32_t *const sb = sseg[(threadIdx.x >> 5) % kBuildWarps];
-    const int32_t seg0 = a_rp[row0];
-    const bool staged = seg <= kBuildStage;
-    if (staged) {
-      for (int32_t i0 = 0; i0 < seg; i0 += 512) {
-        int32_t c[16];
-#pragma unroll
-        for (int u = 0; u < 16; ++u) {
-          const int32_t i = i0 + u * 32 + lane;
-          c[u] = i < seg ? __ldg(a_col + seg0 + i) : 0;
+  __syncthreads();
+  const int64_t nchunks = (int64_t(n) + 31) / 32;
+  for (int it = 0; it < per_block; ++it) {
+    const int64_t chunk = (int64_t(blockIdx.x) * per_block + it) * kBuildWarps + wib;
+    const int64_t row0 = chunk * 32;
+    const int64_t row = row0 + lane;
+    const int32_t pid = row < n ? pid_of_row[row] : -1;
+    const unsigned peers = __match_any_sync(kFull, pid);
+    const int cnt = pid >= 0 ? __popc(peers) : 0;
+    const int leader = __ffs(peers) - 1;
+    const int key = cnt > 0 ? (cnt << 5) | (31 - leader) : 0;
+    const int best = __reduce_max_sync(kFull, key);
+    bool ok = (best >> 5) >= kTileMinRows;
+    const int32_t bpid = __shfl_sync(kFull, pid, 31 - (best & 31));
+    const bool in = ok && pid == bpid;
+    int4 d = make_int4(-1, 0, 0, 0);
+    if (ok) {
+      d = desc[bpid];
+      ok = d.x > 0;
+    }
+    int32_t seg = 0;
+    if (ok) {
+      const int64_t last = row0 + 32 < n ? row0 + 32 : n;
+      seg = a_rp[last] - a_rp[row0];
+      bool fits = seg <= kTileASegMax;
+      if (in)
+        fits = fits && (c_rp[row + 1] - c_rp[row] == d.y) && (a_rp[row + 1] - a_rp[row] == d.x);
+      ok = __all_sync(kFull, fits);
+    }
+    const unsigned inmask = __ballot_sync(kFull, ok && in);
+    int32_t lo = INT_MAX, hi = INT_MIN;  // of A nonzero `lane` over the tile's rows
+    if (ok) {
+      const int first = __ffs(inmask) - 1, last = 31 - __clz(inmask);
+      const int32_t len = lane < d.x ? lens[size_t(bpid) * 32 + lane] : 0;
+      if (kShifted) {
+        if (lane < d.x) {
+          const int64_t k = row0 + offs[size_t(bpid) * 32 + lane];
+          lo = __ldg(b_rp + k + first);
+          hi = __ldg(b_rp + k + last) + len;
         }
-#pragma unroll
-        for (int u = 0; u < 16; ++u) {
-          const int32_t i = i0 + u * 32 + lane;
-          c[u] = i < seg ? __ldg(b_rp + c[u]) : 0;
+      } else {
+        const int32_t p = in ? a_rp[row] : 0;
+        for (int32_t j = 0; j < d.x; ++j) {
+          const int32_t r = in ? __ldg(b_rp + __ldg(a_col + p + j)) : 0;
+          const int32_t l = __reduce_min_sync(kFull, in ? r : INT_MAX);
+          const int32_t h = __reduce_max_sync(kFull, in ? r : INT_MIN);
+          if (lane == j) {
+            lo = l;
+            hi = h + len;
+          }
         }
+      }
+      const int32_t need = lane < d.x ? hi - (lo & ~3) + 8 : 0;
+      const int32_t stage = __reduce_max_sync(kFull, need);
+      ok = stage <= kTileStageMax;
+      if (ok) {
+        int32_t first_pid = 0;
+        if (lane == 0) {
+          first_pid = atomicCAS(&s_main, -1, bpid);
+          if (first_pid == -1) first_pid = bpid;
+        }
+        const bool own = __shfl_sync(kFull, first_pid, 0) == bpid;
+        if (len == 0) {  // an empty B row reads nothing
+          lo = INT_MAX;
+          hi = INT_MIN;
+        }
+        int32_t ul = lo, uh = hi;
 #pragma unroll
-        for (int u = 0; u < 16; ++u) {
-          const int32_t i = i0 + u * 32 + lane;
-          if (i < seg) sb[i] = c[u];
+        for (int g = 1; g <= kJitMaxGroup; ++g) {
+          const int at = lane * kJitMaxGroup + g - 1;
+          if (lane + g <= d.x && uh > ul)
+            raise(own ? s_span + at : spans + size_t(bpid) * kSpans + at, uh - ul);
+          const int32_t l = __shfl_down_sync(kFull, lo, g), h = __shfl_down_sync(kFull, hi, g);
+          ul = min(ul, l);
+          uh = max(uh, h);
+        }
+        if (lane == 0) {
+          raise(s_max + kStageNeedWord, stage);
+          raise(s_max + kASegWord, seg);
+          raise(s_max + kMaxOutWord, d.y);
+          raise(own ? &s_seg : pseg + bpid, a_rp[row0 + last + 1] - a_rp[row0 + first]);
+          atomicAdd(own ? &s_own : pcount + bpid, 1);
+          atomicAdd(&s_tiles, 1);
         }
       }
     }
-    __syncwarp();
-    const int32_t p = in ? a_rp[row] - seg0 : 0;
-    for (int32_t j = 0; j < d.x; ++j) {
-      const int32_t lj = lens[size_t(bpid) * 32 + j];
-      const int32_t rp =
-          in ? (staged ? sb[p + j] : __ldg(b_rp + __ldg(a_col + seg0 + p + j))) : 0;
-      const int32_t lo = __reduce_min_sync(kFull, in ? rp : INT_MAX);
-      const int32_t hi = __reduce_max_sync(kFull, in ? rp + lj : INT_MIN);
-      need = max(need, hi - (lo & ~3) + 8);
+    // leftovers: table rows that are not in the tile
+    const bool left = pid >= 0 && !(ok && in);
+    const unsigned lmask = __ballot_sync(kFull, left);
+    if (lane == 0) {
+      s_left[wib] = __popc(lmask);
+      if (chunk < nchunks)
+        tiles[chunk] = make_int4(static_cast<int32_t>(row0), static_cast<int32_t>(inmask),
+                                 ok ? bpid : -1, 0);
     }
-    ok = need <= kTileStageMax;
-  }
-  const unsigned tmask = __ballot_sync(kFull, ok && in);
-  if (ok && lane == 0) {
-    const int32_t t = atomicAdd(ntiles, 1);
-    tiles[t] = make_int4(static_cast<int32_t>(row0), static_cast<int32_t>(tmask), bpid, 0);
-    atomicMax(maxima + kStageNeedWord, need);
-    atomicMax(maxima + kASegWord, seg);
-    atomicMax(maxima + kMaxOutWord, d.y);
-  }
-  // leftovers: table rows that are not in the tile
-  const bool left = pid >= 0 && !(ok && in);
-  const unsigned lmask = __ballot_sync(kFull, left);
-  if (lmask) {
-    int32_t base = 0;
-    if (lane == 0) base = atomicAdd(lo_n, __popc(lmask));
-    base = __shfl_sync(kFull, base, 0);
+    __syncthreads();
+    if (wib == 0) {
+      const int32_t nl = lane < kBuildWarps ? s_left[lane] : 0;
+      const int32_t incl = warp_incl_scan(nl);
+      int32_t lbase = 0;
+      if (lane == 31 && incl) lbase = atomicAdd(counts + 1, incl);
+      lbase = __shfl_sync(kFull, lbase, 31);
+      if (lane < kBuildWarps) s_left[lane] = lbase + incl - nl;
+    }
+    __syncthreads();
     if (left) {
-      const int32_t at = base + __popc(lmask & lanemask_lt());
-      lo_rows[at] = row;
+      const int at = s_left[wib] + __popc(lmask & lanemask_lt());
+      lo_rows[at] = static_cast<int32_t>(row);
       lo_ids[at] = pid;
     }
+    __syncthreads();  // the next chunks overwrite s_left
+  }
+  const int32_t main_pid = s_main;
+  if (main_pid < 0) return;
+  for (int i = threadIdx.x; i < kSpans; i += blockDim.x)
+    if (s_span[i]) raise(spans + size_t(main_pid) * kSpans + i, s_span[i]);
+  if (threadIdx.x < 3) raise(counts + 2 + threadIdx.x, s_max[threadIdx.x]);
+  if (threadIdx.x == 0) {
+    raise(pseg + main_pid, s_seg);
+    atomicAdd(pcount + main_pid, s_own);
+    atomicAdd(counts, s_tiles);
   }
 }
 
@@ -439,23 +507,30 @@ void launch_tile_list(int32_t n, const int32_t *pid_of_row, int32_t *rows, int32
 void launch_tile_tab(int32_t npat, const int32_t *pat_canon, const int32_t *psteps,
                      const int32_t *a_rp, const int32_t *a_col, const int32_t *b_rp,
                      const int32_t *c_rp, const int64_t *moff, const uint16_t *map,
-                     uint16_t *tab, uint16_t *lens, int4 *desc, cudaStream_t s) {
+                     int32_t b_rows, uint16_t *tab, uint16_t *lens, int32_t *offs, int4 *desc,
+                     int32_t *b_nnz, cudaStream_t s) {
   if (npat <= 0) return;
   tile_tab_kernel<<<(npat + 3) / 4, 128, 0, s>>>(npat, pat_canon, psteps, a_rp, a_col, b_rp,
-                                                 c_rp, moff, map, kTileMaxOut, tab, lens, desc);
+                                                 c_rp, moff, map, kTileMaxOut, b_rows, tab,
+                                                 lens, offs, desc, b_nnz);
 }
 
-void launch_tile_build(int32_t n, const int32_t *pid_of_row, const int4 *desc,
-                       const uint16_t *lens, const int32_t *a_rp, const int32_t *a_col,
-                       const int32_t *b_rp, const int32_t *c_rp, int4 *tiles, int32_t *ntiles,
-                       int32_t *lo_rows, int32_t *lo_ids, int32_t *lo_n, int32_t *maxima,
+void launch_tile_build(int32_t n, bool shifted, const int32_t *pid_of_row, const int4 *desc,
+                       const uint16_t *lens, const int32_t *offs, const int32_t *a_rp,
+                       const int32_t *a_col, const int32_t *b_rp, const int32_t *c_rp,
+                       int4 *tiles, int32_t *pcount, int32_t *pseg, int32_t *spans,
+                       int32_t *lo_rows, int32_t *lo_ids, int32_t *counts, int num_sms,
                        cudaStream_t s) {
   if (n <= 0) return;
-  const int64_t chunks = (int64_t(n) + 31) / 32;
-  const int64_t grid = (chunks + kBuildWarps - 1) / kBuildWarps;
-  tile_build_kernel<<<static_cast<unsigned>(grid), kBuildWarps * 32, 0, s>>>(
-      n, pid_of_row, desc, lens, a_rp, a_col, b_rp, c_rp, tiles, ntiles, lo_rows, lo_ids, lo_n,
-      maxima);
+  // four blocks of 512 threads an SM, each a run of chunks
+  const int64_t steps = ((int64_t(n) + 31) / 32 + kBuildWarps - 1) / kBuildWarps;
+  const int64_t blocks = int64_t(num_sms > 0 ? num_sms : 148) * 4;
+  const int64_t per_block = (steps + blocks - 1) / blocks;
+  const int64_t grid = (steps + per_block - 1) / per_block;
+  auto kern = shifted ? tile_build_kernel<true> : tile_build_kernel<false>;
+  kern<<<static_cast<unsigned>(grid), kBuildWarps * 32, 0, s>>>(
+      n, static_cast<int32_t>(per_block), pid_of_row, desc, lens, offs, a_rp, a_col, b_rp, c_rp, tiles, pcount, pseg, spans,
+      lo_rows, lo_ids, counts);
 }
 
 size_t tile_smem_per_warp(int32_t stage_need, int32_t a_seg, int32_t max_out,

@@ -350,6 +350,8 @@ void launch_pat_select(const int32_t *rows, int32_t nrows, const int32_t *canon,
                        const int32_t *c_rp, const int32_t *mops, int32_t *pat_of,
                        int32_t *pat_canon, int32_t *pat_cap, int32_t *npat, int32_t *maxima,
                        cudaStream_t s);
+// The most records one table can take.
+int64_t pat_max_records();
 // Build: the npat tables at rec + pat_off[id]; psteps[id] = steps, or -1.
 void launch_pat_build(int32_t npat, const int32_t *pat_canon, const int32_t *a_rp,
                       const int32_t *a_col, const int32_t *b_rp, const int32_t *c_rp,
@@ -376,22 +378,30 @@ void launch_pat_numeric(const Operands &op, const int64_t *ops, const int32_t *p
 // kernel; uint16 entries per pattern in
 // the tile tables (tab has npat * tile_tab_stride() entries).
 constexpr int kTileKernelWarps = 2;
+// A nonzeros staged together by a pattern kernel (k_jit.cu): runs of at most
+// this many.
+constexpr int kJitMaxGroup = 8;
 int32_t tile_tab_stride();
-// Per pattern: its table, B row lengths (lens[id * 32 + j]) and desc[id] =
-// (na, m, ops, 0), or na = -1 when the pattern is not tiled.
+// Per pattern: its table, B row lengths (lens[id * 32 + j]), column offsets of
+// its canonical row (offs[id * 32 + j]) and desc[id] = (na, m, ops, 0), or
+// na = -1 when the pattern is not tiled; *b_nnz = B's entries.
 void launch_tile_tab(int32_t npat, const int32_t *pat_canon, const int32_t *psteps,
                      const int32_t *a_rp, const int32_t *a_col, const int32_t *b_rp,
                      const int32_t *c_rp, const int64_t *moff, const uint16_t *map,
-                     uint16_t *tab, uint16_t *lens, int4 *desc, cudaStream_t s);
+                     int32_t b_rows, uint16_t *tab, uint16_t *lens, int32_t *offs, int4 *desc,
+                     int32_t *b_nnz, cudaStream_t s);
 // Tiles of the n rows (pid_of_row: pattern of each table row, -1 for the
-// others): tiles[*ntiles] = (first row, lane mask, pattern, 0); the table rows
-// no tile takes go to lo_rows / lo_ids (count *lo_n).  maxima (3 words,
-// zeroed by the caller): stage floats, A segment entries and C row the tile
-// kernel must hold.
-void launch_tile_build(int32_t n, const int32_t *pid_of_row, const int4 *desc,
-                       const uint16_t *lens, const int32_t *a_rp, const int32_t *a_col,
-                       const int32_t *b_rp, const int32_t *c_rp, int4 *tiles, int32_t *ntiles,
-                       int32_t *lo_rows, int32_t *lo_ids, int32_t *lo_n, int32_t *maxima,
+// others; shifted: a pattern's rows are its canonical row moved), one per
+// chunk of 32 rows: tiles[chunk] = (first row, lane mask, pattern or -1, 0);
+// the table rows no tile takes go to lo_rows / lo_ids.  counts[0] tiles, [1] leftovers, [2..4] the stage floats, A segment
+// entries and C row the tile kernel must hold; per pattern its tiles, its
+// longest A segment and its union spans (32 * kJitMaxGroup; see k_tile.cu).
+// counts, pcount, pseg and spans are zeroed by the caller.
+void launch_tile_build(int32_t n, bool shifted, const int32_t *pid_of_row, const int4 *desc,
+                       const uint16_t *lens, const int32_t *offs, const int32_t *a_rp,
+                       const int32_t *a_col, const int32_t *b_rp, const int32_t *c_rp,
+                       int4 *tiles, int32_t *pcount, int32_t *pseg, int32_t *spans,
+                       int32_t *lo_rows, int32_t *lo_ids, int32_t *counts, int num_sms,
                        cudaStream_t s);
 // rows / ids (count at *count, zeroed by the caller): every row with
 // pid_of_row[row] >= 0 and its pattern.
@@ -430,8 +440,6 @@ void launch_persist_numeric(const Operands &op, const int64_t *ops, const Persis
                             cudaStream_t s);
 
 // ---- k_jit.cu --------------------------------------------------------------
-// A nonzeros staged together by a pattern kernel: runs of at most this many.
-constexpr int kJitMaxGroup = 8;
 // One pattern for a compiled kernel (see k_jit.cu): na A nonzeros, B row
 // lengths len[j], slot[t] = output position of flattened product t, m
 // outputs, groups = [first, end) runs of A nonzeros whose B values are
@@ -447,35 +455,41 @@ struct JitRequest {
 // returns how many compiled.
 int jit_pattern_kernels(std::vector<JitRequest> &reqs);
 void jit_stats(int32_t *compiles, double *ms);
-// The groups of a pattern from its union spans (launch_jit_spans): runs of
+// The groups of a pattern from its union spans (launch_tile_build): runs of
 // A nonzeros grown while the next one adds less than half its own span and
 // the union stays within max_span floats.  *stage_need = the largest union.
 std::vector<std::pair<int, int>> jit_groups(int na, const int *len, const int32_t *span,
                                             int32_t max_span, int32_t *stage_need);
-// span[j0 * kJitMaxGroup + g - 1] = the largest B range (floats) that one of
-// a sample of the tiles reads for A nonzeros j0 .. j0 + g - 1 (span zeroed by
-// the caller; desc->x = the pattern's A nonzeros, nothing done unless in
-// 1..32).
-void launch_jit_spans(const int4 *tiles, int32_t ntiles, const int4 *desc, const uint16_t *lens,
-                      const int32_t *a_rp, const int32_t *a_col, const int32_t *b_rp,
-                      int32_t *span, int num_sms, cudaStream_t s);
-// Marks pattern pid's tiles for the table kernel to skip (desc[pid].w = 1).
-void launch_mark_pattern(int4 *desc, int32_t pid, cudaStream_t s);
-// out[*n] = the tiles whose pattern is not marked (*n zeroed by the caller).
-void launch_table_tiles(const int4 *tiles, int32_t ntiles, const int4 *desc, int4 *out,
+// out[*n] = the tiles whose pattern has no compiled kernel (desc[pid].w == 0;
+// *n zeroed by the caller).
+void launch_table_tiles(const int4 *tiles, int32_t nchunks, const int4 *desc, int4 *out,
                         int32_t *n, cudaStream_t s);
 // Words of one tile record of a pattern kernel (na A nonzeros, ngroups
 // staging groups).
 int32_t jit_record_words(int na, int ngroups);
-// The tile records of a pattern (see k_jit.cu): prog[ntiles * record words],
-// arange[ntiles] = the A range of each tile, maxima[0] = the longest,
-// maxima[1 + g] = group g's largest B range (zeroed by the caller);
-// groups_dev = the groups as int2 on the device.
-void launch_jit_programs(const int4 *tiles, int32_t ntiles, int32_t na,
-                         const std::vector<std::pair<int, int>> &groups, const int2 *groups_dev,
-                         const uint16_t *lens, const int32_t *a_rp, const int32_t *a_col,
-                         const int32_t *b_rp, int32_t *prog, int2 *arange, int32_t *maxima,
-                         int num_sms, cudaStream_t s);
+// The compiled patterns of a tile set: pattern pid of na A nonzeros, group[j]
+// the staging group of A nonzero j (of ng; kNoGroup outside them), its records
+// (rw words a tile) and the tiles' A ranges.
+constexpr int kJitMaxPatterns = 12;
+constexpr uint8_t kNoGroup = 255;
+struct TileProgram {
+  int32_t *prog;
+  int2 *arange;
+  int32_t pid, na, ng, rw;
+  uint8_t group[32];
+};
+struct TilePrograms {
+  TileProgram p[kJitMaxPatterns];
+  int32_t n = 0;
+};
+// Their tile records (see k_jit.cu), in row order, from the tiles of
+// launch_tile_build (whose last words it uses); sets desc[pid].w = 1, which
+// makes the table kernel skip their tiles.  rank: tile_rank_words(nchunks).
+size_t tile_rank_words(int32_t nchunks);
+void launch_tile_records(int4 *tiles, int32_t nchunks, bool shifted, const TilePrograms &P,
+                         int32_t *rank, const uint16_t *lens, const int32_t *offs,
+                         const int32_t *a_rp, const int32_t *a_col, const int32_t *b_rp,
+                         int4 *desc, cudaStream_t s);
 // Shared memory of one warp of a pattern kernel, in floats: two tile buffers
 // (record + A values) of *abuf_floats and two B stage buffers of *stage_cap
 // (the largest B range `need` plus widening; room for 16 output rows).

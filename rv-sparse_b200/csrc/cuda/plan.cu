@@ -106,19 +106,18 @@ constexpr int kPatCountWords = 4 + kNumClasses;
 namespace rvsp {
 // Row tiles over one set of term-table patterns (k_tile.cu): per pattern its
 // tile table, B row lengths and shape; per row its pattern (pid, -1 for rows
-// outside the set); the tiles and the pattern rows left to the warp-per-row
-// table kernel (lo_rows / lo_ids); for the shift classes also every pattern
-// row (all_rows / all_ids, for when tiles are off).
+// outside the set); the tiles, one entry per chunk of 32 rows; the pattern
+// rows left to the warp-per-row table kernel (lo_rows / lo_ids); for the shift
+// classes also every pattern row (all_rows / all_ids, listed when tiles are
+// off).
 struct JitPattern {
   void *kernel = nullptr;
-  DevArray<int4> tiles;
   DevArray<int32_t> prog;  // tile records (k_jit.cu)
   DevArray<int2> arange;   // per tile its A range
   DevArray<int32_t> head;  // the launch's tile queue
   int32_t n = 0, m = 0, stage_cap = 0, abuf_floats = 0, work_floats = 0;
   int grid = 0;
   void release() {
-    tiles.release();
     prog.release();
     arange.release();
     head.release();
@@ -127,19 +126,24 @@ struct JitPattern {
 struct TileBuild {
   std::vector<JitPattern> jit;   // patterns with their own kernel (k_jit.cu)
   std::vector<JitPattern> pool;  // device arrays of earlier builds, for reuse
-  DevArray<int32_t> jwords;      // per chosen pattern: spans, record extent
-  DevArray<int2> jgroups;        // per chosen pattern: its staging groups
-  HostArray staging;             // host side of the builds' transfers
+  HostArray staging;             // host side of the build's read-back
   int ready = 0;
+  bool listed = false;  // all_rows / all_ids hold the current analysis's rows
   int32_t n_tiles = 0, n_lo = 0, stage = 0, aseg = 0, max_out = 0, b_nnz = 0;
+  // counts, then per pattern its tiles, its longest A segment and its union
+  // spans: one array, zeroed and read back whole
+  DevArray<int32_t> counts;
   DevArray<uint16_t> tab, lens;
+  DevArray<int32_t> offs, rank;
   DevArray<int4> desc, tiles;
-  DevArray<int4> table;  // the tiles left to the table kernel, when patterns are compiled
+  DevArray<int4> table;  // the tiles left to the table kernel
   int32_t n_table = 0;
-  DevArray<int32_t> pid, lo_rows, lo_ids, counts, all_rows, all_ids;
+  DevArray<int32_t> pid, lo_rows, lo_ids, all_rows, all_ids;
   void release() {
     tab.release();
     lens.release();
+    offs.release();
+    rank.release();
     desc.release();
     tiles.release();
     table.release();
@@ -154,8 +158,6 @@ struct TileBuild {
     for (auto &j : pool) j.release();
     jit.clear();
     pool.clear();
-    jwords.release();
-    jgroups.release();
     staging.release();
     ready = 0;
   }
@@ -388,7 +390,8 @@ struct Lanes {
   rvsp_cuda_plan *pl;
   cudaStream_t s;
   bool forked = false;
-  bool used[rvsp_cuda_plan::kSide] = {};
+  bool used[rvsp_cuda_plan::kSide] = {};    // has work to join
+  bool behind[rvsp_cuda_plan::kSide] = {};  // waits for the last fork
   int turn = 0;
   Lanes(rvsp_cuda_plan *p, cudaStream_t st, bool want) : pl(p), s(st) {
     forked = want && side_streams(p, st) && cudaEventRecord(p->fork_ev, st) == cudaSuccess;
@@ -398,11 +401,18 @@ struct Lanes {
     if (!forked) return s;
     const int i = turn;
     turn = (turn + 1) % rvsp_cuda_plan::kSide;
-    if (!used[i]) {
+    if (!behind[i]) {
       if (cudaStreamWaitEvent(pl->side[i], pl->fork_ev, 0) != cudaSuccess) return s;
-      used[i] = true;
+      behind[i] = used[i] = true;
     }
     return pl->side[i];
+  }
+  // What next() hands out from here on also comes after the work queued on
+  // the caller's stream so far; work already on a side stream stays there.
+  void refork() {
+    if (!forked) return;
+    if (cudaEventRecord(pl->fork_ev, s) != cudaSuccess) return join();
+    for (bool &b : behind) b = false;
   }
   void join() {
     if (!forked) return;
@@ -410,7 +420,7 @@ struct Lanes {
       if (!used[i]) continue;
       cudaEventRecord(pl->join_ev[i], pl->side[i]);
       cudaStreamWaitEvent(s, pl->join_ev[i], 0);
-      used[i] = false;
+      used[i] = behind[i] = false;
     }
     forked = false;
   }
@@ -1369,311 +1379,226 @@ constexpr size_t kTileTablesMaxBytes = size_t(256) << 20;
 // the kJitMaxPatterns largest of them, when their rows have at most
 // kJitMaxOut outputs (one register each).
 constexpr int32_t kJitMinTiles = 128;
-constexpr int kJitMaxPatterns = 12;
 constexpr int32_t kJitMaxOut = 160;
 // Largest B range (floats) one stage buffer of a pattern kernel takes.
 constexpr int32_t kJitMaxSpan = 4096;
 
-// Compiled kernels for the patterns that cover the most tiles.  The tile
-// list is read back once to count each pattern's tiles and list them in row
-// order; then, for all the chosen patterns at once, the union spans of runs
-// of their A nonzeros are measured on a sample of their tiles (one round
-// trip with their tables), the staging groups chosen and the kernels
-// compiled side by side (k_jit.cu), their tile records built (one round
-// trip for the records' A extents and every group's largest B range), and
-// their tiles marked so the table kernel skips them (one round trip for the
-// table kernel's own list).  A pattern whose compile fails stays on the
-// table kernel.  The device arrays of earlier builds are kept and reused;
-// every transfer goes through page-locked staging.  Synchronizes `s`.
-cudaError_t build_pattern_kernels(rvsp_cuda_plan *p, cudaStream_t s, const Operands &op,
-                                  int32_t npat, TileBuild &tb) {
-  for (auto &j : tb.jit) tb.pool.push_back(j);
-  tb.jit.clear();
-  // per chosen pattern: spans (32 x kJitMaxGroup words), its records' A
-  // extent and groups' B ranges
-  constexpr size_t W = size_t(32 * kJitMaxGroup) + 2;
-  const size_t KM = size_t(kJitMaxPatterns);
-  const int32_t stride = tile_tab_stride();
-  const size_t nt = static_cast<size_t>(tb.n_tiles), np = static_cast<size_t>(npat);
-  // the staging layout: tiles read back, desc, lens, tables, sorted tile
-  // lists, words, groups (16-byte aligned pieces)
-  auto up16 = [](size_t x) { return (x + 15) & ~size_t(15); };
-  const size_t o_tiles = 0, o_desc = o_tiles + up16(nt * sizeof(int4));
-  const size_t o_lens = o_desc + up16(np * sizeof(int4));
-  const size_t o_tabs = o_lens + up16(np * 32 * sizeof(uint16_t));
-  const size_t o_lists = o_tabs + up16(KM * size_t(stride) * sizeof(uint16_t));
-  const size_t o_words = o_lists + up16(nt * sizeof(int4));
-  const size_t o_groups = o_words + up16(KM * W * sizeof(int32_t));
-  const size_t total = o_groups + up16(KM * 32 * sizeof(int2));
-  if (tb.staging.reserve(total) != cudaSuccess) {
-    cudaGetLastError();
-    return cudaSuccess;
-  }
-  int4 *const tiles = reinterpret_cast<int4 *>(tb.staging.p + o_tiles);
-  int4 *const desc = reinterpret_cast<int4 *>(tb.staging.p + o_desc);
-  uint16_t *const lens = reinterpret_cast<uint16_t *>(tb.staging.p + o_lens);
-  uint16_t *const tabs = reinterpret_cast<uint16_t *>(tb.staging.p + o_tabs);
-  int4 *const lists = reinterpret_cast<int4 *>(tb.staging.p + o_lists);
-  int32_t *const words = reinterpret_cast<int32_t *>(tb.staging.p + o_words);
-  int2 *const gh = reinterpret_cast<int2 *>(tb.staging.p + o_groups);
-  cudaError_t e = cudaMemcpyAsync(tiles, tb.tiles.p, nt * sizeof(int4), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(desc, tb.desc.p, np * sizeof(int4), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(lens, tb.lens.p, np * 32 * sizeof(uint16_t), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return e;
-  std::vector<int32_t> count(np, 0);
-  for (size_t i = 0; i < nt; ++i)
-    if (tiles[i].z >= 0 && tiles[i].z < npat) ++count[size_t(tiles[i].z)];
-  std::vector<int32_t> order;
-  for (int32_t id = 0; id < npat; ++id)
-    if (count[size_t(id)] >= kJitMinTiles) order.push_back(id);
-  std::sort(order.begin(), order.end(),
-            [&](int32_t a, int32_t b) { return count[size_t(a)] > count[size_t(b)]; });
-  if (order.size() > KM) order.resize(KM);
-  if (order.empty()) return cudaSuccess;
+constexpr int kTileCountWords = 8;  // tiles, leftovers, 3 maxima, b_nnz, table tiles, all rows
+constexpr int kCountBnnz = 5, kCountTable = 6, kCountAll = 7;
+constexpr size_t kSpanWords = size_t(32) * kJitMaxGroup;  // a pattern's union spans
+// Patterns whose spans and tables are read back with the counts, before it is
+// known which of them get a kernel (1 MB at most).
+constexpr int32_t kReadAllPatterns = 256;
+
+// Compiled kernels for the patterns that cover the most tiles, from what the
+// tile builder measured (on the host): the staging groups are chosen from the
+// union spans, the kernels compiled side by side (k_jit.cu; a structure seen
+// before finds them compiled) and the tile records of all of them queued as
+// one launch.  A pattern whose compile fails stays on the table kernel.  The
+// device arrays of earlier builds are kept and reused.
+void build_pattern_kernels(rvsp_cuda_plan *p, cudaStream_t s, const Operands &op, bool shifted,
+                           const std::vector<int32_t> &order, const int32_t *pcount,
+                           const int32_t *pseg, const int4 *desc, const uint16_t *lens,
+                           const std::vector<const int32_t *> &spans,
+                           const std::vector<const uint16_t *> &tabs, TileBuild &tb) {
   const size_t K = order.size();
-  if (tb.jwords.reserve(K * W) != cudaSuccess || tb.jgroups.reserve(K * 32) != cudaSuccess) {
-    cudaGetLastError();
-    return cudaSuccess;
-  }
-  std::vector<JitPattern> cand(K);
-  auto give_back = [&tb](JitPattern &jp) { tb.pool.push_back(jp); jp = JitPattern(); };
-  // each chosen pattern's tiles in order of their first row (one tile per
-  // chunk of 32 rows: a counting pass over the chunks), so that the
-  // persistent warps, which take tiles in list order, work on neighbouring
-  // rows at any one time and their B ranges stay in L2 between tiles
-  std::vector<int32_t> kof(np, -1);
-  for (size_t k = 0; k < K; ++k) kof[size_t(order[k])] = static_cast<int32_t>(k);
-  std::vector<size_t> lbeg(K + 1, 0), lfill(K, 0);
-  for (size_t k = 0; k < K; ++k) lbeg[k + 1] = lbeg[k] + size_t(count[size_t(order[k])]);
-  {
-    const int64_t nchunks = (int64_t(p->a_rows) + 31) / 32;
-    std::vector<int32_t> at(static_cast<size_t>(nchunks), -1);
-    for (size_t i = 0; i < nt; ++i) {
-      const int64_t c = int64_t(tiles[i].x) / 32;
-      if (c >= 0 && c < nchunks) at[size_t(c)] = static_cast<int32_t>(i);
+  std::vector<JitRequest> reqs(K);
+  std::vector<int32_t> need(K, 0);
+  for (size_t k = 0; k < K; ++k) {
+    const int4 d = desc[size_t(order[k])];
+    if (d.x <= 0 || d.x > 32 || d.y <= 0 || d.y > kJitMaxOut) continue;
+    JitRequest rq;
+    rq.na = d.x;
+    rq.m = d.y;
+    int32_t off = 0;
+    rq.slot.reserve(size_t(d.z));
+    for (int j = 0; j < d.x; ++j) {
+      rq.len[j] = lens[size_t(order[k]) * 32 + j];
+      for (int e = 0; e < rq.len[j]; ++e) rq.slot.push_back(tabs[k][off + e] & 0x7fff);
+      off += (rq.len[j] + 7) & ~7;
     }
-    for (const int32_t i : at) {
-      if (i < 0) continue;
-      const int4 &t = tiles[size_t(i)];
-      if (t.z < 0 || t.z >= npat || kof[size_t(t.z)] < 0) continue;
-      const size_t k = size_t(kof[size_t(t.z)]);
-      lists[lbeg[k] + lfill[k]++] = t;
-    }
+    rq.groups = jit_groups(d.x, rq.len, spans[k], kJitMaxSpan, &need[k]);
+    // (offsets into a group's B range are 16 bits)
+    if (!rq.groups.empty() && need[k] > 0 && need[k] <= kJitMaxSpan) reqs[k] = std::move(rq);
   }
-  for (size_t k = 0; k < K && e == cudaSuccess; ++k)
-    e = cudaMemcpyAsync(tabs + k * size_t(stride), tb.tab.p + size_t(order[k]) * stride,
-                        size_t(stride) * sizeof(uint16_t), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(tb.jwords.p, 0, K * W * sizeof(int32_t), s);
-  // the patterns' span and record kernels are small and bound by latency:
-  // they run side by side on the plan's side streams
-  Lanes ln(p, s, true);
-  for (size_t k = 0; k < K && e == cudaSuccess; ++k) {
-    const int32_t id = order[k];
-    JitPattern &jp = cand[k];
-    // the device arrays of an earlier build: the smallest whose tile
-    // capacity holds this pattern's tiles, else the largest (so that a
-    // repeated analysis of the same structure allocates nothing)
+  jit_pattern_kernels(reqs);
+  int dev_max = 0;
+  cudaDeviceGetAttribute(&dev_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, p->device);
+  TilePrograms P;
+  for (size_t k = 0; k < K; ++k) {
+    const JitRequest &rq = reqs[k];
+    if (!rq.kernel) continue;
+    const int32_t n = pcount[order[k]], rw = jit_record_words(rq.na, int(rq.groups.size()));
+    // the arrays of an earlier build: the smallest whose tile capacity holds
+    // this pattern's tiles, else the largest (so that a repeated analysis of
+    // the same structure allocates nothing)
+    JitPattern jp;
     if (!tb.pool.empty()) {
-      const size_t need = lfill[k];
       size_t best = 0;
       for (size_t q = 1; q < tb.pool.size(); ++q) {
-        const size_t c = tb.pool[q].tiles.cap, bc = tb.pool[best].tiles.cap;
-        const bool f = c >= need, bf = bc >= need;
+        const size_t c = tb.pool[q].arange.cap, bc = tb.pool[best].arange.cap;
+        const bool f = c >= size_t(n), bf = bc >= size_t(n);
         if ((f && (!bf || c < bc)) || (!f && !bf && c > bc)) best = q;
       }
       jp = tb.pool[best];
       tb.pool.erase(tb.pool.begin() + static_cast<std::ptrdiff_t>(best));
     }
-    jp.n = static_cast<int32_t>(lfill[k]);
-    if (jp.n <= 0 || jp.tiles.reserve(size_t(jp.n)) != cudaSuccess) {
-      cudaGetLastError();
-      give_back(jp);
-      continue;
-    }
-    const cudaStream_t ks = k == 0 ? ln.main() : ln.next();
-    e = cudaMemcpyAsync(jp.tiles.p, lists + lbeg[k], lfill[k] * sizeof(int4),
-                        cudaMemcpyHostToDevice, ks);
-    if (e != cudaSuccess) break;
-    launch_jit_spans(jp.tiles.p, jp.n, tb.desc.p + id, tb.lens.p + size_t(id) * 32, op.a_rp,
-                     op.a_col, op.b_rp, tb.jwords.p + k * W, p->num_sms, ks);
-  }
-  ln.join();
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(words, tb.jwords.p, K * W * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) {
-    for (auto &c : cand) give_back(c);
-    return e;
-  }
-  // requests for the patterns that can have a kernel
-  std::vector<JitRequest> reqs(K);
-  for (size_t k = 0; k < K; ++k) {
-    JitPattern &jp = cand[k];
-    const int4 d = desc[size_t(order[k])];
-    if (!jp.tiles.p || d.x <= 0 || d.x > 32 || d.y <= 0 || d.y > kJitMaxOut) {
-      give_back(jp);
-      continue;
-    }
-    JitRequest &rq = reqs[k];
-    rq.na = d.x;
-    rq.m = d.y;
-    const uint16_t *tab = tabs + k * size_t(stride);
-    int32_t off = 0;
-    for (int j = 0; j < d.x; ++j) {
-      rq.len[j] = lens[size_t(order[k]) * 32 + j];
-      for (int ee = 0; ee < rq.len[j]; ++ee) rq.slot.push_back(tab[size_t(off + ee)] & 0x7fff);
-      off += (rq.len[j] + 7) & ~7;
-    }
-    int32_t need = 0;
-    rq.groups = jit_groups(d.x, rq.len, words + k * W, kJitMaxSpan, &need);
-    if (rq.groups.empty() || need <= 0 || need > kJitMaxSpan) {
-      rq = JitRequest();
-      give_back(jp);
-      continue;
-    }
-    jp.m = d.y;
-  }
-  jit_pattern_kernels(reqs);
-  // tile records of the compiled patterns (their maxima: the records' A
-  // extent, then each group's largest B range over every tile)
-  cudaMemsetAsync(tb.jwords.p, 0, K * W * sizeof(int32_t), s);
-  std::vector<int32_t> rws(K, 0);
-  Lanes lr(p, s, true);
-  for (size_t k = 0; k < K; ++k) {
-    JitPattern &jp = cand[k];
-    const JitRequest &rq = reqs[k];
-    if (!jp.tiles.p) continue;
-    if (!rq.kernel) {
-      give_back(jp);
-      continue;
-    }
-    rws[k] = jit_record_words(rq.na, static_cast<int>(rq.groups.size()));
-    if (jp.prog.reserve(size_t(jp.n) * size_t(rws[k])) != cudaSuccess ||
-        jp.arange.reserve(size_t(jp.n)) != cudaSuccess || jp.head.reserve(1) != cudaSuccess) {
-      cudaGetLastError();
-      give_back(jp);
-      continue;
-    }
-    for (size_t g = 0; g < rq.groups.size(); ++g)
-      gh[k * 32 + g] = make_int2(rq.groups[g].first, rq.groups[g].second);
-    const cudaStream_t ks = k == 0 ? lr.main() : lr.next();
-    cudaMemcpyAsync(tb.jgroups.p + k * 32, gh + k * 32, rq.groups.size() * sizeof(int2),
-                    cudaMemcpyHostToDevice, ks);
-    launch_jit_programs(jp.tiles.p, jp.n, rq.na, rq.groups, tb.jgroups.p + k * 32,
-                        tb.lens.p + size_t(order[k]) * 32, op.a_rp, op.a_col, op.b_rp,
-                        jp.prog.p, jp.arange.p, tb.jwords.p + k * W, p->num_sms, ks);
-  }
-  lr.join();
-  e = cudaMemcpyAsync(words, tb.jwords.p, K * W * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) {
-    for (auto &c : cand) if (c.tiles.p) give_back(c);
-    return e;
-  }
-  int dev_max = 0;
-  cudaDeviceGetAttribute(&dev_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, p->device);
-  for (size_t k = 0; k < K; ++k) {
-    JitPattern &jp = cand[k];
-    if (!jp.tiles.p) continue;
-    // the largest B range any tile's group reads (the sample only chose
-    // the groups); past kJitMaxSpan the uint16 offsets would not hold
-    int32_t need = 0;
-    for (size_t g = 0; g < reqs[k].groups.size(); ++g)
-      need = std::max(need, words[k * W + 1 + g]);
-    if (need <= 0 || need > kJitMaxSpan) {
-      give_back(jp);
-      continue;
-    }
-    jit_layout(rws[k], words[k * W], need, jp.m, &jp.stage_cap, &jp.abuf_floats,
+    jp.n = n;
+    jp.m = rq.m;
+    jit_layout(rw, pseg[order[k]], need[k], jp.m, &jp.stage_cap, &jp.abuf_floats,
                &jp.work_floats);
     // two warps must fit one block's shared memory
-    if (size_t(2) * size_t(jp.work_floats) * sizeof(float) > size_t(dev_max)) {
-      give_back(jp);
+    if (n <= 0 || size_t(2) * size_t(jp.work_floats) * sizeof(float) > size_t(dev_max) ||
+        jp.prog.reserve(size_t(n) * size_t(rw)) != cudaSuccess ||
+        jp.arange.reserve(size_t(n)) != cudaSuccess || jp.head.reserve(1) != cudaSuccess) {
+      cudaGetLastError();
+      tb.pool.push_back(jp);
       continue;
     }
-    jp.grid = jit_grid(reqs[k].kernel, jp.n, jp.work_floats, jp.m, p->num_sms);
-    jp.kernel = reqs[k].kernel;
-    launch_mark_pattern(tb.desc.p, order[k], s);
+    jp.kernel = rq.kernel;
+    jp.grid = jit_grid(jp.kernel, n, jp.work_floats, jp.m, p->num_sms);
+    TileProgram &q = P.p[P.n++];
+    q.prog = jp.prog.p;
+    q.arange = jp.arange.p;
+    q.pid = order[k];
+    q.na = rq.na;
+    q.ng = static_cast<int32_t>(rq.groups.size());
+    q.rw = rw;
+    std::fill(q.group, q.group + 32, kNoGroup);
+    for (size_t g = 0; g < rq.groups.size(); ++g)
+      std::fill(q.group + rq.groups[g].first, q.group + rq.groups[g].second,
+                static_cast<uint8_t>(g));
     tb.jit.push_back(jp);
   }
-  // the table kernel's own list: the tiles of the patterns left to it
-  if (!tb.jit.empty() && tb.table.reserve(size_t(tb.n_tiles)) == cudaSuccess) {
-    cudaMemsetAsync(tb.counts.p + 6, 0, sizeof(int32_t), s);
-    launch_table_tiles(tb.tiles.p, tb.n_tiles, tb.desc.p, tb.table.p, tb.counts.p + 6, s);
-    e = cudaMemcpyAsync(words, tb.counts.p + 6, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return e;
-    tb.n_table = words[0];
-  } else {
-    cudaGetLastError();
-  }
-  return cudaGetLastError();
+  launch_tile_records(tb.tiles.p, static_cast<int32_t>((int64_t(p->a_rows) + 31) / 32), shifted, P,
+                      tb.rank.p, tb.lens.p, tb.offs.p, op.a_rp, op.a_col, op.b_rp, tb.desc.p, s);
 }
-constexpr int kTileCountWords = 8;  // ntiles, leftovers, 3 maxima, list count, spare
 
 // Row tiles of a set of table patterns (k_tile.cu): the per-pattern tile
 // tables (from each pattern's canonical row map: moff[row], map), then tiles
 // over chunks of 32 consecutive rows of tb.pid (the pattern of each row, -1
-// elsewhere, filled by the caller) and the leftover list.  Leaves tb.ready 0
-// (every pattern row on the warp-per-row kernel) when nothing is tiled.
-// With `required` (the shift classes, whose rows have no other path) a
-// failed allocation is an error, and the list of every pattern row is built
-// too.  Synchronizes `s`.
+// elsewhere, filled by the caller) and the leftover list; one read-back of
+// what the builder counted, from which the compiled patterns are chosen and
+// everything else is queued.  Leaves tb.ready 0 (every pattern row on the
+// warp-per-row kernel) when nothing is tiled.  With `shifted` (the shift
+// classes: each pattern's rows are its canonical row moved, and they have no
+// other path) a failed allocation is an error.  Synchronizes `s`.
 cudaError_t build_row_tiles(rvsp_cuda_plan *p, cudaStream_t s, const Operands &op,
                             const int32_t *c_rp, int32_t npat, const int32_t *pat_canon,
                             const int32_t *psteps, const int64_t *moff, const uint16_t *map,
-                            TileBuild &tb, bool required = false) {
+                            TileBuild &tb, bool shifted = false) {
   tb.ready = 0;
   tb.n_lo = 0;
-  const size_t n = static_cast<size_t>(p->a_rows);
-  const size_t tab_entries = size_t(npat) * size_t(tile_tab_stride());
-  if (tb.tab.reserve(tab_entries) != cudaSuccess ||
-      tb.lens.reserve(size_t(npat) * 32) != cudaSuccess ||
-      tb.desc.reserve(size_t(npat)) != cudaSuccess ||
-      tb.tiles.reserve((n + 31) / 32) != cudaSuccess ||
+  tb.n_tiles = 0;
+  tb.n_table = 0;
+  tb.listed = false;
+  for (auto &j : tb.jit) tb.pool.push_back(j);
+  tb.jit.clear();
+  const size_t n = static_cast<size_t>(p->a_rows), np = static_cast<size_t>(npat);
+  const size_t stride = size_t(tile_tab_stride()), nchunks = (n + 31) / 32;
+  // counts | tiles per pattern | A segment per pattern | spans per pattern
+  const size_t words = kTileCountWords + np * (2 + kSpanWords);
+  if (tb.tab.reserve(np * stride) != cudaSuccess || tb.lens.reserve(np * 32) != cudaSuccess ||
+      tb.offs.reserve(np * 32) != cudaSuccess || tb.desc.reserve(np) != cudaSuccess ||
+      tb.tiles.reserve(nchunks) != cudaSuccess || tb.table.reserve(nchunks) != cudaSuccess ||
+      tb.rank.reserve(tile_rank_words(static_cast<int32_t>(nchunks))) != cudaSuccess ||
       tb.lo_rows.reserve(n) != cudaSuccess || tb.lo_ids.reserve(n) != cudaSuccess ||
-      tb.counts.reserve(kTileCountWords) != cudaSuccess ||
-      (required && (tb.all_rows.reserve(n) != cudaSuccess ||
-                    tb.all_ids.reserve(n) != cudaSuccess))) {
+      tb.counts.reserve(words) != cudaSuccess ||
+      (shifted && (tb.all_rows.reserve(n) != cudaSuccess ||
+                   tb.all_ids.reserve(n) != cudaSuccess))) {
     const cudaError_t err = cudaGetLastError();
-    return required ? err : cudaSuccess;
+    return shifted ? err : cudaSuccess;
   }
-  int32_t b_nnz = 0;
-  cudaError_t e = cudaMemcpyAsync(&b_nnz, op.b_rp + p->b_rows, sizeof(int32_t),
-                                  cudaMemcpyDeviceToHost, s);
-  if (e != cudaSuccess) return e;
-  cudaMemsetAsync(tb.counts.p, 0, kTileCountWords * sizeof(int32_t), s);
-  if (required)
-    launch_tile_list(p->a_rows, tb.pid.p, tb.all_rows.p, tb.all_ids.p, tb.counts.p + 5, s);
-  launch_tile_tab(npat, pat_canon, psteps, op.a_rp, op.a_col, op.b_rp, c_rp, moff, map,
-                  tb.tab.p, tb.lens.p, tb.desc.p, s);
-  launch_tile_build(p->a_rows, tb.pid.p, tb.desc.p, tb.lens.p, op.a_rp, op.a_col, op.b_rp,
-                    c_rp, tb.tiles.p, tb.counts.p, tb.lo_rows.p, tb.lo_ids.p,
-                    tb.counts.p + 1, tb.counts.p + 2, s);
-  int32_t h[kTileCountWords] = {};
-  e = cudaMemcpyAsync(h, tb.counts.p, sizeof(h), cudaMemcpyDeviceToHost, s);
+  // the read-back: the words above (spans only of few patterns), then desc,
+  // lens and, of few patterns, the tables (16-byte aligned pieces)
+  const bool all = npat <= kReadAllPatterns;
+  auto up16 = [](size_t x) { return (x + 15) & ~size_t(15); };
+  const size_t word_bytes = (all ? words : kTileCountWords + 2 * np) * sizeof(int32_t);
+  const size_t o_desc = up16(word_bytes), o_lens = o_desc + up16(np * sizeof(int4));
+  const size_t o_tabs = o_lens + up16(np * 32 * sizeof(uint16_t));
+  const size_t tab_bytes = stride * sizeof(uint16_t);
+  const size_t o_spans = o_tabs + up16((all ? np : size_t(kJitMaxPatterns)) * tab_bytes);
+  const size_t total = o_spans + (all ? 0 : kJitMaxPatterns * kSpanWords * sizeof(int32_t));
+  cudaError_t e = tb.staging.reserve(total);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return shifted ? e : cudaSuccess;
+  }
+  int32_t *const d_count = tb.counts.p + kTileCountWords, *const d_seg = d_count + np;
+  int32_t *const d_spans = d_seg + np;
+  cudaMemsetAsync(tb.counts.p, 0, words * sizeof(int32_t), s);
+  launch_tile_tab(npat, pat_canon, psteps, op.a_rp, op.a_col, op.b_rp, c_rp, moff, map, p->b_rows,
+                  tb.tab.p, tb.lens.p, tb.offs.p, tb.desc.p, tb.counts.p + kCountBnnz, s);
+  launch_tile_build(p->a_rows, shifted, tb.pid.p, tb.desc.p, tb.lens.p, tb.offs.p, op.a_rp,
+                    op.a_col, op.b_rp, c_rp, tb.tiles.p, d_count, d_seg, d_spans, tb.lo_rows.p,
+                    tb.lo_ids.p, tb.counts.p, p->num_sms, s);
+  char *const h = tb.staging.p;
+  e = cudaMemcpyAsync(h, tb.counts.p, word_bytes, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(h + o_desc, tb.desc.p, np * sizeof(int4), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(h + o_lens, tb.lens.p, np * 32 * sizeof(uint16_t),
+                        cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess && all && p->pattern_kernels)
+    e = cudaMemcpyAsync(h + o_tabs, tb.tab.p, np * tab_bytes, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return e;
-  tb.n_lo = h[1];
-  if (h[0] <= 0) return cudaSuccess;
+  const int32_t *const hc = reinterpret_cast<const int32_t *>(h);
+  const int32_t *const pcount = hc + kTileCountWords;
+  const int4 *const desc = reinterpret_cast<const int4 *>(h + o_desc);
+  const uint16_t *const lens = reinterpret_cast<const uint16_t *>(h + o_lens);
+  tb.n_lo = hc[1];
+  if (hc[0] <= 0) return cudaSuccess;
   int32_t acc_rows = 0, work = 0, stage_cap = 0;
-  const size_t per_warp = tile_smem_per_warp(h[2], h[3], h[4], &acc_rows, &work, &stage_cap);
+  const size_t per_warp = tile_smem_per_warp(hc[2], hc[3], hc[4], &acc_rows, &work, &stage_cap);
   int dev_max = 0;
   cudaDeviceGetAttribute(&dev_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, p->device);
   // (cannot happen: the tile limits keep one block under 140 KB)
   if (per_warp * kTileKernelWarps > size_t(dev_max))
-    return required ? cudaErrorInvalidValue : cudaSuccess;
-  tb.n_tiles = h[0];
-  tb.stage = h[2];
-  tb.aseg = h[3];
-  tb.max_out = h[4];
-  tb.b_nnz = b_nnz;
+    return shifted ? cudaErrorInvalidValue : cudaSuccess;
+  tb.n_tiles = hc[0];
+  tb.stage = hc[2];
+  tb.aseg = hc[3];
+  tb.max_out = hc[4];
+  tb.b_nnz = hc[kCountBnnz];
   tb.ready = 1;
-  if (p->pattern_kernels) return build_pattern_kernels(p, s, op, npat, tb);
-  return cudaSuccess;
+  tb.n_table = tb.n_tiles;
+  if (p->pattern_kernels) {
+    std::vector<int32_t> order;
+    for (int32_t id = 0; id < npat; ++id)
+      if (pcount[id] >= kJitMinTiles) order.push_back(id);
+    std::sort(order.begin(), order.end(),
+              [&](int32_t a, int32_t b) { return pcount[a] > pcount[b]; });
+    if (order.size() > size_t(kJitMaxPatterns)) order.resize(size_t(kJitMaxPatterns));
+    std::vector<const int32_t *> spans;
+    std::vector<const uint16_t *> tabs;
+    for (size_t k = 0; k < order.size(); ++k) {
+      const size_t id = size_t(order[k]);
+      if (all) {
+        spans.push_back(pcount + 2 * np + id * kSpanWords);
+        tabs.push_back(reinterpret_cast<const uint16_t *>(h + o_tabs) + id * stride);
+        continue;
+      }
+      char *const ht = h + o_tabs + k * tab_bytes;
+      char *const hs = h + o_spans + k * kSpanWords * sizeof(int32_t);
+      tabs.push_back(reinterpret_cast<const uint16_t *>(ht));
+      spans.push_back(reinterpret_cast<const int32_t *>(hs));
+      e = cudaMemcpyAsync(ht, tb.tab.p + id * stride, tab_bytes, cudaMemcpyDeviceToHost, s);
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(hs, d_spans + id * kSpanWords, kSpanWords * sizeof(int32_t),
+                            cudaMemcpyDeviceToHost, s);
+      if (e != cudaSuccess) return e;
+    }
+    if (!all && !order.empty()) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return e;
+    build_pattern_kernels(p, s, op, shifted, order, pcount, pcount + np, desc, lens, spans, tabs,
+                          tb);
+    for (const auto &j : tb.jit) tb.n_table -= j.n;
+  }
+  if (tb.n_table > 0)
+    launch_table_tiles(tb.tiles.p, static_cast<int32_t>(nchunks), tb.desc.p, tb.table.p,
+                       tb.counts.p + kCountTable, s);
+  return cudaGetLastError();
 }
 
 // Builds the reuse map of the W<T> rows for the structure in c_col (written
@@ -1792,36 +1717,38 @@ cudaError_t build_shift_tables(rvsp_cuda_plan *p, cudaStream_t s, const Operands
   launch_scan_i64(npat, p->sh_pat_cap.p, p->sh_pat_off.p, p->partials.p, p->total.p, s);
   cudaMemsetAsync(p->sh_counts.p, 0, 4 * sizeof(int32_t), s);
   launch_pat_maxima(npat, p->sh_pat_canon.p, p->sh_pat_m.p, p->ops.p, p->sh_counts.p, s);
-  int64_t records = 0;
-  int32_t maxima[4] = {};
-  e = cudaMemcpyAsync(&records, p->total.p, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(maxima, p->sh_counts.p, sizeof(maxima), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  // The tables' records: few patterns take the most they can need, so that the
+  // host need not ask (12 KB a pattern); many take the scan's total.
+  int64_t records = int64_t(npat) * pat_max_records();
+  int32_t *const maxima = p->h_misc;  // (read with the tile builder's counts)
+  e = cudaMemcpyAsync(maxima, p->sh_counts.p, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess && npat > 4096) {
+    e = cudaMemcpyAsync(p->h_total, p->total.p, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    records = *p->h_total;
+  }
   if (e != cudaSuccess) return e;
   e = p->sh_rec.reserve(size_t(records > 0 ? records : 1));
   if (e != cudaSuccess) return e;
   launch_pat_build(npat, p->sh_pat_canon.p, op.a_rp, op.a_col, op.b_rp, c_rp, p->sh_moff.p,
                    p->sh_map.p, p->sh_pat_off.p, p->sh_pat_cap.p, p->sh_rec.p, p->sh_steps.p,
                    s);
-  p->sh_max_ops = maxima[0];
-  p->sh_max_out = maxima[1];
   e = build_row_tiles(p, s, op, c_rp, npat, p->sh_pat_canon.p, p->sh_steps.p, p->sh_moff.p,
                       p->sh_map.p, p->st, true);
   if (e != cudaSuccess) return e;
+  p->sh_max_ops = maxima[0];
+  p->sh_max_out = maxima[1];
   p->shift_tables = 1;
   return cudaSuccess;
 }
 
-// The table kernel over the tiles of the patterns without a compiled
-// kernel (every tile when none is compiled); returns the launches.
+// The table kernel over the tiles of the patterns without a compiled kernel;
+// returns the launches.
 int launch_table_tile_kernel(const TileBuild &tb, const Operands &op, const int32_t *c_rp,
                              float *c_val, cudaStream_t s) {
-  const bool own = !tb.jit.empty() && tb.table.p;
-  const int32_t n = own ? tb.n_table : tb.n_tiles;
-  if (n <= 0) return 0;
-  launch_tile_numeric(op, tb.b_nnz, own ? tb.table.p : tb.tiles.p, n, tb.desc.p, tb.lens.p,
-                      tb.tab.p, c_rp, c_val, tb.stage, tb.aseg, tb.max_out, s);
+  if (tb.n_table <= 0) return 0;
+  launch_tile_numeric(op, tb.b_nnz, tb.table.p, tb.n_table, tb.desc.p, tb.lens.p, tb.tab.p, c_rp,
+                      c_val, tb.stage, tb.aseg, tb.max_out, s);
   return 1;
 }
 
@@ -1862,6 +1789,13 @@ int launch_shift_numeric(rvsp_cuda_plan *p, Lanes &ln, const Operands &op,
     launches += launch_pattern_kernels(p->st, op, c_rp, c_val, p->misc.p + kStatus, ln, false);
     launches += launch_pattern_kernels(p->st, op, c_rp, c_val, p->misc.p + kStatus, ln, true);
   } else {
+    if (!p->st.listed) {
+      cudaMemsetAsync(p->st.counts.p + kCountAll, 0, sizeof(int32_t), ln.main());
+      launch_tile_list(p->a_rows, p->st.pid.p, p->st.all_rows.p, p->st.all_ids.p,
+                       p->st.counts.p + kCountAll, ln.main());
+      p->st.listed = true;
+      ++launches;
+    }
     launch_pat_numeric(op, p->ops.p, p->st.all_rows.p, p->st.all_ids.p, p->shift_members,
                        c_rp, c_val, p->sh_pat_off.p, p->sh_steps.p, p->sh_rec.p,
                        p->sh_max_ops, p->sh_max_out, ln.main());
@@ -2173,9 +2107,12 @@ rvsp_status_t rvsp_cuda_numeric(rvsp_cuda_plan_t p, void *stream,
   if (p->shift_active) {
     // Shift-class members: columns by translation of their canonical rows
     // (filled above), values from the canonical rows' term tables.
+    // (the columns beside the table builds: nothing here reads them)
+    Lanes members(p, s, !ln.forked);
     if (fill) {
       PhaseScope ph(p, s, RVSP_PHASE_NUMERIC);
-      launch_shift_fill(p->a_rows, p->st.pid.p, p->sh_rcls.p, c_row_ptr, c_col_idx, s);
+      launch_shift_fill(p->a_rows, p->st.pid.p, p->sh_rcls.p, c_row_ptr, c_col_idx,
+                        members.next());
       ph.launches = 1;
     }
     if (p->shift_tables == 0) {
@@ -2187,7 +2124,7 @@ rvsp_status_t rvsp_cuda_numeric(rvsp_cuda_plan_t p, void *stream,
     }
     if (p->shift_tables != 1) return RVSP_ERROR_DEVICE;
     PhaseScope ph(p, s, RVSP_PHASE_NUMERIC);
-    Lanes members(p, s, !ln.forked);
+    members.refork();
     ph.launches =
         launch_shift_numeric(p, ln.forked ? ln : members, op, c_row_ptr, c_values);
     members.join();
