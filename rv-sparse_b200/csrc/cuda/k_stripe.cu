@@ -71,9 +71,10 @@ constexpr uint32_t kUntouched = 0xffffffffu;
 
 // The values kernel's dynamic shared memory: the accumulator, a word a thread
 // for products that have no slot, and, for each of
-// item_words words of the bitmap, two half words with the outputs before them.
+// item_words words of the bitmap, two half words with the outputs before them,
+// and an empty word.
 constexpr size_t value_bytes(int32_t item_words) {
-  return size_t(kAcc + kValueWarps * 32) * 4 + size_t(item_words) * 8;
+  return size_t(kAcc + kValueWarps * 32) * 4 + size_t(item_words) * 8 + 16;
 }
 
 // ---- stripes of B -------------------------------------------------------------
@@ -245,19 +246,21 @@ __device__ __forceinline__ int owner_of_unit(Runs &r, int32_t u0, unsigned &star
   return own;
 }
 
-// Steps [u0, u0 + 32): step[i] = (first entry, entries, a) of step u0 + i (no
-// entries past the chunk's end); returns how many there are.
+// Steps [u0, u0 + 32): step[i] = (first entry, entries, a) of step u0 + i, past
+// the chunk's end the last run's first entry and no entries; returns how many
+// there are.
 __device__ __forceinline__ int open_steps(Runs &r, const int4 *seg, int4 *step, int32_t u0) {
   const int lane = lane_id();
   unsigned starts;
   const int own = owner_of_unit(r, u0, starts);
   const int32_t u = u0 + lane;
-  int4 s = make_int4(0, 0, 0, 0);
+  int4 s = seg[own];
   if (u < r.total) {
-    s = seg[own];
     const int32_t skip = (u - s.w) << 5;
     s.x += skip;
     s.y = min(32, s.y - skip);
+  } else {
+    s.y = 0;
   }
   __syncwarp();  // the steps before have been read
   step[lane] = s;
@@ -644,15 +647,22 @@ struct Item {
   int32_t c0, width;  // the item's columns
 };
 
-// The accumulator slot of column c0 + rel, or -1 when it has none.
+// The accumulator slot of column c0 + rel; missing turns non-zero when it has
+// none (the slot is then any word of the block's).  A column outside a ranked
+// item meets the empty word past its bitmap.
 template <bool kRank>
-__device__ __forceinline__ int32_t slot_of(const WarpMem &m, int32_t rel, int32_t width) {
-  const bool inside = static_cast<uint32_t>(rel) < static_cast<uint32_t>(width);
-  if (!kRank) return inside ? rel : -1;
-  const uint32_t x = m.half[min(static_cast<uint32_t>(rel), static_cast<uint32_t>(width) - 1u) >> 4];
+__device__ __forceinline__ int32_t slot_of(const WarpMem &m, int32_t rel, int32_t width,
+                                           uint32_t &missing) {
+  if (!kRank) {
+    const bool inside = static_cast<uint32_t>(rel) < static_cast<uint32_t>(width);
+    missing |= inside ? 0u : 1u;
+    return inside ? rel : kAcc;
+  }
+  const uint32_t x =
+      m.half[min(static_cast<uint32_t>(rel) >> 4, static_cast<uint32_t>(width) >> 4)];
   const uint32_t bit = 1u << (rel & 15);
-  return inside & ((x & bit) != 0u) ? static_cast<int32_t>(x >> 16) + __popc(x & (bit - 1u))
-                                    : -1;
+  missing |= bit & ~x;
+  return static_cast<int32_t>((x >> 16) + __popc(x & (bit - 1u)));
 }
 
 // Applies the item's products; returns this lane's first touches.
@@ -663,7 +673,7 @@ __device__ __forceinline__ int walk_item(const Operands &op, const Item &it, con
   const int lane = lane_id();
   int touched = 0;
   const int32_t spare = kAcc + static_cast<int32_t>(threadIdx.x);
-  int32_t missing = 0;  // negative once a column had no slot
+  uint32_t missing = 0;  // non-zero once a column had no slot: B is not the analysed one
   // A's entries of the next chunk, and their stripe starts, are loaded while
   // this one is applied
   int64_t k_next = 0;
@@ -696,9 +706,9 @@ __device__ __forceinline__ int walk_item(const Operands &op, const Item &it, con
       for (int32_t u0 = 0; u0 < run.total; u0 += 32) {
         const int n = open_steps(run, m.seg, m.step, u0);
         // the next steps' entries are loaded while these are applied (lanes
-        // past a step's entries read its first one; b_col has one)
-        int32_t col[kStepUnroll];
-        float val[kStepUnroll];
+        // past a step's entries read its first one and add to a spare word)
+        int32_t col[kStepUnroll], len[kStepUnroll];
+        float val[kStepUnroll], av[kStepUnroll];
         auto load = [&](int i) {
 #pragma unroll
           for (int u = 0; u < kStepUnroll; ++u) {
@@ -706,6 +716,8 @@ __device__ __forceinline__ int walk_item(const Operands &op, const Item &it, con
             const uint32_t e = sg.x + (lane < sg.y ? lane : 0);
             col[u] = __ldg(op.b_col + e);
             val[u] = __ldg(op.b_val + e);
+            len[u] = sg.y;
+            av[u] = __int_as_float(sg.z);
           }
         };
         load(0);
@@ -714,12 +726,9 @@ __device__ __forceinline__ int walk_item(const Operands &op, const Item &it, con
           float term[kStepUnroll];
 #pragma unroll
           for (int u = 0; u < kStepUnroll; ++u) {
-            const int4 sg = m.step[i + u];
-            term[u] = __fmul_rn(__int_as_float(sg.z), val[u]);
-            slot[u] = slot_of<kRank>(m, col[u] - it.c0, it.width);
-            // a column without a slot: B is not the analysed one
-            missing |= lane < sg.y ? slot[u] : 0;
-            slot[u] = lane < sg.y && slot[u] >= 0 ? slot[u] : spare;
+            term[u] = __fmul_rn(av[u], val[u]);
+            slot[u] = slot_of<kRank>(m, col[u] - it.c0, it.width, missing);
+            slot[u] = lane < len[u] ? slot[u] : spare;
           }
           if (i + kStepUnroll < n) load(i + kStepUnroll);
 #pragma unroll
@@ -746,12 +755,8 @@ __device__ __forceinline__ int walk_item(const Operands &op, const Item &it, con
         }
       }
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
-        const bool v = slot[u] != INT_MAX;
-        slot[u] = slot_of<kRank>(m, slot[u], it.width);
-        missing |= v ? slot[u] : 0;
-        slot[u] = slot[u] >= 0 ? slot[u] : spare;
-      }
+      for (int u = 0; u < kUnroll; ++u)
+        slot[u] = slot[u] != INT_MAX ? slot_of<kRank>(m, slot[u], it.width, missing) : spare;
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
         if (t + 32 * u >= run.total) break;
@@ -760,7 +765,7 @@ __device__ __forceinline__ int walk_item(const Operands &op, const Item &it, con
       }
     }
   }
-  bad |= missing < 0;
+  bad |= missing != 0u;
   return touched;
 }
 
@@ -843,6 +848,7 @@ stripe_values_kernel(Operands op, const int4 *__restrict__ items, int64_t cap,
         }
       }
       for (int32_t e = tid; e < nout; e += kThreads) m.acc[e] = 0u;
+      if (tid == 0) m.half[it.width >> 4] = 0u;
     }
     __syncthreads();
     if (tid == 0) s_next = atomicAdd(head, 1);  // (read after the next barriers)
@@ -860,7 +866,9 @@ stripe_values_kernel(Operands op, const int4 *__restrict__ items, int64_t cap,
         c_val[out + e] = __uint_as_float(m.acc[e]);
         m.acc[e] = kUntouched;
         if (verify) {
-          bad |= slot_of<true>(m, __ldg(c_col + out + e) - it.c0, it.width) != e;
+          uint32_t missing = 0;
+          bad |= slot_of<true>(m, __ldg(c_col + out + e) - it.c0, it.width, missing) != e;
+          bad |= missing != 0u;
         }
       }
       continue;
