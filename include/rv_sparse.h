@@ -52,7 +52,9 @@ rvsp_status_t rvsp_csr_create(rvsp_csr_matrix_t *A, int32_t rows, int32_t cols,
 rvsp_status_t rvsp_csr_validate(const rvsp_csr_matrix_t *A);
 
 /* rv_sparse.h:50.  Frees host arrays when owns_data == 1, device arrays when
- * owns_data == 2, then resets the struct.  NULL is accepted. */
+ * owns_data == 2, then resets the struct.  NULL is accepted.  Host arrays are
+ * plain malloc blocks; up to six large ones (64 MB together) are kept for the
+ * next one-shot results and freed when a thread that made products ends. */
 void rvsp_csr_destroy(rvsp_csr_matrix_t *A);
 
 /* rv_sparse.h:63-67.  One-shot C = A * B on host arrays.  Checks canonical

@@ -85,9 +85,9 @@ void rvsp_csr_destroy(rvsp_csr_matrix_t *A)
     if (!A)
         return;
     if (A->owns_data == 1) {
-        free(A->row_ptr);
-        free(A->col_idx);
-        free(A->values);
+        rvsp_result_free(A->row_ptr);
+        rvsp_result_free(A->col_idx);
+        rvsp_result_free(A->values);
     } else if (A->owns_data == 2) {
         cudaFree(A->row_ptr);
         cudaFree(A->col_idx);

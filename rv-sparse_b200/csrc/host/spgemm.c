@@ -49,6 +49,7 @@ static void ctx_free(void *p)
     if (c->stream)
         cudaStreamDestroy(c->stream);
     free(c);
+    rvsp_result_trim();
 }
 
 static void ctx_key_init(void)
@@ -200,9 +201,9 @@ static rvsp_status_t oneshot_host(const rvsp_csr_matrix_t *A, const rvsp_csr_mat
         return st;
 
     const size_t alloc = (size_t)(c_nnz > 0 ? c_nnz : 1);
-    int32_t *rp = (int32_t *)rvsp_malloc(((size_t)A->rows + 1) * sizeof(int32_t));
-    int32_t *ci = (int32_t *)rvsp_malloc(alloc * sizeof(int32_t));
-    float *cv = (float *)rvsp_malloc(alloc * sizeof(float));
+    int32_t *rp = (int32_t *)rvsp_result_alloc(((size_t)A->rows + 1) * sizeof(int32_t));
+    int32_t *ci = (int32_t *)rvsp_result_alloc(alloc * sizeof(int32_t));
+    float *cv = (float *)rvsp_result_alloc(alloc * sizeof(float));
     if (!rp || !ci || !cv) {
         free(rp);
         free(ci);

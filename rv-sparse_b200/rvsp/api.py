@@ -18,6 +18,32 @@ from .csr import CSR
 CUDA_STREAM_LEGACY = 0x1  # cudaStreamLegacy
 
 
+class _HostArray:
+    """One host array of a library result, freed with the last numpy view of
+    it (rvsp_csr_destroy on a struct that holds this array alone)."""
+
+    def __init__(self, lib, m, field, n, dtype):
+        self._lib, self._one = lib, L.CsrMatrix()
+        self._one.owns_data = 1
+        setattr(self._one, field, getattr(m, field))
+        setattr(m, field, None)
+        self.__array_interface__ = {"data": (getattr(self._one, field), False), "shape": (n,),
+                                    "typestr": np.dtype(dtype).str, "version": 3}
+
+    def __del__(self):
+        self._lib.rvsp_csr_destroy(C.byref(self._one))
+
+
+def _host_result(lib, c, vout):
+    """The arrays of a one-shot result, taken over as they are: a copy of
+    each cost 0.4 ms for 5 MB and, in fresh pages, 4 ms for 19 MB."""
+    rp = np.asarray(_HostArray(lib, c, "row_ptr", c.rows + 1, np.int32))
+    if c.nnz <= 0:
+        return rp, np.zeros(0, np.int32), np.zeros(0, vout)
+    return (rp, np.asarray(_HostArray(lib, c, "col_idx", c.nnz, np.int32)),
+            np.asarray(_HostArray(lib, c, "values", c.nnz, vout)))
+
+
 def spgemm_csr(A: CSR, B: CSR, backend: int | None = L.BACKEND_CUDA) -> CSR:
     """One-shot C = A * B on host arrays (rvsp_spgemm_csr).  backend=None
     passes NULL options."""
@@ -31,18 +57,7 @@ def spgemm_csr(A: CSR, B: CSR, backend: int | None = L.BACKEND_CUDA) -> CSR:
                              C.byref(opts) if opts is not None else None)
     L.check(st, "rvsp_spgemm_csr")
     try:
-        n = c.nnz
-        rp = np.ctypeslib.as_array(C.cast(c.row_ptr, C.POINTER(C.c_int32)),
-                                   shape=(c.rows + 1,)).copy()
-        if n > 0:
-            ci = np.ctypeslib.as_array(C.cast(c.col_idx, C.POINTER(C.c_int32)),
-                                       shape=(n,)).copy()
-            cv = np.ctypeslib.as_array(C.cast(c.values, C.POINTER(C.c_float)),
-                                       shape=(n,)).copy()
-        else:
-            ci = np.zeros(0, np.int32)
-            cv = np.zeros(0, np.float32)
-        return CSR(c.rows, c.cols, rp, ci, cv)
+        return CSR(c.rows, c.cols, *_host_result(lib, c, np.float32))
     finally:
         lib.rvsp_csr_destroy(C.byref(c))
 
@@ -57,7 +72,7 @@ def spgemm_typed(A, B, kind: str, backend: int = L.BACKEND_CUDA):
     (rows, cols, row_ptr, col_idx, values) tuples of host arrays; returns
     (row_ptr, col_idx, values) or raises RvspError."""
     lib = L.load()
-    din, dout, vin, vout, ct = _TYPED_CODES[kind]
+    din, dout, vin, vout, _ = _TYPED_CODES[kind]
     keep = []
 
     def struct(M):
@@ -76,17 +91,8 @@ def spgemm_typed(A, B, kind: str, backend: int = L.BACKEND_CUDA):
     L.check(lib.rvsp_spgemm_csr(C.byref(a), C.byref(b), C.byref(c), C.byref(opts)),
             "rvsp_spgemm_csr")
     try:
-        n = c.nnz
-        rp = np.ctypeslib.as_array(C.cast(c.row_ptr, C.POINTER(C.c_int32)),
-                                   shape=(c.rows + 1,)).copy()
-        if n > 0:
-            ci = np.ctypeslib.as_array(C.cast(c.col_idx, C.POINTER(C.c_int32)),
-                                       shape=(n,)).copy()
-            cv = np.ctypeslib.as_array(C.cast(c.values, C.POINTER(ct)), shape=(n,)).copy()
-        else:
-            ci, cv = np.zeros(0, np.int32), np.zeros(0, vout)
         assert c.dtype == dout
-        return rp, ci, cv.astype(vout, copy=False)
+        return _host_result(lib, c, vout)
     finally:
         lib.rvsp_csr_destroy(C.byref(c))
 
