@@ -398,6 +398,16 @@ rvsp_status_t rvsp_cuda_coo_to_csr(void *stream, int32_t rows, int32_t cols, int
                                    int32_t **c_col_out, float **c_val_out,
                                    int32_t *c_nnz_out);
 
+/* The entries of a Matrix Market text (host memory: what follows the size
+ * line, len bytes; fields 2 or 3 tokens an entry, at most limit entries),
+ * parsed on the device and made canonical as above.  *parsed = 0, with
+ * RVSP_SUCCESS and nothing allocated: the text holds tokens that only the
+ * host's sequential reading can place, or no memory was free for it. */
+rvsp_status_t rvsp_cuda_mtx_to_csr(void *stream, const char *text, size_t len, int fields,
+                                   int64_t limit, int32_t rows, int32_t cols, int symmetric,
+                                   int32_t *c_row_ptr, int32_t **c_col_out,
+                                   float **c_val_out, int32_t *c_nnz_out, int *parsed);
+
 /* ---- Batches ------------------------------------------------------------
  * No reference counterpart: the reference computes one product per call.
  * A batch of independent products C_i = A_i * B_i is packed, a group of

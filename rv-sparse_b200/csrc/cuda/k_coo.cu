@@ -25,6 +25,7 @@
 #include "device_common.cuh"
 #include "kernels.cuh"
 #include "rvsp_cuda.h"
+#include "scratch.cuh"
 
 namespace rvsp {
 
@@ -268,7 +269,7 @@ rvsp_status_t status_of(cudaError_t e) {
 }
 
 // A stream-ordered memory pool per device, owned by this file: the
-// canonicalisation's scratch (a few buffers per call, tens of MB for large
+// scratch of reading a matrix (a few buffers per call, tens of MB for large
 // files) comes from it, and up to kPoolKeepBytes stay reserved between calls,
 // so repeated reads pay no cudaMalloc / cudaFree (which synchronise and map
 // or unmap pages).  Created on first use on each device.
@@ -276,6 +277,8 @@ constexpr int kMaxDevices = 64;
 constexpr unsigned long long kPoolKeepBytes = 1ull << 30;
 cudaMemPool_t g_pool[kMaxDevices] = {};
 std::once_flag g_pool_once[kMaxDevices];
+
+}  // namespace
 
 cudaMemPool_t scratch_pool() {
   int dev = 0;
@@ -296,32 +299,6 @@ cudaMemPool_t scratch_pool() {
   });
   return g_pool[dev];
 }
-
-// Device scratch of one call, from the pool (cudaMalloc when the pool could
-// not be made), released in stream order when the call returns.
-struct Scratch {
-  static constexpr int kSlots = 16;
-  void *p[kSlots] = {};
-  int n = 0;
-  cudaStream_t s = nullptr;
-  cudaMemPool_t pool = nullptr;
-  explicit Scratch(cudaStream_t st) : s(st), pool(scratch_pool()) {}
-  cudaError_t alloc(void **out, size_t bytes) {
-    if (n >= kSlots) return cudaErrorMemoryAllocation;  // more buffers than slots
-    const size_t b = bytes ? bytes : 1;
-    cudaError_t e = pool ? cudaMallocFromPoolAsync(out, b, pool, s) : cudaMalloc(out, b);
-    if (e == cudaSuccess) p[n++] = *out;
-    return e;
-  }
-  ~Scratch() {
-    for (int i = 0; i < n; ++i) {
-      if (pool) cudaFreeAsync(p[i], s);
-      else cudaFree(p[i]);
-    }
-  }
-};
-
-}  // namespace
 
 }  // namespace rvsp
 

@@ -17,10 +17,12 @@
  * RVSP_ERROR_INVALID_CSR (the reference writes out of bounds), and the
  * result carries N as its column count (the reference's CSR struct has none).
  *
- * The entries are parsed on all host cores: the text after the size line is
- * cut at whitespace into one piece per thread, each thread counts its tokens,
- * and then converts them knowing each token's global index (entry = index /
- * fields, field = index % fields).  That equals fscanf's reading whenever each
+ * A text of MTX_DEVICE_MIN bytes or more is parsed on the device.  What it
+ * hands back, and a smaller one, is parsed here, from MTX_PARALLEL_MIN bytes
+ * on all host cores: the text after the size line is cut at whitespace into
+ * one piece per thread, each thread counts its tokens, and then converts them
+ * knowing each token's global index (entry = index / fields, field = index %
+ * fields).  That equals fscanf's reading whenever each
  * conversion consumes its whole token; if any does not (say "1.5" read as an
  * integer), the file is read again by a sequential scanner that advances
  * exactly as fscanf does.
@@ -35,6 +37,11 @@
 #include "rvsp_internal.h"
 
 #define MTX_LINE 2048 /* the reference's fgets buffer */
+/* From this much text the device parses (rvsp_cuda_mtx_to_csr).  Up to 8 KB
+ * both sides take the 0.87 ms of the result's allocations; host / device in
+ * ms a read: 17 KB 0.94 / 0.87, 150 KB 1.6 / 0.84, 2.7 MB 13.8 / 1.1, 23 MB
+ * (host cores in parallel) 18.7 / 3.7. */
+#define MTX_DEVICE_MIN ((size_t)8 << 10)
 #define MTX_PARALLEL_MIN ((size_t)4 << 20)
 #define MTX_MAX_THREADS 64
 
@@ -259,20 +266,21 @@ static int64_t read_entries(const char *t, size_t len, size_t pos, int pattern,
     return n;
 }
 
-/* COO (device) to CSR in the requested memory space. */
-static rvsp_status_t finish(int32_t M, int32_t N, int64_t n, int symmetric, const int32_t *row,
-                            const int32_t *col, const float *val, rvsp_memory_space_t space,
-                            rvsp_csr_matrix_t *out)
+/* Host entries to device CSR arrays (*d_rp: M + 1, made here unless given). */
+static rvsp_status_t canonical_from_host(int32_t M, int32_t N, int64_t n, int symmetric,
+                                         const int32_t *row, const int32_t *col,
+                                         const float *val, int32_t **d_rp, int32_t **c_col,
+                                         float **c_val, int32_t *nnz)
 {
-    int32_t *d_row = NULL, *d_col = NULL, *d_rp = NULL, *c_col = NULL;
-    float *d_val = NULL, *c_val = NULL;
-    int32_t nnz = 0;
+    int32_t *d_row = NULL, *d_col = NULL;
+    float *d_val = NULL;
     const size_t nb = (size_t)(n > 0 ? n : 1);
     rvsp_status_t st = RVSP_SUCCESS;
     cudaError_t e = cudaMalloc((void **)&d_row, nb * sizeof(int32_t));
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_col, nb * sizeof(int32_t));
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_val, nb * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&d_rp, ((size_t)M + 1) * sizeof(int32_t));
+    if (e == cudaSuccess && !*d_rp)
+        e = cudaMalloc((void **)d_rp, ((size_t)M + 1) * sizeof(int32_t));
     if (e == cudaSuccess && n > 0) {
         e = cudaMemcpy(d_row, row, (size_t)n * sizeof(int32_t), cudaMemcpyHostToDevice);
         if (e == cudaSuccess)
@@ -280,12 +288,61 @@ static rvsp_status_t finish(int32_t M, int32_t N, int64_t n, int symmetric, cons
         if (e == cudaSuccess)
             e = cudaMemcpy(d_val, val, (size_t)n * sizeof(float), cudaMemcpyHostToDevice);
     }
-    if (e != cudaSuccess) {
-        st = rvsp_map_cuda(e);
-        goto done;
+    st = rvsp_map_cuda(e);
+    if (st == RVSP_SUCCESS)
+        st = rvsp_cuda_coo_to_csr(NULL, M, N, n, symmetric, d_row, d_col, d_val, *d_rp, c_col,
+                                  c_val, nnz);
+    cudaFree(d_row);
+    cudaFree(d_col);
+    cudaFree(d_val);
+    return st;
+}
+
+/* The entries of text (NUL-terminated here, in a copy: strtol / strtof must
+ * not run past it) by the host parser, then as above. */
+static rvsp_status_t parse_on_host(const char *text, size_t len, int pattern, int64_t limit,
+                                   int32_t M, int32_t N, int symmetric, int32_t **d_rp,
+                                   int32_t **c_col, float **c_val, int32_t *nnz)
+{
+    const size_t nb = (size_t)(limit > 0 ? limit : 1);
+    rvsp_status_t st = RVSP_ERROR_ALLOCATION_FAILED;
+    char *t = (char *)rvsp_malloc(len + 1);
+    int32_t *row = (int32_t *)rvsp_malloc(nb * sizeof(int32_t));
+    int32_t *col = (int32_t *)rvsp_malloc(nb * sizeof(int32_t));
+    float *val = (float *)rvsp_malloc(nb * sizeof(float));
+    if (t && row && col && val) {
+        memcpy(t, text, len);
+        t[len] = '\0';
+        const int64_t n = read_entries(t, len, 0, pattern, limit, row, col, val);
+        st = canonical_from_host(M, N, n, symmetric, row, col, val, d_rp, c_col, c_val, nnz);
     }
-    st = rvsp_cuda_coo_to_csr(NULL, M, N, n, symmetric, d_row, d_col, d_val, d_rp, &c_col,
-                              &c_val, &nnz);
+    free(row);
+    free(col);
+    free(val);
+    free(t);
+    return st;
+}
+
+/* The entries of text to CSR in the requested memory space. */
+static rvsp_status_t finish(const char *text, size_t len, int pattern, int64_t limit, int32_t M,
+                            int32_t N, int symmetric, rvsp_memory_space_t space,
+                            rvsp_csr_matrix_t *out)
+{
+    int32_t *d_rp = NULL, *c_col = NULL;
+    float *c_val = NULL;
+    int32_t nnz = 0;
+    int parsed = 0;
+    rvsp_status_t st = RVSP_SUCCESS;
+    cudaError_t e;
+    if (len >= MTX_DEVICE_MIN) {
+        st = rvsp_map_cuda(cudaMalloc((void **)&d_rp, ((size_t)M + 1) * sizeof(int32_t)));
+        if (st == RVSP_SUCCESS)
+            st = rvsp_cuda_mtx_to_csr(NULL, text, len, pattern ? 2 : 3, limit, M, N, symmetric,
+                                      d_rp, &c_col, &c_val, &nnz, &parsed);
+    }
+    if (st == RVSP_SUCCESS && !parsed)
+        st = parse_on_host(text, len, pattern, limit, M, N, symmetric, &d_rp, &c_col, &c_val,
+                           &nnz);
     if (st != RVSP_SUCCESS)
         goto done;
     memset(out, 0, sizeof(*out));
@@ -334,9 +391,6 @@ static rvsp_status_t finish(int32_t M, int32_t N, int64_t n, int symmetric, cons
         out->owns_data = 1;
     }
 done:
-    cudaFree(d_row);
-    cudaFree(d_col);
-    cudaFree(d_val);
     cudaFree(d_rp);
     cudaFree(c_col);
     cudaFree(c_val);
@@ -351,48 +405,25 @@ rvsp_status_t rvsp_csr_parse_mtx(const char *text, size_t len, rvsp_memory_space
     memset(out, 0, sizeof(*out)); /* every failure leaves out empty */
     if (space != RVSP_MEM_HOST && space != RVSP_MEM_DEVICE)
         return RVSP_ERROR_INVALID_ARGUMENT;
-    /* a NUL-terminated copy: strtol / strtof must not run past the text */
-    char *t = (char *)rvsp_malloc(len + 1);
-    if (!t)
-        return RVSP_ERROR_ALLOCATION_FAILED;
-    memcpy(t, text, len);
-    t[len] = '\0';
     char buf[MTX_LINE];
     size_t pos = 0;
     int pattern = 0, symmetric = 0;
-    rvsp_status_t st = RVSP_SUCCESS;
     buf[0] = '\0';
-    if (next_line(t, len, &pos, buf))
+    if (next_line(text, len, &pos, buf))
         parse_banner(buf, &pattern, &symmetric);
-    while (next_line(t, len, &pos, buf))
+    while (next_line(text, len, &pos, buf))
         if (buf[0] != '%')
             break;
     int M, N, L;
-    if (sscanf(buf, "%d %d %d", &M, &N, &L) != 3 || M < 0 || N < 0 || L < 0) {
-        free(t);
+    if (sscanf(buf, "%d %d %d", &M, &N, &L) != 3 || M < 0 || N < 0 || L < 0)
         return RVSP_ERROR_INVALID_ARGUMENT;
-    }
     /* an entry takes at least fields tokens and separators */
     const int fields = pattern ? 2 : 3;
     int64_t limit = L;
     const int64_t fit = (int64_t)((len - pos) / (size_t)(2 * fields)) + 1;
     if (limit > fit)
         limit = fit;
-    const size_t nb = (size_t)(limit > 0 ? limit : 1);
-    int32_t *row = (int32_t *)rvsp_malloc(nb * sizeof(int32_t));
-    int32_t *col = (int32_t *)rvsp_malloc(nb * sizeof(int32_t));
-    float *val = (float *)rvsp_malloc(nb * sizeof(float));
-    if (!row || !col || !val) {
-        st = RVSP_ERROR_ALLOCATION_FAILED;
-    } else {
-        const int64_t n = read_entries(t, len, pos, pattern, limit, row, col, val);
-        st = finish(M, N, n, symmetric, row, col, val, space, out);
-    }
-    free(row);
-    free(col);
-    free(val);
-    free(t);
-    return st;
+    return finish(text + pos, len - pos, pattern, limit, M, N, symmetric, space, out);
 }
 
 rvsp_status_t rvsp_csr_read_mtx(const char *path, rvsp_memory_space_t space,

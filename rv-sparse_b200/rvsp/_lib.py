@@ -96,6 +96,8 @@ SIGNATURES = {
     "rvsp_debug_host_allocs": (_i64, []),
     "rvsp_cuda_coo_to_csr": (_int, [_vp, _i32, _i32, _i64, _int, _vp, _vp, _vp, _vp,
                                     _P(_vp), _P(_vp), _P(_i32)]),
+    "rvsp_cuda_mtx_to_csr": (_int, [_vp, C.c_char_p, _sz, _int, _i64, _i32, _i32, _int, _vp,
+                                    _P(_vp), _P(_vp), _P(_i32), _P(_int)]),
     "rvsp_cuda_symbolic_checked": (_int, [_vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _vp,
                                           _vp, _vp, _vp, _int, _vp, _P(_i64)]),
     "rvsp_cuda_typed_numeric": (_int, [_vp, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
