@@ -103,7 +103,9 @@ __device__ __forceinline__ int32_t fill_row(const Operands &op, int32_t p0, int3
 }
 
 // Rows: rows[0..nrows) (rows == nullptr: rows 0..nrows).  With sel, rows
-// whose sel entry is not this kernel's class are skipped.
+// whose sel entry is not this kernel's class are skipped; there the M8 kernel
+// takes the M4 rows too (a launch of their own, over the classes of a million
+// rows, took 9 us).
 template <int K>
 __global__ void __launch_bounds__(kMergeThreads, MergeOccupancy<K, false>::value)
 merge_symbolic_kernel(Operands op, const int32_t *__restrict__ rows,
@@ -112,13 +114,19 @@ merge_symbolic_kernel(Operands op, const int32_t *__restrict__ rows,
   const int32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nrows) return;
   const int32_t row = row_of(rows, t);
-  if (sel && sel[row] != merge_class_of<K>()) return;
+  if (sel) {
+    const int c = sel[row];
+    if (c != merge_class_of<K>() && !(K == 8 && c == kM4)) return;
+  }
   if (guard.failed()) return;
   const int32_t p0 = op.a_rp[row];
   const int32_t k = op.a_rp[row + 1] - p0;
   // a warp whose rows all fit fewer lists runs the narrower merge
   constexpr int KN = NarrowK<K>::value;
-  if (KN < K && __all_sync(__activemask(), k <= KN))
+  const unsigned warp = __activemask();
+  if (K == 8 && __all_sync(warp, k <= 4))
+    counts[row] = count_row<4>(op, p0, k);
+  else if (KN < K && __all_sync(warp, k <= KN))
     counts[row] = count_row<KN>(op, p0, k);
   else
     counts[row] = count_row<K>(op, p0, k);
@@ -265,7 +273,6 @@ void launch_merge_symbolic(int cls, const Operands &op, const int32_t *rows,
 void launch_merge_symbolic_all(const Operands &op, const uint8_t *cls, int32_t a_rows,
                                int32_t *counts, CheckGuard guard, cudaStream_t s) {
   if (a_rows <= 0) return;
-  sym<4>(op, nullptr, a_rows, counts, s, cls, guard);
   sym<8>(op, nullptr, a_rows, counts, s, cls, guard);
   sym<16>(op, nullptr, a_rows, counts, s, cls, guard);
 }

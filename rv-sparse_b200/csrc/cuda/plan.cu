@@ -883,7 +883,7 @@ rvsp_status_t symbolic_impl(rvsp_cuda_plan_t p, cudaStream_t s, int32_t a_rows,
   }
   const int32_t *skip = shift ? p->st.pid.p : nullptr;
   // Merge-class rows need no host-side census: their symbolic pass (one
-  // launch per merge class over all rows, each skipping the other classes)
+  // launch for M4 and M8 and one for M16, over all rows, each skipping the rest)
   // and the scan are queued at once, behind the check verdict, so a product
   // whose rows are all merge rows takes one host round trip.  When other
   // classes turn up, their pass and the scan follow the census.  The early
@@ -894,7 +894,7 @@ rvsp_status_t symbolic_impl(rvsp_cuda_plan_t p, cudaStream_t s, int32_t a_rows,
     {
       PhaseScope ph(p, s, RVSP_PHASE_SYMBOLIC);
       launch_merge_symbolic_all(op, p->cls.p, a_rows, p->counts.p, guard, s);
-      ph.launches = 3;
+      ph.launches = 2;
     }
     {
       PhaseScope ph(p, s, RVSP_PHASE_SCAN);
