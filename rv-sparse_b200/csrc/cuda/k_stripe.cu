@@ -20,7 +20,9 @@
 //             row's outputs in them, so a hub row is many items and a row of a
 //             few thousand products one or two; rows of many products are
 //             drawn first;
-//   values    persistent warps draw items; per item a warp walks its products
+//   values    persistent blocks of four warps draw items and cut each into four
+//             runs of stripes of about equal products, a warp each over one
+//             accumulator; a warp walks its products
 //             in flattened order (ascending A nonzero, then column), up to 32
 //             of one B row at a time, or 32 across short B rows with equal
 //             columns in lane order, into an accumulator in shared memory: a
@@ -38,6 +40,21 @@
 // returns (results that are NaN are the canonical one), and the counts of
 // first touches, of gathered words and of outputs must agree; with a slot an
 // output, C's columns are compared with the bitmap.
+//
+// Bound: issue slots.  A product is a column, a value, a slot look-up, an add
+// and its share of the walk, some 20 instructions for a lane; none of it waits
+// for another warp.  R-MAT 2^16, 16 entries a row (402 M products), whole
+// product on one B200, in ms: block-per-row kernels 13.1; a warp an item 7.2;
+// four warps sharing one accumulator (runs of B entries four times longer),
+// outputs ranked where columns do not fit, hub rows counted in parts 4.3; with
+// items placed by one atomic a warp and slot checks folded into the bitmap
+// word 3.5, of which the values take 1.8, the count 0.7, the columns 0.5.
+// Numeric-only repeat at 2^15: 2.6 -> 0.92.  Measured and left: 5 warps (one
+// reading ahead) 3.70 against 3.58, 6 to 9 blocks an SM by launch bounds 3.7
+// to 4.4 (spills), accumulators of 2048 and 8192 slots, 8 or 2 steps in flight
+// and items of 8 K to 128 K products each within 5%.  B wider than
+// kStripeMaxCols keeps the block kernels: a row's bitmap no longer fits shared
+// memory beside its prefix.
 #include <climits>
 
 #include "device_common.cuh"
@@ -167,6 +184,7 @@ stripe_bounds_kernel(int32_t words, int32_t ns_max, const int32_t *__restrict__ 
   }
 }
 
+// Bound by the latency of the searches.
 // ptr[k * (ns_max + 1) + t] = first entry of B row k in stripe t or after it
 // (the row's end for t = ns_max).  A warp per row, a lane per stripe, each a
 // binary search of the row: short rows cost a few cached loads, and a hub row
@@ -328,6 +346,9 @@ stripe_tasks_kernel(const int32_t *__restrict__ rows, int32_t nrows,
     for (int w = threadIdx.x; w < words; w += 128) bits[int64_t(s_cut[i]) * words + w] = 0u;
 }
 
+// Bound by shared-memory atomics on a row's bitmap, read before they are set
+// (a byte a column instead of a bit: 1.37 ms against 0.93 at 2^16 then, two
+// blocks an SM).
 // rows[r]: counts[row], hslot[row] = r, the row's bitmap at bits + r * words,
 // the outputs before each 32 words of it at gpre + r * stripe_groups(words)
 // and the outputs before stripe t at soff[r * (ns_max + 1) + t].  The parts of
@@ -550,6 +571,8 @@ stripe_items_kernel(const int32_t *__restrict__ rows, int32_t nrows,
 
 // ---- columns ----------------------------------------------------------------------
 
+// Bound by issue slots (lanes walk bits of words of unequal population; 0.5 ms
+// for R-MAT 2^16).
 // 32 words at a time, a lane per word: each lane drops its set bits' columns
 // into the warp's staging in order, and the warp copies them out together.
 __global__ void __launch_bounds__(kColumnWarps * 32)

@@ -6,6 +6,8 @@
 // positions are distinct) for all but the shortest B rows, flattened tiles with
 // ordered_apply for those.  The walk waits on loads: the map and the values of
 // kMapUnroll steps are loaded together before the first of them is applied.
+// Repeat of a 48-product batch: 1.65 -> 1.42 ms; uniform rows of six to eight
+// entries, stepped instead of tiled, 1.2 times as fast.
 #pragma once
 
 #include "device_common.cuh"
