@@ -23,15 +23,17 @@ class _HostArray:
     it (rvsp_csr_destroy on a struct that holds this array alone)."""
 
     def __init__(self, lib, m, field, n, dtype):
-        self._lib, self._one = lib, L.CsrMatrix()
-        self._one.owns_data = 1
-        setattr(self._one, field, getattr(m, field))
+        one = L.CsrMatrix()
+        one.owns_data = 1
+        setattr(one, field, getattr(m, field))
         setattr(m, field, None)
-        self.__array_interface__ = {"data": (getattr(self._one, field), False), "shape": (n,),
+        # (held here: a module's names may be gone when the last view goes)
+        self._destroy, self._one = lib.rvsp_csr_destroy, C.byref(one)
+        self.__array_interface__ = {"data": (getattr(one, field), False), "shape": (n,),
                                     "typestr": np.dtype(dtype).str, "version": 3}
 
     def __del__(self):
-        self._lib.rvsp_csr_destroy(C.byref(self._one))
+        self._destroy(self._one)
 
 
 def _host_result(lib, c, vout):
