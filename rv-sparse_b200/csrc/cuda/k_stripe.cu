@@ -35,7 +35,8 @@
 // with accum_scalar_f32.c:20-71); the columns are the row's bitmap in order
 // (rvsp_symbolic.c:91-137).
 //
-// A C whose columns are not this product's is reported.  With a slot a column
+// A row of C that is not as long as the analysed one is reported and left as it
+// is.  A C whose columns are not this product's is reported.  With a slot a column
 // an accumulator word starts as kUntouched, a NaN pattern that no addition
 // returns (results that are NaN are the canonical one), and the counts of
 // first touches, of gathered words and of outputs must agree; with a slot an
@@ -807,9 +808,9 @@ stripe_values_kernel(Operands op, const int4 *__restrict__ items, int64_t cap,
                      const float *__restrict__ share, const int32_t *__restrict__ ptr,
                      const int32_t *__restrict__ hslot,
                      const uint32_t *__restrict__ bits, const int32_t *__restrict__ gpre,
-                     int32_t words, int32_t item_words, const int32_t *__restrict__ c_rp,
-                     const int32_t *__restrict__ c_col, float *__restrict__ c_val, bool verify,
-                     int32_t *__restrict__ status) {
+                     int32_t words, int32_t item_words, const int32_t *__restrict__ counts,
+                     const int32_t *__restrict__ c_rp, const int32_t *__restrict__ c_col,
+                     float *__restrict__ c_val, bool verify, int32_t *__restrict__ status) {
   extern __shared__ __align__(16) uint32_t s_mem[];
   __shared__ int4 s_seg[kValueWarps][32], s_step[kValueWarps][32];
   __shared__ int32_t s_next, s_touched, s_found;
@@ -843,6 +844,15 @@ stripe_values_kernel(Operands op, const int4 *__restrict__ items, int64_t cap,
     if (at >= n_items) break;
     const int4 q = items[at < n_front ? int64_t(at) : cap - 1 - (at - n_front)];
     const int32_t row = q.x, nout = q.w, before = q.z;
+    if (c_rp[row + 1] - c_rp[row] != counts[row]) {  // (uniform)
+      // C's row pointers are not this analysis's: the row stays as it is
+      __syncthreads();  // s_next has been read
+      if (tid == 0) {
+        report(status, kDevCountMismatch);
+        s_next = atomicAdd(head, 1);
+      }
+      continue;
+    }
     const int32_t t0 = q.y & 0xffff, t1 = q.y >> 16;
     Item it;
     it.c0 = bound[t0] << 5;
@@ -1003,8 +1013,9 @@ void launch_stripe_values(const StripeShape &g, const Operands &op, int32_t nrow
                           const int4 *items, int64_t cap, const int32_t *cnt, int32_t *head,
                           const int32_t *bound, const float *share, const int32_t *ptr,
                           const int32_t *hslot, const uint32_t *bits, const int32_t *gpre,
-                          const int32_t *c_rp, const int32_t *c_col, float *c_val, bool verify, int32_t *status,
-                          int num_sms, cudaStream_t s) {
+                          const int32_t *counts, const int32_t *c_rp, const int32_t *c_col,
+                          float *c_val, bool verify, int32_t *status, int num_sms,
+                          cudaStream_t s) {
   if (nrows <= 0) return;
   int32_t item_words = g.words < kItemWords ? g.words : kItemWords;
   item_words = (item_words + 7) & ~7;
@@ -1018,8 +1029,8 @@ void launch_stripe_values(const StripeShape &g, const Operands &op, int32_t nrow
     per_sm = 1;
   cudaMemsetAsync(head, 0, sizeof(int32_t), s);
   stripe_values_kernel<<<num_sms * per_sm, kValueWarps * 32, smem, s>>>(
-      op, items, cap, cnt, head, g.ns_max, bound, share, ptr, hslot, bits, gpre, g.words, item_words,
-      c_rp, c_col, c_val, verify, status);
+      op, items, cap, cnt, head, g.ns_max, bound, share, ptr, hslot, bits, gpre, g.words,
+      item_words, counts, c_rp, c_col, c_val, verify, status);
 }
 
 }  // namespace rvsp

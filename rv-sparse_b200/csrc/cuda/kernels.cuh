@@ -293,13 +293,15 @@ void launch_stripe_columns(const StripeShape &g, const int32_t *rows, int32_t nr
                            int32_t *status, cudaStream_t s);
 // C's values of the items' rows (columns in C; verify: not written by this
 // plan just now, so they are compared with the bitmaps).  nrows: the rows the
-// items cover.
+// items cover; a row whose length in c_rp is not counts[row] is reported and
+// left alone.
 void launch_stripe_values(const StripeShape &g, const Operands &op, int32_t nrows,
                           const int4 *items, int64_t cap, const int32_t *cnt, int32_t *head,
                           const int32_t *bound, const float *share, const int32_t *ptr,
                           const int32_t *hslot, const uint32_t *bits, const int32_t *gpre,
-                          const int32_t *c_rp, const int32_t *c_col, float *c_val, bool verify, int32_t *status,
-                          int num_sms, cudaStream_t s);
+                          const int32_t *counts, const int32_t *c_rp, const int32_t *c_col,
+                          float *c_val, bool verify, int32_t *status, int num_sms,
+                          cudaStream_t s);
 
 // ---- k_reuse.cu ------------------------------------------------------------
 // Reuse map of the W<T> classes: per product, its position in C's row.

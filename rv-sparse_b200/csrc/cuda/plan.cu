@@ -1829,8 +1829,9 @@ int launch_stripe_rows(rvsp_cuda_plan *p, const Operands &op, const int32_t *c_r
     launch_stripe_columns(p->sp, sr.rows, sr.n, p->sp_hslot.p, p->sp_bits.p, p->sp_gpre.p,
                           p->sp_soff.p, c_rp, c_col, status, s);
   launch_stripe_values(p->sp, op, sr.n, p->sp_items.p, p->sp_cap, p->sp_cnt.p,
-                       p->sp_cnt.p + 2, p->sp_bound.p, p->sp_share.p, p->sp_ptr.p, p->sp_hslot.p, p->sp_bits.p,
-                       p->sp_gpre.p, c_rp, c_col, c_val, !fill, status, p->num_sms, s);
+                       p->sp_cnt.p + 2, p->sp_bound.p, p->sp_share.p, p->sp_ptr.p,
+                       p->sp_hslot.p, p->sp_bits.p, p->sp_gpre.p, p->counts.p, c_rp, c_col,
+                       c_val, !fill, status, p->num_sms, s);
   return fill ? 2 : 1;
 }
 
