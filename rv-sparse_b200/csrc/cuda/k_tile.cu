@@ -476,20 +476,30 @@ tile_numeric_kernel(const int32_t *__restrict__ a_rp, const int32_t *__restrict_
   }
 }
 
-// rows / ids: every row with pid_of_row[row] >= 0, in chunk order.
-__global__ void __launch_bounds__(256)
+// rows / ids: every row with pid_of_row[row] >= 0, in row order within a block.
+// One addition to the count a block (one a warp is 40,000 of them on one word
+// for 1.3 M rows).
+constexpr int kListThreads = 1024;
+__global__ void __launch_bounds__(kListThreads)
 tile_list_kernel(int32_t n, const int32_t *__restrict__ pid_of_row, int32_t *__restrict__ rows,
                  int32_t *__restrict__ ids, int32_t *__restrict__ count) {
-  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ int32_t s_at[kListThreads / 32];
+  const int lane = lane_id(), wid = threadIdx.x >> 5;
+  const int64_t i = int64_t(blockIdx.x) * kListThreads + threadIdx.x;
   const int32_t pid = i < n ? pid_of_row[i] : -1;
   const unsigned b = __ballot_sync(kFull, pid >= 0);
-  if (!b) return;
-  int32_t base = 0;
-  if (lane_id() == 0) base = atomicAdd(count, __popc(b));
-  base = __shfl_sync(kFull, base, 0);
+  if (lane == 0) s_at[wid] = __popc(b);
+  __syncthreads();
+  if (wid == 0) {
+    const int32_t c = s_at[lane], incl = warp_incl_scan(c);
+    int32_t base = 0;
+    if (lane == 31 && incl) base = atomicAdd(count, incl);
+    s_at[lane] = __shfl_sync(kFull, base, 31) + incl - c;
+  }
+  __syncthreads();
   if (pid >= 0) {
-    const int32_t at = base + __popc(b & lanemask_lt());
-    rows[at] = i;
+    const int at = s_at[wid] + __popc(b & lanemask_lt());
+    rows[at] = static_cast<int32_t>(i);
     ids[at] = pid;
   }
 }
@@ -501,7 +511,9 @@ int32_t tile_tab_stride() { return kTileTabStride; }
 void launch_tile_list(int32_t n, const int32_t *pid_of_row, int32_t *rows, int32_t *ids,
                       int32_t *count, cudaStream_t s) {
   if (n <= 0) return;
-  tile_list_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, pid_of_row, rows, ids, count);
+  const int64_t grid = (int64_t(n) + kListThreads - 1) / kListThreads;
+  tile_list_kernel<<<static_cast<unsigned>(grid), kListThreads, 0, s>>>(n, pid_of_row, rows, ids,
+                                                                        count);
 }
 
 void launch_tile_tab(int32_t npat, const int32_t *pat_canon, const int32_t *psteps,

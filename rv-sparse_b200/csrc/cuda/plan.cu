@@ -108,8 +108,9 @@ namespace rvsp {
 // tile table, B row lengths and shape; per row its pattern (pid, -1 for rows
 // outside the set); the tiles, one entry per chunk of 32 rows; the pattern
 // rows left to the warp-per-row table kernel (lo_rows / lo_ids); for the shift
-// classes also every pattern row (all_rows / all_ids, listed when tiles are
-// off).
+// classes also every pattern row (all_rows / all_ids, for calls with tiles off;
+// listed before the build's wait, so that they are there for every later call,
+// on any stream and under capture).
 struct JitPattern {
   void *kernel = nullptr;
   DevArray<int32_t> prog;  // tile records (k_jit.cu)
@@ -128,7 +129,6 @@ struct TileBuild {
   std::vector<JitPattern> pool;  // device arrays of earlier builds, for reuse
   HostArray staging;             // host side of the build's read-back
   int ready = 0;
-  bool listed = false;  // all_rows / all_ids hold the current analysis's rows
   int32_t n_tiles = 0, n_lo = 0, stage = 0, aseg = 0, max_out = 0, b_nnz = 0;
   // counts, then per pattern its tiles, its longest A segment and its union
   // spans: one array, zeroed and read back whole
@@ -1505,7 +1505,6 @@ cudaError_t build_row_tiles(rvsp_cuda_plan *p, cudaStream_t s, const Operands &o
   tb.n_lo = 0;
   tb.n_tiles = 0;
   tb.n_table = 0;
-  tb.listed = false;
   for (auto &j : tb.jit) tb.pool.push_back(j);
   tb.jit.clear();
   const size_t n = static_cast<size_t>(p->a_rows), np = static_cast<size_t>(npat);
@@ -1541,6 +1540,9 @@ cudaError_t build_row_tiles(rvsp_cuda_plan *p, cudaStream_t s, const Operands &o
   int32_t *const d_count = tb.counts.p + kTileCountWords, *const d_seg = d_count + np;
   int32_t *const d_spans = d_seg + np;
   cudaMemsetAsync(tb.counts.p, 0, words * sizeof(int32_t), s);
+  if (shifted)
+    launch_tile_list(p->a_rows, tb.pid.p, tb.all_rows.p, tb.all_ids.p, tb.counts.p + kCountAll,
+                     s);
   launch_tile_tab(npat, pat_canon, psteps, op.a_rp, op.a_col, op.b_rp, c_rp, moff, map, p->b_rows,
                   tb.tab.p, tb.lens.p, tb.offs.p, tb.desc.p, tb.counts.p + kCountBnnz, s);
   launch_tile_build(p->a_rows, shifted, tb.pid.p, tb.desc.p, tb.lens.p, tb.offs.p, op.a_rp,
@@ -1803,13 +1805,6 @@ int launch_shift_numeric(rvsp_cuda_plan *p, Lanes &ln, const Operands &op,
     launches += launch_pattern_kernels(p->st, op, c_rp, c_val, p->misc.p + kStatus, ln, false);
     launches += launch_pattern_kernels(p->st, op, c_rp, c_val, p->misc.p + kStatus, ln, true);
   } else {
-    if (!p->st.listed) {
-      cudaMemsetAsync(p->st.counts.p + kCountAll, 0, sizeof(int32_t), ln.main());
-      launch_tile_list(p->a_rows, p->st.pid.p, p->st.all_rows.p, p->st.all_ids.p,
-                       p->st.counts.p + kCountAll, ln.main());
-      p->st.listed = true;
-      ++launches;
-    }
     launch_pat_numeric(op, p->ops.p, p->st.all_rows.p, p->st.all_ids.p, p->shift_members,
                        c_rp, c_val, p->sh_pat_off.p, p->sh_steps.p, p->sh_rec.p,
                        p->sh_max_ops, p->sh_max_out, ln.main());
