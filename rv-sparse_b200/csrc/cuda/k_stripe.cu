@@ -59,6 +59,7 @@
 #include <climits>
 
 #include "device_common.cuh"
+#include "index.cuh"
 #include "kernels.cuh"
 
 namespace rvsp {
@@ -205,7 +206,7 @@ stripe_ptr_kernel(int32_t b_rows, const int32_t *__restrict__ b_rp,
       const int32_t c = s_bound[t];
       int32_t lo = b0, hi = b1;
       while (lo < hi) {
-        const int32_t mid = (lo + hi) >> 1;
+        const int32_t mid = middle(lo, hi);  // (entries of all of B)
         if (__ldg(b_col + mid) < c) lo = mid + 1;
         else hi = mid;
       }

@@ -2,7 +2,7 @@
 
 A call whose row pointers do not give a heavy row its analysed length reports
 it and leaves that row alone, whether the row grew or shrank, in a fill and in
-a numeric-only repeat.
+a numeric-only repeat.  B may have more than 2^30 entries.
 """
 import ctypes as C
 
@@ -106,4 +106,27 @@ def test_row_pointers_of_another_length(b_cols, more, fill):
         p.numeric(p.rp, c_ci, c_cv, f)
         assert np.array_equal(c_ci.cpu().numpy(), ci)
         assert np.array_equal(c_cv.cpu().numpy().view(np.uint32), cv.view(np.uint32))
+    p.close()
+
+
+def test_b_of_more_than_2_30_entries():
+    import torch
+    rows, cols = 8300, 131072  # 1.09e9 entries
+    k = [8200, 8299]
+    a = np.array([0.75, -1.25], np.float32)
+    p = _Plan(CSR(1, rows, np.array([0, 2]), np.array(k), a), CSR(1, 1, [0, 0], [], []))
+    g = torch.Generator(device="cuda").manual_seed(1)
+    p.b = DeviceCSR(rows, cols,
+                    torch.arange(rows + 1, dtype=torch.int32, device="cuda") * cols,
+                    torch.arange(cols, dtype=torch.int32, device="cuda").repeat(rows),
+                    torch.rand(rows * cols, generator=g, device="cuda"))
+    assert p.analyse() == cols
+    ci = torch.zeros(cols, dtype=torch.int32, device="cuda")
+    cv = torch.zeros(cols, dtype=torch.float32, device="cuda")
+    b = p.b.values.view(rows, cols)
+    want = float(a[0]) * b[k[0]] + float(a[1]) * b[k[1]]
+    for fill in (1, 0):
+        p.numeric(p.rp, ci, cv, fill)
+        assert torch.equal(ci, torch.arange(cols, dtype=torch.int32, device="cuda"))
+        assert torch.equal(cv, want)
     p.close()
