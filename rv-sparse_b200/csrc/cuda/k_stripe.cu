@@ -704,25 +704,25 @@ __device__ __forceinline__ int walk_item(const Operands &op, const Item &it, con
   int64_t k_next = 0;
   float a = 0.0f, a_next = 0.0f;
   int32_t beg = 0, len = 0;
-  auto load_k = [&](int32_t q) {
-    if (q + lane < it.p1) {
+  auto load_k = [&](uint32_t q) {
+    if (before(q, lane, it.p1)) {
       k_next = __ldg(op.a_col + q + lane) * stride;
       a_next = __ldg(op.a_val + q + lane);
     }
   };
-  auto load_run = [&](int32_t q) {  // of the entries load_k(q) read
+  auto load_run = [&](uint32_t q) {  // of the entries load_k(q) read
     a = a_next;
     beg = len = 0;
-    if (q + lane < it.p1) {
+    if (before(q, lane, it.p1)) {
       beg = __ldg(ptr + k_next + it.t0);
       len = __ldg(ptr + k_next + it.t1) - beg;
     }
   };
-  int32_t p = it.p0;
+  uint32_t p = it.p0;  // (runs past p1, which may be 2^31 - 1)
   load_k(p);
   load_run(p);
   load_k(p + 32);
-  while (p < it.p1) {
+  while (before(p, 0, it.p1)) {
     Runs run = open_runs(m.seg, beg, len, a);
     p += 32;
     load_run(p);

@@ -23,3 +23,13 @@ def _run(tmp_path, body):
                                    (2**31 - 2, 2**31 - 1)])
 def test_middle(tmp_path, lo, hi):
     assert _run(tmp_path, "if (middle(%d, %d) != %d) return 1;" % (lo, hi, (lo + hi) // 2)) == 0
+
+
+@pytest.mark.parametrize("base,step,end", [(0, 0, 0), (3, 4, 8), (3, 5, 8),
+                                           (2**31 - 33, 31, 2**31 - 1),
+                                           (2**31 - 33, 32, 2**31 - 1),
+                                           (2**31 - 1, 31, 2**31 - 1),
+                                           (2**31 + 62, 31, 2**31 - 1)])
+def test_before(tmp_path, base, step, end):
+    want = int(base + step < end)
+    assert _run(tmp_path, "if (before(%dU, %d, %d) != %d) return 1;" % (base, step, end, want)) == 0
