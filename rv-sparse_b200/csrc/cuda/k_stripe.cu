@@ -860,11 +860,16 @@ stripe_values_kernel(Operands op, const int4 *__restrict__ items, int64_t cap,
     it.width = (bound[t1] << 5) - it.c0;
     it.p0 = op.a_rp[row];
     it.p1 = op.a_rp[row + 1];
-    // this warp's stripes: about one share of the item's products
+    // this warp's stripes: about one share of the item's products, up to the
+    // next warp's (each end is computed by two warps, so it is rounded once
+    // and explicitly: no stripe may be taken twice or left out)
     const float first = s_cum[t0], part = (s_cum[t1] - first) * (1.0f / kValueWarps);
-    it.t0 = t0 + stripes_below(s_cum, t0, t1, first + part * wid);
-    it.t1 = wid == kValueWarps - 1 ? t1
-                                   : t0 + stripes_below(s_cum, t0, t1, first + part * (wid + 1));
+    auto cut = [&](int w) {
+      return w == kValueWarps ? t1
+                              : t0 + stripes_below(s_cum, t0, t1, __fmaf_rn(part, w, first));
+    };
+    it.t0 = cut(wid);
+    it.t1 = cut(wid + 1);
     const int64_t out = int64_t(c_rp[row]) + before;
     const bool rank = it.width > kAcc;
     if (rank) {  // a slot an output: the bitmap, and zeroed slots
