@@ -208,6 +208,13 @@ int32_t rvsp_cuda_plan_overflow_rows(rvsp_cuda_plan_t plan);
  * and 2 to time both accumulators on the same rows. */
 rvsp_status_t rvsp_cuda_plan_set_merge_policy(rvsp_cuda_plan_t plan, int32_t policy);
 
+/* Device memory that the stripe rows (rows of more than 1024 possible outputs,
+ * B of at most 2^17 columns) of one analysis may take, from the next analysis
+ * on: 3 GiB by default, and never more than a quarter of what is free where it
+ * has to grow.  Rows without room take the block-per-row kernels, with the
+ * same results.  The plan keeps what its analyses took. */
+rvsp_status_t rvsp_cuda_plan_set_stripe_memory(rvsp_cuda_plan_t plan, size_t bytes);
+
 /* Row tiles for numeric-only repeats (1, the default) or not (0).  The GPU
  * form of the reference's numeric-only compute (spgemm_descr.c:330-349) for
  * runs of consecutive rows that share one term pattern: a warp computes 32

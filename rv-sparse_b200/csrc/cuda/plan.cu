@@ -164,6 +164,11 @@ struct TileBuild {
 };
 }  // namespace rvsp
 
+// Memory of the stripe rows of one analysis.  A square product of 2^17 columns
+// with every row a stripe row takes 2.5 GiB (18.8 KB a row, of which 16 are its
+// bitmap); at 1025 columns a row takes 0.8 KB (0.7 of them items and offsets).
+constexpr size_t kStripeBytesMax = size_t(3) << 30;
+
 struct rvsp_cuda_plan {
   int device = 0;
   int num_sms = 148;
@@ -274,6 +279,7 @@ struct rvsp_cuda_plan {
   // stripe, their slot by row, and the value items of the numeric STRIPE rows.
   StripeShape sp;
   int sp_ready = 0;
+  size_t stripe_max = kStripeBytesMax;  // bytes
   int64_t sp_cap = 0;
   DevArray<int32_t> sp_hist, sp_bound, sp_ptr, sp_gpre, sp_soff, sp_hslot, sp_done;
   DevArray<int32_t> sp_cnt;  // items from the front, from the back, queue head
@@ -516,33 +522,44 @@ void finish_numeric_bins(rvsp_cuda_plan *p, int32_t a_rows, int32_t b_cols,
 
 // The exact counts of the nrows STRIPE rows listed at rows (null: every row),
 // with what their columns and values need later.  Sets sp_ready; it stays 0,
-// and nothing was counted, when the row bitmaps (one bit a column) would take
-// more than kStripeBitsMax or a quarter of the free memory.
-constexpr size_t kStripeBitsMax = size_t(2) << 30;
+// and nothing was counted, when all of that would take more than stripe_max
+// bytes or, where it has to grow, a quarter of the free memory.
 cudaError_t count_stripe_rows(rvsp_cuda_plan *p, const Operands &op, int32_t b_rows,
                               const int32_t *rows, int32_t nrows, cudaStream_t s) {
   const StripeShape &g = p->sp;
   const size_t n = static_cast<size_t>(nrows), stops = static_cast<size_t>(g.ns_max) + 1;
   const size_t words = static_cast<size_t>(g.words);
-  const size_t need = n * words * sizeof(uint32_t);
-  if (need > kStripeBitsMax) return cudaSuccess;
-  if (n * words > p->sp_bits.cap) {
+  p->sp_cap = int64_t(nrows) * g.ns_max;
+  auto each = [&](auto f) {
+    f(p->sp_bits, n * words);
+    f(p->sp_gpre, n * size_t(stripe_groups(g.words)));
+    f(p->sp_soff, n * stops);
+    f(p->sp_items, std::max(size_t(p->sp_cap), stripe_tasks(nrows)));
+    f(p->sp_done, n);
+    f(p->sp_hslot, size_t(op.a_rows));
+    f(p->sp_hist, words);
+    f(p->sp_bound, stops);
+    f(p->sp_share, stops);
+    f(p->sp_cnt, size_t(3));
+    f(p->sp_ptr, size_t(b_rows) * stops);
+  };
+  size_t need = 0, grow = 0;
+  each([&](auto &a, size_t count) {
+    const size_t bytes = count * sizeof(*a.p);
+    need += bytes;
+    if (count > a.cap) grow += bytes;
+  });
+  if (need > p->stripe_max) return cudaSuccess;
+  if (grow > 0) {
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return cudaGetLastError();
-    if (need > free_b / 4) return cudaSuccess;
+    if (grow > free_b / 4) return cudaSuccess;
   }
-  p->sp_cap = int64_t(nrows) * g.ns_max;
-  if (p->sp_bits.reserve(n * words) != cudaSuccess ||
-      p->sp_gpre.reserve(n * size_t(stripe_groups(g.words))) != cudaSuccess ||
-      p->sp_soff.reserve(n * stops) != cudaSuccess ||
-      p->sp_items.reserve(std::max(size_t(p->sp_cap), stripe_tasks(nrows))) != cudaSuccess ||
-      p->sp_done.reserve(n) != cudaSuccess ||
-      p->sp_hslot.reserve(size_t(op.a_rows)) != cudaSuccess ||
-      p->sp_hist.reserve(words) != cudaSuccess ||
-      p->sp_bound.reserve(stops) != cudaSuccess || p->sp_share.reserve(stops) != cudaSuccess ||
-      p->sp_cnt.reserve(3) != cudaSuccess ||
-      p->sp_ptr.reserve(size_t(b_rows) * stops) != cudaSuccess) {
-    cudaGetLastError();  // out of memory: the rows keep the block-per-row kernels
+  bool room = true;
+  each([&](auto &a, size_t count) { room = room && a.reserve(count) == cudaSuccess; });
+  if (!room) {  // the rows take the block-per-row kernels, which get the memory back
+    cudaGetLastError();
+    each([](auto &a, size_t) { a.release(); });
     return cudaSuccess;
   }
   launch_stripe_table(g, b_rows, op.b_rp, op.b_col, p->sp_hist.p, p->sp_bound.p, p->sp_share.p,
@@ -1300,6 +1317,12 @@ rvsp_status_t rvsp_cuda_plan_set_merge_policy(rvsp_cuda_plan_t p, int32_t policy
   if (!p) return RVSP_ERROR_NULL_POINTER;
   if (policy < kMergeAuto || policy > kMergeAlways) return RVSP_ERROR_INVALID_ARGUMENT;
   p->merge_policy = policy;
+  return RVSP_SUCCESS;
+}
+
+rvsp_status_t rvsp_cuda_plan_set_stripe_memory(rvsp_cuda_plan_t p, size_t bytes) {
+  if (!p) return RVSP_ERROR_NULL_POINTER;
+  p->stripe_max = bytes;
   return RVSP_SUCCESS;
 }
 

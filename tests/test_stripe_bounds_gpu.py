@@ -2,7 +2,9 @@
 
 A call whose row pointers do not give a heavy row its analysed length reports
 it and leaves that row alone, whether the row grew or shrank, in a fill and in
-a numeric-only repeat.  B may have more than 2^30 entries.
+a numeric-only repeat.  B may have more than 2^30 entries.  All that the rows
+keep counts against their memory, and rows without room give the same results
+by the block-per-row kernels, on the plain and on the learned path.
 """
 import ctypes as C
 
@@ -46,6 +48,15 @@ class _Plan:
         self.h = C.c_void_p()
         L.check(self.lib.rvsp_cuda_plan_create(C.byref(self.h)), "plan")
         self.rp = torch.zeros(A.rows + 1, dtype=torch.int32, device="cuda")
+
+    def learned(self, model, scale=1.0):
+        a, b, total = self.a, self.b, C.c_int64()
+        L.check(self.lib.rvsp_cuda_learned_symbolic(
+            self.h, model.h, _stream(), a.rows, b.rows, b.cols, a.row_ptr.data_ptr(),
+            a.col_idx.data_ptr(), a.values.data_ptr(), a.nnz, b.row_ptr.data_ptr(),
+            b.col_idx.data_ptr(), b.values.data_ptr(), b.nnz, C.c_float(scale),
+            self.rp.data_ptr(), C.byref(total)), "learned")
+        return total.value
 
     def analyse(self):
         a, b, total = self.a, self.b, C.c_int64()
@@ -129,4 +140,86 @@ def test_b_of_more_than_2_30_entries():
         p.numeric(p.rp, ci, cv, fill)
         assert torch.equal(ci, torch.arange(cols, dtype=torch.int32, device="cuda"))
         assert torch.equal(cv, want)
+    p.close()
+
+
+def test_memory_counts_items_and_offsets():
+    # 400,000 rows of three B rows of 400 columns each: 56 MB of bitmaps and
+    # 270 MB of items and offsets
+    import torch
+    rng = np.random.default_rng(3)
+    n = 400000
+    B = _rows(rng, [400] * 50, 1100)
+    picks = np.sort(rng.permuted(np.tile(np.arange(50), (n, 1)), axis=1)[:, :3], axis=1)
+    A = CSR(n, 50, np.arange(0, 3 * n + 1, 3), picks.reshape(-1), np.ones(3 * n, np.float32))
+    p, q = _Plan(A, B), _Plan(A, B)
+    for plan in (p, q):  # all else that an analysis takes
+        L.check(plan.lib.rvsp_cuda_plan_set_stripe_memory(plan.h, 0), "set_stripe_memory")
+        nnz = plan.analyse()
+
+    def grows(plan, limit):
+        L.check(plan.lib.rvsp_cuda_plan_set_stripe_memory(plan.h, limit), "set_stripe_memory")
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        assert plan.analyse() == nnz
+        torch.cuda.synchronize()
+        return before - torch.cuda.mem_get_info()[0]
+
+    assert grows(p, 200 << 20) <= 200 << 20
+    assert grows(q, 400 << 20) > 200 << 20
+    p.close()
+    q.close()
+
+
+@pytest.mark.parametrize("b_cols", [1100, 40000])
+@pytest.mark.parametrize("path", ["plain", "learned"])
+def test_rows_without_room(path, b_cols):
+    import torch
+    from rvsp.learn import RowModel, weights_for
+    A, B = _operands(b_cols, b_cols + 1)
+    rp, ci, cv, _ = oracle.spgemm(A, B)
+    assert (np.diff(rp) > 1024).sum() > 1
+    p = _Plan(A, B)
+    model = RowModel(path=weights_for("rmat"))
+    for limit in (0, 1 << 30, 0):
+        L.check(p.lib.rvsp_cuda_plan_set_stripe_memory(p.h, limit), "set_stripe_memory")
+        assert (p.learned(model) if path == "learned" else p.analyse()) == ci.size
+        assert np.array_equal(p.rp.cpu().numpy(), rp)
+        if path == "learned":  # without room they are redone by the plain passes
+            assert (p.lib.rvsp_cuda_plan_overflow_rows(p.h) >= 2) == (limit == 0)
+        c_ci = torch.zeros(ci.size, dtype=torch.int32, device="cuda")
+        c_cv = torch.zeros(ci.size, dtype=torch.float32, device="cuda")
+        for fill in (1, 0):
+            p.numeric(p.rp, c_ci, c_cv, fill)
+            assert np.array_equal(c_ci.cpu().numpy(), ci)
+            assert np.array_equal(c_cv.cpu().numpy().view(np.uint32), cv.view(np.uint32))
+    p.close()
+
+
+def test_more_parts_of_rows_than_the_count_holds():
+    # 600 rows of 63 parts of the count each, of which 520 rows' fit and leave 8
+    # places; all rows have one structure and values a power of two apart, so
+    # one row gives all
+    import torch
+    rng = np.random.default_rng(4)
+    rows, inner, cols = 600, 4096, 4096
+    B = _rows(rng, [1000] * inner, cols)
+    one = CSR(1, inner, [0, inner], np.arange(inner),
+              rng.uniform(-1, 1, inner).astype(np.float32))
+    rp, ci, cv, ops = oracle.spgemm(one, B)
+    assert -(-ops[0] // 65536) == 63
+    p = _Plan(one, B)
+    scale = torch.exp2(torch.randint(-3, 4, (rows, 1), device="cuda").float())
+    p.a = DeviceCSR(rows, inner, torch.arange(rows + 1, dtype=torch.int32, device="cuda") * inner,
+                    torch.arange(inner, dtype=torch.int32, device="cuda").repeat(rows),
+                    (scale * torch.from_numpy(one.values).cuda()).reshape(-1).contiguous())
+    p.rp = torch.zeros(rows + 1, dtype=torch.int32, device="cuda")
+    assert p.analyse() == rows * ci.size
+    c_ci = torch.zeros(rows * ci.size, dtype=torch.int32, device="cuda")
+    c_cv = torch.zeros(rows * ci.size, dtype=torch.float32, device="cuda")
+    for fill in (1, 0):
+        p.numeric(p.rp, c_ci, c_cv, fill)
+        assert torch.equal(c_ci.view(rows, -1),
+                           torch.from_numpy(ci).cuda().expand(rows, -1))
+        assert torch.equal(c_cv.view(rows, -1), scale * torch.from_numpy(cv).cuda())
     p.close()
