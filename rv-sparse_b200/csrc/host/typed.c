@@ -15,8 +15,8 @@
  * Then, unlike the legacy kernels (which accept unsorted rows), both operands
  * must be canonical: RVSP_ERROR_INVALID_CSR otherwise, since the GPU passes
  * rely on sorted, duplicate-free rows.  The passes over the columns run on the
- * device for all but small operands, and again on the host, for the code, only
- * if the device finds a fault.  Two host passes over 550,000 entries took
+ * device for all but small operands, and on the host, for the code, only if the
+ * device finds a fault or cannot look.  Two host passes over 550,000 entries took
  * 1.1 ms of a 2.8 ms INT8 call.
  *
  * Work: the FP32 path's symbolic pass and column fill give C's structure;
@@ -191,6 +191,7 @@ rvsp_status_t rvsp_typed_oneshot(const rvsp_csr_matrix_t *A, const rvsp_csr_matr
 {
     const int f64 = in_dtype == RVSP_DTYPE_FP64;
     const int on_device = columns_to_device(A, B, in_dtype);
+    int unchecked = on_device;
     rvsp_status_t st = on_device ? RVSP_SUCCESS : checks_host(A, B, f64);
     if (st != RVSP_SUCCESS)
         return st;
@@ -214,7 +215,7 @@ rvsp_status_t rvsp_typed_oneshot(const rvsp_csr_matrix_t *A, const rvsp_csr_matr
     typed_ctx_t *c = NULL;
     st = typed_ctx(&c);
     if (st != RVSP_SUCCESS)
-        return st;
+        goto done;
     cudaStream_t s = c->stream;
     const int b_is_a = A->row_ptr == B->row_ptr && A->col_idx == B->col_idx &&
                        A->values == B->values && A->rows == B->rows;
@@ -239,13 +240,9 @@ rvsp_status_t rvsp_typed_oneshot(const rvsp_csr_matrix_t *A, const rvsp_csr_matr
         if (st == RVSP_SUCCESS && !(b_is_a && A->cols == B->cols))
             st = rvsp_device_check(c->plan, s, B->rows, B->cols, d_brp, d_bci, b_nnz,
                                    RVSP_REJECT_ALL);
-        if (st == RVSP_ERROR_INVALID_CSR) {
-            /* the code that the checks above give in their order */
-            const rvsp_status_t exact = checks_host(A, B, f64);
-            st = exact != RVSP_SUCCESS ? exact : st;
-        }
         if (st != RVSP_SUCCESS)
             goto done;
+        unchecked = 0;
     }
     st = rvsp_cuda_symbolic(c->plan, s, A->rows, B->rows, B->cols, (const int32_t *)c->a_rp.p,
                             (const int32_t *)c->a_ci.p, d_brp, d_bci, (int32_t *)c->c_rp.p,
@@ -326,5 +323,11 @@ done:
     free(h_rp);
     free(h_ci);
     free(h_v);
+    if (unchecked) {
+        /* The device found a fault, or could not look (no device, no memory):
+         * the code is the one that the host's checks give in their order. */
+        const rvsp_status_t exact = checks_host(A, B, f64);
+        st = exact != RVSP_SUCCESS ? exact : st;
+    }
     return st;
 }
