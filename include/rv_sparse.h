@@ -53,9 +53,13 @@ rvsp_status_t rvsp_csr_validate(const rvsp_csr_matrix_t *A);
 
 /* rv_sparse.h:50.  Frees host arrays when owns_data == 1, device arrays when
  * owns_data == 2, then resets the struct.  NULL is accepted.  Host arrays are
- * plain malloc blocks; up to six large ones (64 MB together) are kept for the
- * next one-shot results and freed when a thread that made products ends. */
+ * plain malloc blocks; while some thread that made one-shot products lives, up
+ * to six large ones (64 MB together) are kept for the next results. */
 void rvsp_csr_destroy(rvsp_csr_matrix_t *A);
+
+/* New: frees the host arrays that rvsp_csr_destroy kept (as the end of the
+ * last thread that made one-shot products does). */
+void rvsp_release_kept_results(void);
 
 /* rv_sparse.h:63-67.  One-shot C = A * B on host arrays.  Checks canonical
  * CSR (RVSP_ERROR_INVALID_CSR), allocates C's host arrays (owns_data = 1)

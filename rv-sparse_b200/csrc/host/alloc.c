@@ -54,8 +54,10 @@ void *rvsp_realloc(void *p, size_t n)
  * INT8 result do on every call (1.5 us a page on the measured host: a 19 MB
  * INT8 result 5.4 -> 1.8 ms a call).
  * At most RESULT_KEEP_BYTES in RESULT_KEEP arrays, all plain malloc blocks;
- * the oldest go first, and the end of a thread that made products gives all
- * of them back.
+ * the oldest go first.  Arrays are kept only while some thread holds a
+ * context of one-shot products (rvsp_result_user): a process that makes none
+ * keeps none, and the end of the last such thread gives all of them back, as
+ * rvsp_release_kept_results does.
  */
 #define RESULT_KEEP 6
 #define RESULT_KEEP_BYTES ((size_t)64 << 20)
@@ -65,6 +67,7 @@ static pthread_mutex_t g_kept_lock = PTHREAD_MUTEX_INITIALIZER;
 static void *g_kept[RESULT_KEEP]; /* oldest first */
 static int g_nkept = 0;
 static size_t g_kept_bytes = 0;
+static int g_users = 0;
 
 /* Takes entry i out of the list (the lock is held). */
 static void *take(int i)
@@ -112,17 +115,31 @@ void rvsp_result_free(void *p)
     void *out[RESULT_KEEP];
     int n = 0;
     pthread_mutex_lock(&g_kept_lock);
-    while (g_nkept == RESULT_KEEP || g_kept_bytes + size > RESULT_KEEP_BYTES)
-        out[n++] = take(0);
-    g_kept[g_nkept++] = p;
-    g_kept_bytes += size;
+    if (g_users > 0) {
+        while (g_nkept == RESULT_KEEP || g_kept_bytes + size > RESULT_KEEP_BYTES)
+            out[n++] = take(0);
+        g_kept[g_nkept++] = p;
+        g_kept_bytes += size;
+        p = NULL;
+    }
     pthread_mutex_unlock(&g_kept_lock);
+    free(p);
     while (n > 0)
         free(out[--n]);
 }
 
-/* Gives every kept array back. */
-void rvsp_result_trim(void)
+/* A thread's one-shot context is made (1) or ends (-1). */
+void rvsp_result_user(int change)
+{
+    pthread_mutex_lock(&g_kept_lock);
+    g_users += change;
+    const int none = g_users == 0;
+    pthread_mutex_unlock(&g_kept_lock);
+    if (none)
+        rvsp_release_kept_results();
+}
+
+void rvsp_release_kept_results(void)
 {
     void *out[RESULT_KEEP];
     int n = 0;

@@ -29,7 +29,7 @@ void *rvsp_calloc(size_t n, size_t size);
 void *rvsp_realloc(void *p, size_t n);
 void *rvsp_result_alloc(size_t n);
 void rvsp_result_free(void *p);
-void rvsp_result_trim(void);
+void rvsp_result_user(int change);
 
 rvsp_status_t rvsp_dbuf_reserve(rvsp_dbuf_t *b, size_t bytes);
 void rvsp_dbuf_release(rvsp_dbuf_t *b);

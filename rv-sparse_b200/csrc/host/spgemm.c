@@ -49,7 +49,7 @@ static void ctx_free(void *p)
     if (c->stream)
         cudaStreamDestroy(c->stream);
     free(c);
-    rvsp_result_trim();
+    rvsp_result_user(-1);
 }
 
 static void ctx_key_init(void)
@@ -77,6 +77,7 @@ static rvsp_status_t get_ctx(oneshot_ctx_t **out)
             return rvsp_map_cuda(e);
         }
         pthread_setspecific(g_ctx_key, c);
+        rvsp_result_user(1);
     }
     *out = c;
     return RVSP_SUCCESS;

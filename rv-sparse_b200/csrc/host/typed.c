@@ -148,7 +148,7 @@ static void typed_ctx_free(void *p)
     if (c->stream)
         cudaStreamDestroy(c->stream);
     free(c);
-    rvsp_result_trim();
+    rvsp_result_user(-1);
 }
 
 static void typed_key_init(void) { pthread_key_create(&g_typed_key, typed_ctx_free); }
@@ -173,6 +173,7 @@ static rvsp_status_t typed_ctx(typed_ctx_t **out)
             return rvsp_map_cuda(e);
         }
         pthread_setspecific(g_typed_key, c);
+        rvsp_result_user(1);
     }
     *out = c;
     return RVSP_SUCCESS;

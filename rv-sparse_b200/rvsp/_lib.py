@@ -77,6 +77,7 @@ SIGNATURES = {
     "rvsp_csr_create": (_int, [_P(CsrMatrix), _i32, _i32, _i32, _vp, _vp, _vp, _int]),
     "rvsp_csr_validate": (_int, [_P(CsrMatrix)]),
     "rvsp_csr_destroy": (None, [_P(CsrMatrix)]),
+    "rvsp_release_kept_results": (None, []),
     "rvsp_spgemm_csr": (_int, [_P(CsrMatrix), _P(CsrMatrix), _P(CsrMatrix),
                                _P(SpgemmOptions)]),
     "rvsp_spgemm_descr_create": (_int, [_P(_vp)]),
@@ -152,8 +153,8 @@ SIGNATURES = {
     "rvsp_spgemm_set_row_tiles": (_int, [_vp, _i32]),
     "rvsp_spgemm_get_tiled_rows": (_int, [_vp, _P(_i32)]),
     "rvsp_cuda_plan_set_row_tiles": (_int, [_vp, _i32]),
-    "rvsp_cuda_plan_tiled_rows": (_i32, [_vp]),
     "rvsp_cuda_plan_set_stripe_memory": (_int, [_vp, _sz]),
+    "rvsp_cuda_plan_tiled_rows": (_i32, [_vp]),
     "rvsp_cuda_plan_set_shift_classes": (_int, [_vp, _i32]),
     "rvsp_cuda_plan_shift_rows": (_i32, [_vp]),
     "rvsp_spgemm_set_shift_classes": (_int, [_vp, _i32]),
