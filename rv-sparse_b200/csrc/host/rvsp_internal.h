@@ -30,6 +30,8 @@ void *rvsp_realloc(void *p, size_t n);
 void *rvsp_result_alloc(size_t n);
 void rvsp_result_free(void *p);
 void rvsp_result_user(int change);
+void *rvsp_numpy_handler(void);
+void *rvsp_numpy_array(void *const *api, int type, intptr_t n, void *p);
 
 rvsp_status_t rvsp_dbuf_reserve(rvsp_dbuf_t *b, size_t bytes);
 void rvsp_dbuf_release(rvsp_dbuf_t *b);
