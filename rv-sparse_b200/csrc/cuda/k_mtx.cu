@@ -241,6 +241,87 @@ int convert_left(const char *text, size_t len, int64_t pos, bool index, int32_t 
   return stop == buf + n ? 1 : -1;
 }
 
+rvsp_status_t status_of(cudaError_t e) {
+  return e == cudaErrorMemoryAllocation ? RVSP_ERROR_ALLOCATION_FAILED : RVSP_ERROR_DEVICE;
+}
+
+// The entries of text (at least one byte of it, and of limit) into row, col
+// and val of limit; *n_out of them.  *parsed stays 0 when the host parser has
+// to read it.
+rvsp_status_t parse_entries(cudaStream_t s, const char *text, size_t len, int fields,
+                            int64_t limit, int32_t *row, int32_t *col, float *val,
+                            int64_t *n_out, int *parsed) {
+  const int64_t chunks = static_cast<int64_t>((len + kMtxChunk - 1) / kMtxChunk);
+  const size_t padded = size_t(chunks) * kMtxChunk + kMtxHalo;
+  Scratch sc(s);
+  uint8_t *d_text = nullptr;
+  int32_t *counts = nullptr;
+  int64_t *first = nullptr, *partials = nullptr;
+  unsigned long long *meta = nullptr;  // tokens, tokens left
+  LeftToken *d_left = nullptr;
+  const size_t nc = size_t(chunks);
+  int64_t &n = *n_out;
+  cudaError_t e = sc.alloc(reinterpret_cast<void **>(&d_text), padded);
+  if (e == cudaSuccess) e = sc.alloc(reinterpret_cast<void **>(&counts), nc * sizeof(int32_t));
+  if (e == cudaSuccess) e = sc.alloc(reinterpret_cast<void **>(&first), nc * sizeof(int64_t));
+  if (e == cudaSuccess)
+    e = sc.alloc(reinterpret_cast<void **>(&partials),
+                 scan_partials_bytes(static_cast<int32_t>(chunks)));
+  if (e == cudaSuccess)
+    e = sc.alloc(reinterpret_cast<void **>(&meta), 2 * sizeof(unsigned long long));
+  if (e == cudaSuccess)
+    e = sc.alloc(reinterpret_cast<void **>(&d_left), kMaxLeft * sizeof(LeftToken));
+  if (e != cudaSuccess) return status_of(e);
+  cudaMemcpyAsync(d_text, text, len, cudaMemcpyHostToDevice, s);
+  cudaMemsetAsync(d_text + len, ' ', padded - len, s);
+  cudaMemsetAsync(meta, 0, 2 * sizeof(unsigned long long), s);
+  mtx_count_kernel<<<static_cast<unsigned>(chunks), kMtxThreads, 0, s>>>(d_text, counts);
+  launch_scan_i64(static_cast<int32_t>(chunks), counts, first, partials,
+                  reinterpret_cast<int64_t *>(meta), s);
+  if (fields == 2)
+    mtx_convert_kernel<2><<<static_cast<unsigned>(chunks), kMtxThreads, 0, s>>>(
+        d_text, first, limit, row, col, val, meta + 1, d_left);
+  else
+    mtx_convert_kernel<3><<<static_cast<unsigned>(chunks), kMtxThreads, 0, s>>>(
+        d_text, first, limit, row, col, val, meta + 1, d_left);
+  unsigned long long h_meta[2] = {0, 0};
+  e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(h_meta, meta, sizeof(h_meta), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) return status_of(e);
+  if (h_meta[1] > kMaxLeft) return RVSP_SUCCESS;
+  n = static_cast<int64_t>(h_meta[0]) / fields;
+  if (n > limit) n = limit;
+  if (h_meta[1] > 0) {
+    LeftToken left[kMaxLeft];
+    e = cudaMemcpyAsync(left, d_left, size_t(h_meta[1]) * sizeof(LeftToken),
+                        cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return status_of(e);
+    for (unsigned long long q = 0; q < h_meta[1]; ++q) {
+      const int64_t entry = left[q].index / fields;
+      const int f = static_cast<int>(left[q].index % fields);
+      int32_t iv = 0;
+      float fv = 0.0f;
+      const int r = convert_left(text, len, left[q].pos, f < 2, &iv, &fv);
+      if (r < 0) return RVSP_SUCCESS;
+      if (r == 0) {
+        if (entry < n) n = entry;
+        continue;
+      }
+      if (f < 2)
+        e = cudaMemcpyAsync((f == 0 ? row : col) + entry, &iv, sizeof(iv),
+                            cudaMemcpyHostToDevice, s);
+      else
+        e = cudaMemcpyAsync(val + entry, &fv, sizeof(fv), cudaMemcpyHostToDevice, s);
+      if (e != cudaSuccess) return status_of(e);
+    }
+  }
+  *parsed = 1;
+  return RVSP_SUCCESS;
+}
+
 }  // namespace
 
 }  // namespace rvsp
@@ -267,79 +348,31 @@ extern "C" rvsp_status_t rvsp_cuda_mtx_to_csr(void *stream, const char *text, si
   if (limit == 0 || chunks == 0 || chunks > INT32_MAX / 2 || point[0] != '.' || point[1])
     return RVSP_SUCCESS;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const size_t padded = size_t(chunks) * kMtxChunk + kMtxHalo;
-  Scratch sc(s);
-  uint8_t *d_text = nullptr;
-  int32_t *counts = nullptr, *row = nullptr, *col = nullptr;
-  float *val = nullptr;
-  int64_t *first = nullptr, *partials = nullptr;
-  unsigned long long *meta = nullptr;  // tokens, tokens left
-  LeftToken *d_left = nullptr;
-  const size_t nc = size_t(chunks), nl = size_t(limit);
-  cudaError_t e = sc.alloc(reinterpret_cast<void **>(&d_text), padded);
-  if (e == cudaSuccess) e = sc.alloc(reinterpret_cast<void **>(&counts), nc * sizeof(int32_t));
-  if (e == cudaSuccess) e = sc.alloc(reinterpret_cast<void **>(&first), nc * sizeof(int64_t));
-  if (e == cudaSuccess)
-    e = sc.alloc(reinterpret_cast<void **>(&partials),
-                 scan_partials_bytes(static_cast<int32_t>(chunks)));
-  if (e == cudaSuccess)
-    e = sc.alloc(reinterpret_cast<void **>(&meta), 2 * sizeof(unsigned long long));
-  if (e == cudaSuccess)
-    e = sc.alloc(reinterpret_cast<void **>(&d_left), kMaxLeft * sizeof(LeftToken));
-  if (e == cudaSuccess) e = sc.alloc(reinterpret_cast<void **>(&row), nl * sizeof(int32_t));
-  if (e == cudaSuccess) e = sc.alloc(reinterpret_cast<void **>(&col), nl * sizeof(int32_t));
-  if (e == cudaSuccess) e = sc.alloc(reinterpret_cast<void **>(&val), nl * sizeof(float));
-  if (e != cudaSuccess) {  // no room for the text: the host parser needs less
+  rvsp_status_t st = RVSP_SUCCESS;
+  {
+    Scratch entries(s);
+    int32_t *row = nullptr, *col = nullptr;
+    float *val = nullptr;
+    int64_t n = 0;
+    const size_t nl = size_t(limit);
+    cudaError_t e = entries.alloc(reinterpret_cast<void **>(&row), nl * sizeof(int32_t));
+    if (e == cudaSuccess)
+      e = entries.alloc(reinterpret_cast<void **>(&col), nl * sizeof(int32_t));
+    if (e == cudaSuccess) e = entries.alloc(reinterpret_cast<void **>(&val), nl * sizeof(float));
+    st = e == cudaSuccess ? parse_entries(s, text, len, fields, limit, row, col, val, &n, parsed)
+                          : status_of(e);
+    if (*parsed)  // (the text's memory is given back by now)
+      st = rvsp_cuda_coo_to_csr(stream, rows, cols, n, symmetric, row, col, val, c_row_ptr,
+                                c_col_out, c_val_out, c_nnz_out);
+  }
+  if (st == RVSP_ERROR_ALLOCATION_FAILED) {
+    // no room beside the text: the host parser needs less, and gets all of it
     cudaGetLastError();
-    return e == cudaErrorMemoryAllocation ? RVSP_SUCCESS : RVSP_ERROR_DEVICE;
+    *parsed = 0;
+    st = RVSP_SUCCESS;
+    const cudaMemPool_t pool = scratch_pool();
+    if (cudaStreamSynchronize(s) != cudaSuccess) return RVSP_ERROR_DEVICE;
+    if (pool) cudaMemPoolTrimTo(pool, 0);
   }
-  cudaMemcpyAsync(d_text, text, len, cudaMemcpyHostToDevice, s);
-  cudaMemsetAsync(d_text + len, ' ', padded - len, s);
-  cudaMemsetAsync(meta, 0, 2 * sizeof(unsigned long long), s);
-  mtx_count_kernel<<<static_cast<unsigned>(chunks), kMtxThreads, 0, s>>>(d_text, counts);
-  launch_scan_i64(static_cast<int32_t>(chunks), counts, first, partials,
-                  reinterpret_cast<int64_t *>(meta), s);
-  if (fields == 2)
-    mtx_convert_kernel<2><<<static_cast<unsigned>(chunks), kMtxThreads, 0, s>>>(
-        d_text, first, limit, row, col, val, meta + 1, d_left);
-  else
-    mtx_convert_kernel<3><<<static_cast<unsigned>(chunks), kMtxThreads, 0, s>>>(
-        d_text, first, limit, row, col, val, meta + 1, d_left);
-  unsigned long long h_meta[2] = {0, 0};
-  e = cudaGetLastError();
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(h_meta, meta, sizeof(h_meta), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return RVSP_ERROR_DEVICE;
-  if (h_meta[1] > kMaxLeft) return RVSP_SUCCESS;
-  int64_t n = static_cast<int64_t>(h_meta[0]) / fields;
-  if (n > limit) n = limit;
-  if (h_meta[1] > 0) {
-    LeftToken left[kMaxLeft];
-    e = cudaMemcpyAsync(left, d_left, size_t(h_meta[1]) * sizeof(LeftToken),
-                        cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return RVSP_ERROR_DEVICE;
-    for (unsigned long long q = 0; q < h_meta[1]; ++q) {
-      const int64_t entry = left[q].index / fields;
-      const int f = static_cast<int>(left[q].index % fields);
-      int32_t iv = 0;
-      float fv = 0.0f;
-      const int r = convert_left(text, len, left[q].pos, f < 2, &iv, &fv);
-      if (r < 0) return RVSP_SUCCESS;
-      if (r == 0) {
-        if (entry < n) n = entry;
-        continue;
-      }
-      if (f < 2)
-        e = cudaMemcpyAsync((f == 0 ? row : col) + entry, &iv, sizeof(iv),
-                            cudaMemcpyHostToDevice, s);
-      else
-        e = cudaMemcpyAsync(val + entry, &fv, sizeof(fv), cudaMemcpyHostToDevice, s);
-      if (e != cudaSuccess) return RVSP_ERROR_DEVICE;
-    }
-  }
-  *parsed = 1;
-  return rvsp_cuda_coo_to_csr(stream, rows, cols, n, symmetric, row, col, val, c_row_ptr,
-                              c_col_out, c_val_out, c_nnz_out);
+  return st;
 }
