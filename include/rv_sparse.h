@@ -219,6 +219,11 @@ rvsp_status_t rvsp_spgemm_get_tiled_rows(rvsp_spgemm_descr_t descr, int32_t *n_o
  * 1 (default) or 0.  Results are identical either way. */
 rvsp_status_t rvsp_spgemm_set_pattern_kernels(rvsp_spgemm_descr_t descr, int32_t enable);
 
+/* Long rows by column stripes (see rvsp_cuda_plan_set_stripes): 0 where that
+ * pays (the default), 1 never, 2 always, 3 where it pays for numeric-only
+ * computes; from the next work_estimation on. */
+rvsp_status_t rvsp_spgemm_set_stripes(rvsp_spgemm_descr_t descr, int32_t policy);
+
 /* Shift classes in work_estimation (see rvsp_cuda_plan_set_shift_classes):
  * 1 (default: where they pay), 2 (whenever rows are translates) or 0.
  * Results are identical either way. */

@@ -208,8 +208,13 @@ int32_t rvsp_cuda_plan_overflow_rows(rvsp_cuda_plan_t plan);
  * and 2 to time both accumulators on the same rows. */
 rvsp_status_t rvsp_cuda_plan_set_merge_policy(rvsp_cuda_plan_t plan, int32_t policy);
 
-/* Device memory that the stripe rows (rows of more than 1024 possible outputs,
- * B of at most 2^17 columns) of one analysis may take, from the next analysis
+/* Rows of more than 1024 possible outputs, for B of at most 2^17 columns, by
+ * column stripes: 0 where that pays by their number and length (the default),
+ * 1 never, 2 always, 3 where it pays for numeric-only repeats; from the next
+ * analysis on, with the same results. */
+rvsp_status_t rvsp_cuda_plan_set_stripes(rvsp_cuda_plan_t plan, int32_t policy);
+
+/* Device memory that the rows by column stripes of one analysis may take, from the next analysis
  * on: 3 GiB by default, and never more than a quarter of what is free where it
  * has to grow.  Rows without room take the block-per-row kernels, with the
  * same results.  The plan keeps what its analyses took. */

@@ -172,7 +172,7 @@ predict_kernel(Operands op, float b_mean_len, const float *__restrict__ params,
 //     (2^y0 - 1)) + kCapPad) with ub = min(ops, b_cols); warp hash with
 //     T >= 2 capacity slots up to 2048, the 8192-slot block hash up to 4096,
 //     else DENSE with capacity ub (never overflows); of the last two, rows
-//     are STRIPE8 or STRIPE with no slab slot when op.stripes.
+//     are STRIPE8 or STRIPE when op.stripes, for the pass below to decide.
 // A row whose nnz exceeds its capacity is caught by the fused kernel and
 // redone by the plain two-pass path.  Long rows are spread over the grid's
 // warps (R-MAT 2^14: 171 -> 34 us; a region's long rows used to meet on one).
@@ -183,9 +183,12 @@ __global__ void __launch_bounds__(kThreads)
 learned_plan_kernel(Operands op, float b_mean_len, const float *__restrict__ params,
                     float scale, bool merge_ok, int64_t *__restrict__ ops_out,
                     uint8_t *__restrict__ cls_out, int32_t *__restrict__ cap_out,
-                    int32_t *__restrict__ counts, int32_t *__restrict__ class_count) {
+                    int32_t *__restrict__ counts, int32_t *__restrict__ class_count,
+                    HeavyRows *__restrict__ heavy) {
   __shared__ float P[kMlpParamsPad];
   __shared__ int32_t s_cnt[kNumClasses];
+  __shared__ HeavyRows s_heavy;
+  if (threadIdx.x == 0) s_heavy = HeavyRows{0, 0, 0, 0};
   load_params_transposed(P, params);
   for (int c = threadIdx.x; c < kNumClasses; c += blockDim.x) s_cnt[c] = 0;
   __syncthreads();
@@ -207,9 +210,13 @@ learned_plan_kernel(Operands op, float b_mean_len, const float *__restrict__ par
       if (cap < 1) cap = 1;
       c = classify_row(nnz, ops, cap, false);
       if (c == kDense) cap = ub;
-      // counted exactly by the stripe pass, which needs no slab slot
       c = with_stripes(c, op.stripes);
-      if (c >= kStripe8) cap = 0;
+      if (c >= kStripe8) {
+        atomicAdd(&s_heavy.rows, 1ull);
+        atomicAdd(&s_heavy.ops, static_cast<unsigned long long>(ops));
+        atomicAdd(&s_heavy.nnz, static_cast<unsigned long long>(nnz));
+        atomicMax(&s_heavy.most, static_cast<unsigned long long>(ops));
+      }
     }
     ops_out[row] = ops;
     cls_out[row] = static_cast<uint8_t>(c);
@@ -290,6 +297,36 @@ learned_plan_kernel(Operands op, float b_mean_len, const float *__restrict__ par
   __syncthreads();
   for (int c = threadIdx.x; c < kNumClasses; c += blockDim.x)
     if (s_cnt[c]) atomicAdd(&class_count[c], s_cnt[c]);
+  if (threadIdx.x == 0 && s_heavy.rows) {
+    atomicAdd(&heavy->rows, s_heavy.rows);
+    atomicAdd(&heavy->ops, s_heavy.ops);
+    atomicAdd(&heavy->nnz, s_heavy.nnz);
+    atomicMax(&heavy->most, s_heavy.most);
+  }
+}
+
+// The heavy rows of the plan: where stripes pay they are counted exactly by the
+// stripe pass and need no slab slot, else they are B8192 and DENSE rows.
+__global__ void __launch_bounds__(kThreads)
+learned_heavy_kernel(int32_t n, HeavyRows *__restrict__ heavy, int32_t b_rows, int32_t b_cols,
+                     bool always, bool repeats, uint8_t *__restrict__ cls, int32_t *__restrict__ cap,
+                     int32_t *__restrict__ class_count) {
+  const HeavyRows h = *heavy;
+  if (h.rows == 0) return;
+  const bool pay = always || stripes_pay(h, b_rows, b_cols, repeats);
+  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) {
+    const int c = cls[i];
+    if (c >= kStripe8) {
+      if (pay) cap[i] = 0;
+      else cls[i] = static_cast<uint8_t>(c == kStripe8 ? kB8192 : kDense);
+    }
+  }
+  if (i == 0 && !pay) {
+    class_count[kB8192] += class_count[kStripe8];
+    class_count[kDense] += class_count[kStripe];
+    class_count[kStripe8] = class_count[kStripe] = 0;
+  }
 }
 
 // ---- training ----------------------------------------------------------------
@@ -443,10 +480,14 @@ void launch_predict(const Operands &op, float b_mean_len, const float *params,
 void launch_learned_plan(const Operands &op, float b_mean_len, const float *params,
                          float scale, bool merge_ok, int64_t *ops, uint8_t *cls,
                          int32_t *cap, int32_t *counts, int32_t *class_count,
+                         HeavyRows *heavy, int32_t b_rows, bool always, bool repeats,
                          int num_sms, cudaStream_t s) {
   const int grid = num_sms * 8;
   learned_plan_kernel<<<grid, kThreads, 0, s>>>(op, b_mean_len, params, scale, merge_ok,
-                                                ops, cls, cap, counts, class_count);
+                                                ops, cls, cap, counts, class_count, heavy);
+  if (op.stripes)
+    learned_heavy_kernel<<<(op.a_rows + kThreads - 1) / kThreads, kThreads, 0, s>>>(
+        op.a_rows, heavy, b_rows, op.b_cols, always, repeats, cls, cap, class_count);
 }
 
 void launch_mlp_grad(const float *params, const float *feat, const float *target,

@@ -41,11 +41,20 @@ __device__ __forceinline__ void count_class(int32_t *s_cnt, bool take, int c) {
   if (take && (peers & lanemask_lt()) == 0) atomicAdd(&s_cnt[c], __popc(peers));
 }
 
+__device__ __forceinline__ void add_heavy(HeavyRows *heavy, int rows, long long ops, int32_t nnz,
+                                          unsigned long long most) {
+  atomicAdd(&heavy->rows, static_cast<unsigned long long>(rows));
+  atomicAdd(&heavy->ops, static_cast<unsigned long long>(ops));
+  atomicAdd(&heavy->nnz, static_cast<unsigned long long>(nnz));
+  if (most > *reinterpret_cast<volatile unsigned long long *>(&heavy->most))
+    atomicMax(&heavy->most, most);
+}
+
 __global__ void __launch_bounds__(kThreads)
 rowstats_kernel(Operands op, int64_t *__restrict__ ops, uint8_t *__restrict__ cls,
                 int32_t *__restrict__ counts, int32_t *__restrict__ class_count,
                 int32_t *__restrict__ long_rows, int32_t *__restrict__ long_count,
-                int32_t max_long) {
+                int32_t max_long, HeavyRows *__restrict__ heavy) {
   __shared__ int32_t s_cnt[kNumClasses];
   for (int c = threadIdx.x; c < kNumClasses; c += blockDim.x) s_cnt[c] = 0;
   __syncthreads();
@@ -53,6 +62,8 @@ rowstats_kernel(Operands op, int64_t *__restrict__ ops, uint8_t *__restrict__ cl
   const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   bool take = false;
   int c = kEmpty_;
+  long long row_ops = 0;
+  int32_t row_nnz = 0;
   if (i < op.a_rows) {
     int32_t p0, p1;
     row_range(op, i, p0, p1);
@@ -79,7 +90,19 @@ rowstats_kernel(Operands op, int64_t *__restrict__ ops, uint8_t *__restrict__ cl
       cls[i] = static_cast<uint8_t>(c);
       if (c == kEmpty_) counts[i] = 0;
       take = true;
+      if (c >= kStripe8) {
+        row_ops = s;
+        row_nnz = p1 - p0;
+      }
     }
+  }
+  const unsigned in_heavy = __ballot_sync(kFull, row_nnz > 0);
+  if (in_heavy) {
+    const long long sum = warp_sum64(row_ops);
+    const int32_t nnz = warp_sum(row_nnz);
+    const unsigned most =
+        __reduce_max_sync(kFull, static_cast<unsigned>(min(row_ops, 0xffffffffll)));
+    if (lane_id() == 0) add_heavy(heavy, __popc(in_heavy), sum, nnz, most);
   }
   count_class(s_cnt, take, c);
   __syncthreads();
@@ -93,7 +116,8 @@ rowstats_long_kernel(Operands op, const int32_t *__restrict__ long_rows,
                      const int32_t *__restrict__ long_count,
                      int64_t *__restrict__ ops, uint8_t *__restrict__ cls,
                      int32_t *__restrict__ counts,
-                     int32_t *__restrict__ class_count) {
+                     int32_t *__restrict__ class_count,
+                     HeavyRows *__restrict__ heavy) {
   const int32_t n_long = *long_count;
   const int lane = lane_id();
   const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -121,6 +145,7 @@ rowstats_long_kernel(Operands op, const int32_t *__restrict__ long_rows,
       cls[i] = static_cast<uint8_t>(c);
       if (c == kEmpty_) counts[i] = 0;
       atomicAdd(&class_count[c], 1);
+      if (c >= kStripe8) add_heavy(heavy, 1, s, p1 - p0, s);
     }
   }
 }
@@ -174,21 +199,21 @@ void launch_class_offsets(const int32_t *count, int32_t *off, cudaStream_t s) {
 
 void launch_rowstats(const Operands &op, int64_t *ops, uint8_t *cls,
                      int32_t *counts, int32_t *class_count, int32_t *long_rows,
-                     int32_t *long_count, int32_t max_long, cudaStream_t s) {
+                     int32_t *long_count, int32_t max_long, HeavyRows *heavy, cudaStream_t s) {
   const int grid = (op.a_rows + kThreads - 1) / kThreads;
   rowstats_kernel<<<grid, kThreads, 0, s>>>(op, ops, cls, counts, class_count,
-                                             long_rows, long_count, max_long);
+                                             long_rows, long_count, max_long, heavy);
 }
 
 void launch_rowstats_long(const Operands &op, const int32_t *long_rows,
                           const int32_t *long_count, int64_t *ops, uint8_t *cls,
-                          int32_t *counts, int32_t *class_count, int num_sms,
-                          cudaStream_t s) {
+                          int32_t *counts, int32_t *class_count, HeavyRows *heavy,
+                          int num_sms, cudaStream_t s) {
   // The kernel reads the number of long rows on the device, so no host
   // round trip is needed; the grid strides over however many there are.
   const int grid = num_sms * 8;
   rowstats_long_kernel<<<grid, kThreads, 0, s>>>(op, long_rows, long_count, ops,
-                                                 cls, counts, class_count);
+                                                 cls, counts, class_count, heavy);
 }
 
 void launch_scatter_rows(int32_t n, const uint8_t *cls, const int32_t *class_off,

@@ -66,11 +66,11 @@ namespace rvsp {
 
 namespace {
 
-constexpr int kAcc = 4096;           // accumulator slots of a block (16 KB)
+constexpr int kAcc = kStripeAcc;     // accumulator slots of a block (16 KB)
 constexpr int kStripeWords = 64;     // words (of 32 columns) a stripe spans at most
 constexpr int kItemWords = 2048;     // bitmap words a block can hold for one item
 constexpr int kStripeShares = 32;    // equal shares of B's entries
-constexpr int kItemOps = 32768;      // products an item aims at
+constexpr int kItemOps = kStripeItemOps;  // products an item aims at
 constexpr int kTaskOps = 1 << 16;    // products of a part of a cut row (count)
 constexpr int kSplitTasks = 1 << 15; // parts of cut rows at most
 constexpr int kPtrThreads = 256;

@@ -7,6 +7,8 @@
 #include <vector>
 #include <cuda_runtime.h>
 
+#include "stripe_rule.cuh"
+
 struct rvsp_mlp;
 
 namespace rvsp {
@@ -28,8 +30,8 @@ const float *mlp_device_params(const rvsp_mlp *m);
 //   B8192   one 256-thread block, hash table of 8192 slots (bound <= 4096)
 //   DENSE   one 512-thread block, dense accumulator over all of B's columns
 //   STRIPE8, STRIPE  the B8192 and DENSE rows of a product whose B suits
-//           column stripes: a warp per run of stripes (k_stripe.cu); reported
-//           as the classes they come from
+//           column stripes: a warp per run of stripes (k_stripe.cu), where that
+//           pays (stripe_rule.cuh); reported as the classes they come from
 enum RowClass : int {
   kEmpty_ = 0,
   kM4,
@@ -152,14 +154,15 @@ struct FusedOut {
 
 // ---- k_rowstats.cu ---------------------------------------------------------
 // ops[i] = sum of B row lengths over A row i; cls[i] = symbolic class of the
-// row; class_count[c] += rows per class; counts[i] = 0 for empty rows.
+// row; class_count[c] += rows per class; counts[i] = 0 for empty rows.  *heavy (zeroed
+// by the caller): the STRIPE rows.
 void launch_rowstats(const Operands &op, int64_t *ops, uint8_t *cls,
                      int32_t *counts, int32_t *class_count, int32_t *long_rows,
-                     int32_t *long_count, int32_t max_long, cudaStream_t s);
+                     int32_t *long_count, int32_t max_long, HeavyRows *heavy, cudaStream_t s);
 void launch_rowstats_long(const Operands &op, const int32_t *long_rows,
                           const int32_t *long_count, int64_t *ops, uint8_t *cls,
-                          int32_t *counts, int32_t *class_count, int num_sms,
-                          cudaStream_t s);
+                          int32_t *counts, int32_t *class_count, HeavyRows *heavy,
+                          int num_sms, cudaStream_t s);
 // off[c] = exclusive prefix of count over the non-empty classes.
 void launch_class_offsets(const int32_t *count, int32_t *off, cudaStream_t s);
 // rows_by_class[class_off[c] + r] = i for every non-empty row i of class c.
@@ -602,10 +605,13 @@ void launch_features(const Operands &op, float b_mean_len, float *feat,
 void launch_predict(const Operands &op, float b_mean_len, const float *params,
                     float2 *pred, int64_t *ops, int num_sms, cudaStream_t s);
 // Learned binning for the fused pass: ops, class and slab capacity per row
-// (counts[row] = 0 for empty rows) and rows per class.
+// (counts[row] = 0 for empty rows) and rows per class.  The B8192 and DENSE
+// rows are STRIPE rows without a slab slot where stripes pay (with op.stripes,
+// or always; *heavy, zeroed by the caller, holds them).
 void launch_learned_plan(const Operands &op, float b_mean_len, const float *params,
                          float scale, bool merge_ok, int64_t *ops, uint8_t *cls,
                          int32_t *cap, int32_t *counts, int32_t *class_count,
+                         HeavyRows *heavy, int32_t b_rows, bool always, bool repeats,
                          int num_sms, cudaStream_t s);
 // grad (kMlpTrained floats, accumulated) and *loss_sum (accumulated) of the
 // mean loss over n_total samples, for samples [0, n).

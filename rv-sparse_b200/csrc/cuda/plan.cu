@@ -96,7 +96,12 @@ constexpr int kLongCount = 6 * kNumClasses + 1;
 constexpr int kRetryCount = 6 * kNumClasses + 2;  // two: W1024, W2048 retry lists
 constexpr int kShiftMembers = 6 * kNumClasses + 4;  // shift-class member rows
 constexpr int kShiftNpat = 6 * kNumClasses + 5;     // shift-class pattern candidates
-constexpr int kMiscWords = 6 * kNumClasses + 6;
+constexpr int kHeavy = 6 * kNumClasses + 6;  // a HeavyRows
+constexpr int kMiscWords = kHeavy + sizeof(HeavyRows) / sizeof(int32_t);
+static_assert(kHeavy % 2 == 0, "aligned for 64 bits");
+// Stripes for the heavy rows: where they pay, never, always, where they pay for
+// numeric-only repeats.
+constexpr int kStripesAuto = 0, kStripesNever = 1, kStripesAlways = 2, kStripesRepeats = 3;
 // A map shared by at least this many rows gets a term table.
 constexpr int32_t kPatMinShare = 16;
 constexpr int kPatCountWords = 4 + kNumClasses;
@@ -280,6 +285,7 @@ struct rvsp_cuda_plan {
   StripeShape sp;
   int sp_ready = 0;
   size_t stripe_max = kStripeBytesMax;  // bytes
+  int32_t stripe_policy = kStripesAuto;
   int64_t sp_cap = 0;
   DevArray<int32_t> sp_hist, sp_bound, sp_ptr, sp_gpre, sp_soff, sp_hslot, sp_done;
   DevArray<int32_t> sp_cnt;  // items from the front, from the back, queue head
@@ -446,6 +452,8 @@ struct Lanes {
   }
   ~Lanes() { join(); }
 };
+
+HeavyRows *heavy_rows(int32_t *misc) { return reinterpret_cast<HeavyRows *>(misc + kHeavy); }
 
 // Whether a census has rows in several classes that launch of their own.
 bool several_classes(const int32_t *count) {
@@ -825,7 +833,7 @@ rvsp_status_t symbolic_impl(rvsp_cuda_plan_t p, cudaStream_t s, int32_t a_rows,
   p->analysed = 0;
   p->rmap_state = 0;
   p->rmap_col = nullptr;
-  p->sp = stripe_shape(b_rows, b_cols);
+  p->sp = p->stripe_policy == kStripesNever ? StripeShape() : stripe_shape(b_rows, b_cols);
   p->sp_ready = 0;
   const size_t n = static_cast<size_t>(a_rows);
 
@@ -884,9 +892,9 @@ rvsp_status_t symbolic_impl(rvsp_cuda_plan_t p, cudaStream_t s, int32_t a_rows,
   {
     PhaseScope ph(p, s, RVSP_PHASE_ROWSTATS);
     launch_rowstats(op, p->ops.p, p->cls.p, p->counts.p, misc + kSymCount,
-                    p->long_rows.p, misc + kLongCount, a_rows, s);
+                    p->long_rows.p, misc + kLongCount, a_rows, heavy_rows(misc), s);
     launch_rowstats_long(op, p->long_rows.p, misc + kLongCount, p->ops.p, p->cls.p,
-                         p->counts.p, misc + kSymCount, p->num_sms, s);
+                         p->counts.p, misc + kSymCount, heavy_rows(misc), p->num_sms, s);
     ph.launches = 2;
     if (shift) {
       // Shift classes: the probe decides on the device and one small read
@@ -1047,9 +1055,12 @@ cudaError_t symbolic_rest(rvsp_cuda_plan *p, cudaStream_t s, const Operands &op,
     }
     const RowList sr = stripe_rows(p->sym_count, sym_off, whole, p->rows_sym.p);
     if (sr.n > 0) {
-      e = count_stripe_rows(p, op, b_rows, sr.rows, sr.n, s);
+      if (p->stripe_policy == kStripesAlways ||
+          stripes_pay(*heavy_rows(p->h_misc), b_rows, b_cols,
+                      p->stripe_policy == kStripesRepeats))
+        e = count_stripe_rows(p, op, b_rows, sr.rows, sr.n, s);
       if (e != cudaSuccess) return e;
-      // without room for their bitmaps they are heavy rows (either class)
+      // else, or without room, they take the block kernels (either class)
       ph.launches += p->sp_ready ? 5 : launch_class(kStripe8, sr.rows, sr.n, s);
     }
   }
@@ -1131,7 +1142,7 @@ rvsp_status_t rvsp_cuda_learned_symbolic(
   Operands op{a_rows, b_cols, a_row_ptr, a_col_idx, a_values,
               b_row_ptr, b_col_idx, b_values,
               merge_allowed(p->merge_policy, a_rows)};
-  p->sp = stripe_shape(b_rows, b_cols);
+  p->sp = p->stripe_policy == kStripesNever ? StripeShape() : stripe_shape(b_rows, b_cols);
   p->sp_ready = 0;
   op.stripes = p->sp.on;
   int32_t *misc = p->misc.p;
@@ -1142,9 +1153,11 @@ rvsp_status_t rvsp_cuda_learned_symbolic(
     const float b_mean = static_cast<float>(b_nnz) / static_cast<float>(b_rows);
     launch_learned_plan(op, b_mean, mlp_device_params(model), capacity_scale,
                         op.merge_ok, p->ops.p, p->cls.p, p->cap.p,
-                        p->counts.p, misc + kSymCount, p->num_sms, s);
+                        p->counts.p, misc + kSymCount, heavy_rows(misc), b_rows,
+                        p->stripe_policy == kStripesAlways,
+                        p->stripe_policy == kStripesRepeats, p->num_sms, s);
     launch_scan_i64(a_rows, p->cap.p, p->slab_off.p, p->partials.p, p->total.p, s);
-    ph.launches = 4;
+    ph.launches = op.stripes ? 5 : 4;
   }
   cudaMemcpyAsync(p->h_misc, misc, kNumClasses * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
   cudaMemcpyAsync(p->h_total, p->total.p, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
@@ -1317,6 +1330,13 @@ rvsp_status_t rvsp_cuda_plan_set_merge_policy(rvsp_cuda_plan_t p, int32_t policy
   if (!p) return RVSP_ERROR_NULL_POINTER;
   if (policy < kMergeAuto || policy > kMergeAlways) return RVSP_ERROR_INVALID_ARGUMENT;
   p->merge_policy = policy;
+  return RVSP_SUCCESS;
+}
+
+rvsp_status_t rvsp_cuda_plan_set_stripes(rvsp_cuda_plan_t p, int32_t policy) {
+  if (!p) return RVSP_ERROR_NULL_POINTER;
+  if (policy < kStripesAuto || policy > kStripesRepeats) return RVSP_ERROR_INVALID_ARGUMENT;
+  p->stripe_policy = policy;
   return RVSP_SUCCESS;
 }
 

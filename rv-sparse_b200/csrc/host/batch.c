@@ -484,6 +484,8 @@ static rvsp_status_t pack_group(rvsp_spgemm_batch_t b, batch_group_t *g)
     if (st == RVSP_SUCCESS)
         st = rvsp_cuda_plan_set_merge_policy(g->plan, b->merge_policy);
     if (st == RVSP_SUCCESS)
+        st = rvsp_cuda_plan_set_stripes(g->plan, 3); /* a batch is there to be repeated */
+    if (st == RVSP_SUCCESS)
         st = rvsp_cuda_batch_pack(b->stream, (const rvsp_cuda_batch_item_t *)b->d_items.p +
                                                  g->first,
                                   (const rvsp_cuda_batch_offset_t *)g->off.p, g->count, 1,

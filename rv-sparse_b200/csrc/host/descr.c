@@ -38,6 +38,7 @@ struct rvsp_spgemm_descr {
     int32_t merge_policy;
     int32_t row_tiles;
     int32_t shift_classes;
+    int32_t stripes;
     int32_t pattern_kernels;
 
     int32_t c_nnz;
@@ -117,6 +118,16 @@ rvsp_status_t rvsp_spgemm_set_row_tiles(rvsp_spgemm_descr_t d, int32_t enable)
         return RVSP_ERROR_INVALID_ARGUMENT;
     d->row_tiles = enable;
     return d->plan ? rvsp_cuda_plan_set_row_tiles(d->plan, enable) : RVSP_SUCCESS;
+}
+
+rvsp_status_t rvsp_spgemm_set_stripes(rvsp_spgemm_descr_t d, int32_t policy)
+{
+    if (d == NULL)
+        return RVSP_ERROR_NULL_POINTER;
+    if (policy < 0 || policy > 3)
+        return RVSP_ERROR_INVALID_ARGUMENT;
+    d->stripes = policy;
+    return d->plan ? rvsp_cuda_plan_set_stripes(d->plan, policy) : RVSP_SUCCESS;
 }
 
 rvsp_status_t rvsp_spgemm_set_shift_classes(rvsp_spgemm_descr_t d, int32_t enable)
@@ -284,6 +295,8 @@ static rvsp_status_t ensure_device(rvsp_spgemm_descr_t d)
     rvsp_status_t st = rvsp_cuda_plan_set_row_tiles(d->plan, d->row_tiles);
     if (st == RVSP_SUCCESS)
         st = rvsp_cuda_plan_set_shift_classes(d->plan, d->shift_classes);
+    if (st == RVSP_SUCCESS)
+        st = rvsp_cuda_plan_set_stripes(d->plan, d->stripes);
     if (st == RVSP_SUCCESS)
         st = rvsp_cuda_plan_set_pattern_kernels(d->plan, d->pattern_kernels);
     if (st != RVSP_SUCCESS)

@@ -154,6 +154,8 @@ SIGNATURES = {
     "rvsp_spgemm_get_tiled_rows": (_int, [_vp, _P(_i32)]),
     "rvsp_cuda_plan_set_row_tiles": (_int, [_vp, _i32]),
     "rvsp_cuda_plan_set_stripe_memory": (_int, [_vp, _sz]),
+    "rvsp_cuda_plan_set_stripes": (_int, [_vp, _i32]),
+    "rvsp_spgemm_set_stripes": (_int, [_vp, _i32]),
     "rvsp_cuda_plan_tiled_rows": (_i32, [_vp]),
     "rvsp_cuda_plan_set_shift_classes": (_int, [_vp, _i32]),
     "rvsp_cuda_plan_shift_rows": (_i32, [_vp]),

@@ -335,6 +335,11 @@ class Descriptor:
         L.check(self.lib.rvsp_spgemm_set_pattern_kernels(self.h, int(bool(enable))),
                 "set_pattern_kernels")
 
+    def set_stripes(self, policy: int):
+        """Long rows by column stripes: 0 where that pays, 1 never, 2 always,
+        3 where it pays for numeric-only computes."""
+        L.check(self.lib.rvsp_spgemm_set_stripes(self.h, policy), "set_stripes")
+
     def set_shift_classes(self, enable):
         """Shift classes in work_estimation: False/0 off, True/1 where they pay
         (the default: large matrices of costly rows), 2 on any matrix whose

@@ -4,7 +4,8 @@ A call whose row pointers do not give a heavy row its analysed length reports
 it and leaves that row alone, whether the row grew or shrank, in a fill and in
 a numeric-only repeat.  B may have more than 2^30 entries.  All that the rows
 keep counts against their memory, and rows without room give the same results
-by the block-per-row kernels, on the plain and on the learned path.
+by the block-per-row kernels, on the plain and on the learned path, as do rows
+too few for stripes to pay.
 """
 import ctypes as C
 
@@ -47,6 +48,7 @@ class _Plan:
         self.a, self.b = DeviceCSR.from_host(A), DeviceCSR.from_host(B)
         self.h = C.c_void_p()
         L.check(self.lib.rvsp_cuda_plan_create(C.byref(self.h)), "plan")
+        L.check(self.lib.rvsp_cuda_plan_set_stripes(self.h, 2), "always")
         self.rp = torch.zeros(A.rows + 1, dtype=torch.int32, device="cuda")
 
     def learned(self, model, scale=1.0):
@@ -181,11 +183,14 @@ def test_rows_without_room(path, b_cols):
     assert (np.diff(rp) > 1024).sum() > 1
     p = _Plan(A, B)
     model = RowModel(path=weights_for("rmat"))
-    for limit in (0, 1 << 30, 0):
+    # (limit, policy): no room, room, no room, never, where it pays (not here)
+    for limit, policy in ((0, 2), (1 << 30, 2), (0, 2), (1 << 30, 1), (1 << 30, 0)):
+        L.check(p.lib.rvsp_cuda_plan_set_stripes(p.h, policy), "set_stripes")
         L.check(p.lib.rvsp_cuda_plan_set_stripe_memory(p.h, limit), "set_stripe_memory")
         assert (p.learned(model) if path == "learned" else p.analyse()) == ci.size
         assert np.array_equal(p.rp.cpu().numpy(), rp)
-        if path == "learned":  # without room they are redone by the plain passes
+        if path == "learned" and policy == 2:
+            # without room they are redone by the plain passes
             assert (p.lib.rvsp_cuda_plan_overflow_rows(p.h) >= 2) == (limit == 0)
         c_ci = torch.zeros(ci.size, dtype=torch.int32, device="cuda")
         c_cv = torch.zeros(ci.size, dtype=torch.float32, device="cuda")
