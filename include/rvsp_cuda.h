@@ -42,7 +42,8 @@ void rvsp_cuda_plan_destroy(rvsp_cuda_plan_t plan);
  * c_row_ptr[0..a_rows] (device) and the int64 total.  ALLOCATION_FAILED when
  * the total exceeds INT32_MAX, as in the reference.  One host round trip
  * when every non-empty row falls in the merge classes (at most 16 A
- * nonzeros and 128 products; under the automatic merge policy only when A
+ * nonzeros and 128 products, or 256 where a quarter of A's nonzeros follow
+ * one another; under the automatic merge policy only when A
  * has at least 32768 rows), two otherwise.
  * Synchronizes `stream`. */
 rvsp_status_t rvsp_cuda_symbolic(rvsp_cuda_plan_t plan, void *stream,
@@ -203,7 +204,8 @@ rvsp_status_t rvsp_cuda_learned_symbolic(
 int32_t rvsp_cuda_plan_overflow_rows(rvsp_cuda_plan_t plan);
 
 /* Which rows may use the thread-per-row merge accumulator (rows of at most
- * 16 A nonzeros and 128 products): 0 automatic (when the matrix has at least
+ * 16 A nonzeros and 128 products; 256 in the symbolic pass where a quarter of
+ * A's nonzeros follow one another): 0 automatic (when the matrix has at least
  * 32768 rows), 1 never, 2 whenever a row is eligible.  The autotuner uses 1
  * and 2 to time both accumulators on the same rows. */
 rvsp_status_t rvsp_cuda_plan_set_merge_policy(rvsp_cuda_plan_t plan, int32_t policy);

@@ -54,7 +54,8 @@ __global__ void __launch_bounds__(kThreads)
 rowstats_kernel(Operands op, int64_t *__restrict__ ops, uint8_t *__restrict__ cls,
                 int32_t *__restrict__ counts, int32_t *__restrict__ class_count,
                 int32_t *__restrict__ long_rows, int32_t *__restrict__ long_count,
-                int32_t max_long, HeavyRows *__restrict__ heavy) {
+                int32_t max_long, HeavyRows *__restrict__ heavy,
+                const int32_t *__restrict__ near) {
   __shared__ int32_t s_cnt[kNumClasses];
   for (int c = threadIdx.x; c < kNumClasses; c += blockDim.x) s_cnt[c] = 0;
   __syncthreads();
@@ -84,7 +85,8 @@ rowstats_kernel(Operands op, int64_t *__restrict__ ops, uint8_t *__restrict__ cl
           if (e + u < p1 - p0) s += b_len(op, k[u]);
       }
       c = with_stripes(
-          classify_row(p1 - p0, s, s < op.b_cols ? s : op.b_cols, op.merge_ok),
+          classify_row(p1 - p0, s, s < op.b_cols ? s : op.b_cols, op.merge_ok,
+                       near && *near ? kMergeNearOps : kMergeMaxOps),
           op.stripes);
       ops[i] = s;
       cls[i] = static_cast<uint8_t>(c);
@@ -199,10 +201,11 @@ void launch_class_offsets(const int32_t *count, int32_t *off, cudaStream_t s) {
 
 void launch_rowstats(const Operands &op, int64_t *ops, uint8_t *cls,
                      int32_t *counts, int32_t *class_count, int32_t *long_rows,
-                     int32_t *long_count, int32_t max_long, HeavyRows *heavy, cudaStream_t s) {
+                     int32_t *long_count, int32_t max_long, HeavyRows *heavy,
+                     const int32_t *near, cudaStream_t s) {
   const int grid = (op.a_rows + kThreads - 1) / kThreads;
   rowstats_kernel<<<grid, kThreads, 0, s>>>(op, ops, cls, counts, class_count,
-                                             long_rows, long_count, max_long, heavy);
+                                             long_rows, long_count, max_long, heavy, near);
 }
 
 void launch_rowstats_long(const Operands &op, const int32_t *long_rows,

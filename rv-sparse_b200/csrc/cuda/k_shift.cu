@@ -114,8 +114,11 @@ __device__ __forceinline__ bool shiftable(int32_t na, int64_t ops) {
 }
 
 // Probe: keys of `samples` rows spread over A, computed directly (B keys on
-// the fly).  Warp per sampled row.  Reads nothing when the structure check
-// queued before it failed.
+// the fly), and behind them the rows' products, with their nonzeros in the
+// column after the one before (kNearShift) and their nonzeros (kNnzShift).
+// Warp per sampled row.  Reads nothing when the structure check queued before
+// it failed.
+constexpr int kNearShift = 48, kNnzShift = 56;
 __global__ void __launch_bounds__(kThreads)
 shift_probe_kernel(Operands op, int32_t samples, unsigned long long *__restrict__ keys,
                    CheckGuard guard) {
@@ -147,6 +150,9 @@ shift_probe_kernel(Operands op, int32_t samples, unsigned long long *__restrict_
   // 27-point stencil, 11 us now), its entries kProbeUnroll at a time; the
   // whole warp takes the longer ones.
   const long long ops = warp_sum64(len);
+  const int32_t before = __shfl_up_sync(kFull, k, 1);
+  const int near =
+      __popc(__ballot_sync(kFull, lane > 0 && lane < na && k == before + 1));
   unsigned long long key = 0;
   if (ops <= kShiftMaxOps) {
     unsigned long long h = 0;
@@ -172,7 +178,9 @@ shift_probe_kernel(Operands op, int32_t samples, unsigned long long *__restrict_
   }
   if (lane == 0) {
     keys[w] = key;
-    keys[samples + w] = static_cast<unsigned long long>(ops);
+    keys[samples + w] = static_cast<unsigned long long>(ops) |
+                        static_cast<unsigned long long>(near) << kNearShift |
+                        static_cast<unsigned long long>(na) << kNnzShift;
   }
 }
 
@@ -182,7 +190,9 @@ shift_probe_kernel(Operands op, int32_t samples, unsigned long long *__restrict_
 // and the sampled rows average at least min_mean_ops products (the caller's
 // bar: rows of few products are cheap on the merge kernels, and the
 // analysis and the tile builds would cost more than they save in a single
-// product).  *on stays 0 when the structure check failed.
+// product).  on[1]: that is not so, and at least a quarter of the sampled rows'
+// nonzeros lie in the column after the one before.  Both stay 0 when the
+// structure check failed.
 __global__ void __launch_bounds__(1024)
 shift_decide_kernel(const unsigned long long *__restrict__ keys, int32_t samples,
                     int32_t min_mean_ops, int32_t *__restrict__ on, CheckGuard guard) {
@@ -191,19 +201,29 @@ shift_decide_kernel(const unsigned long long *__restrict__ keys, int32_t samples
   __shared__ uint8_t shared_key[kSlots];
   __shared__ int32_t dup;
   __shared__ unsigned long long total_ops;
+  __shared__ int32_t far;  // nonzeros less four times the near ones
   const int tid = threadIdx.x;
   if (tid == 0) {
-    *on = 0;
+    on[0] = on[1] = 0;
     dup = 0;
     total_ops = 0;
+    far = 0;
   }
   if (guard.failed()) return;
   {
     unsigned long long o = 0;
-    for (int t = tid; t < samples; t += blockDim.x) o += keys[samples + t];
+    int32_t f = 0;
+    for (int t = tid; t < samples; t += blockDim.x) {
+      const unsigned long long x = keys[samples + t];
+      o += x & ((1ull << kNearShift) - 1);
+      f += static_cast<int32_t>(x >> kNnzShift) -
+           4 * static_cast<int32_t>(x >> kNearShift & ((1 << (kNnzShift - kNearShift)) - 1));
+    }
     for (int d = 16; d; d >>= 1) o += __shfl_xor_sync(kFull, o, d);
+    f = warp_sum(f);
     __syncthreads();
     if (lane_id() == 0 && o) atomicAdd(&total_ops, o);
+    if (lane_id() == 0 && f) atomicAdd(&far, f);
   }
   for (int t = tid; t < kSlots; t += blockDim.x) {
     sk[t] = 0ull;
@@ -242,12 +262,14 @@ shift_decide_kernel(const unsigned long long *__restrict__ keys, int32_t samples
   mine = warp_sum(mine);
   if (lane_id() == 0 && mine) atomicAdd(&dup, mine);
   __syncthreads();
-  if (tid == 0)
-    *on = (2 * dup >= samples &&
+  if (tid == 0) {
+    on[0] = (2 * dup >= samples &&
            total_ops >= static_cast<unsigned long long>(min_mean_ops) *
                             static_cast<unsigned long long>(samples))
               ? 1
               : 0;
+    on[1] = !on[0] && total_ops > 0 && far <= 0;
+  }
 }
 
 // Gated fills.

@@ -57,6 +57,19 @@ enum RowClass : int {
 // repeat at 2^15 6.4 ms against 3.1, 2.9, 2.6 and 2.6.  Mesh rows (25
 // products) stay far below any of them.
 constexpr int kMergeMaxOps = 128;
+// Nonzeros in consecutive columns of A select neighbouring rows of B, whose
+// columns, in a mesh's matrix, are mostly the same: the hash pass inserts each
+// of few columns many times, while the merge takes them together.  Where a
+// quarter of the nonzeros (of the rows that the shift probe samples) are like
+// that, the symbolic pass merges rows of up to twice the products.  80^3 grid,
+// 13 points with 3% of the entries dropped (159 products, 70 outputs a row):
+// product 1516 -> 1316 us; 400,000 uniform rows of 12 would take 1963 us instead
+// of 1778.  (By its own nonzeros, row by row, a band of 15 in 60 columns took
+// 1162 instead of 1045: some rows of a warp in each pass.  In the numeric pass
+// a repeat would lose what the product gains: 1316 -> 1141, 515 -> 556.  Where
+// shift classes take most rows, the few that are left, a thread each, would
+// hold the others up: 127x90x113 27-point stencil 1469 -> 1504.)
+constexpr int kMergeNearOps = 256;
 constexpr int kMergeMaxNnz = 16;
 constexpr int kMergeThreads = 128;
 // The merge classes put one row on one thread; below this many rows the GPU
@@ -74,11 +87,12 @@ constexpr int64_t kSmemBitmapMaxCols = 48 * 1024 * 32;
 // rowstats hands rows with more A nonzeros than this to a warp-per-row pass.
 constexpr int kLongRowNnz = 64;
 
-// merge_ok: the matrix has at least kMergeMinRows rows.
-__host__ __device__ inline int classify_row(int32_t nnz_a, int64_t ops,
-                                            int64_t bound, bool merge_ok) {
+// merge_ok: the matrix has at least kMergeMinRows rows; merge_ops: the most
+// products of a merge row.
+__host__ __device__ inline int classify_row(int32_t nnz_a, int64_t ops, int64_t bound,
+                                            bool merge_ok, int merge_ops = kMergeMaxOps) {
   if (ops <= 0) return kEmpty_;
-  if (merge_ok && nnz_a <= kMergeMaxNnz && ops <= kMergeMaxOps)
+  if (merge_ok && nnz_a <= kMergeMaxNnz && ops <= merge_ops)
     return nnz_a <= 4 ? kM4 : nnz_a <= 8 ? kM8 : kM16;
   const int64_t need = 2 * bound;
   for (int l = kWarpHashMinLog2; l <= kWarpHashMaxLog2; ++l)
@@ -155,10 +169,12 @@ struct FusedOut {
 // ---- k_rowstats.cu ---------------------------------------------------------
 // ops[i] = sum of B row lengths over A row i; cls[i] = symbolic class of the
 // row; class_count[c] += rows per class; counts[i] = 0 for empty rows.  *heavy (zeroed
-// by the caller): the STRIPE rows.
+// by the caller): the STRIPE rows.  near (may be null): *near != 0 merges rows of
+// up to kMergeNearOps products.
 void launch_rowstats(const Operands &op, int64_t *ops, uint8_t *cls,
                      int32_t *counts, int32_t *class_count, int32_t *long_rows,
-                     int32_t *long_count, int32_t max_long, HeavyRows *heavy, cudaStream_t s);
+                     int32_t *long_count, int32_t max_long, HeavyRows *heavy,
+                     const int32_t *near, cudaStream_t s);
 void launch_rowstats_long(const Operands &op, const int32_t *long_rows,
                           const int32_t *long_count, int64_t *ops, uint8_t *cls,
                           int32_t *counts, int32_t *class_count, HeavyRows *heavy,

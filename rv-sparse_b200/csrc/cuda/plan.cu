@@ -749,7 +749,7 @@ cudaError_t reserve_shift(rvsp_cuda_plan *p, int32_t a_rows, int32_t b_rows) {
   while (tcap < 2 * (n > nb ? n : nb)) tcap <<= 1;
   p->shift_cap_pat = static_cast<int32_t>(n / kPatMinShare + 1);
   const size_t cp = static_cast<size_t>(p->shift_cap_pat);
-  cudaError_t e = p->sh_on.reserve(1);
+  cudaError_t e = p->sh_on.reserve(2);
   if (e == cudaSuccess) e = p->sh_probe.reserve(2 * size_t(shift_samples()));
   if (e == cudaSuccess) e = p->sh_bkey.reserve(nb);
   if (e == cudaSuccess) e = p->sh_rkey.reserve(n);
@@ -891,8 +891,11 @@ rvsp_status_t symbolic_impl(rvsp_cuda_plan_t p, cudaStream_t s, int32_t a_rows,
   if (!shift) cudaGetLastError();
   {
     PhaseScope ph(p, s, RVSP_PHASE_ROWSTATS);
+    if (shift)
+      launch_shift_decide(op, p->sh_probe.p, shift_bar(p), p->sh_on.p, guard, s);
     launch_rowstats(op, p->ops.p, p->cls.p, p->counts.p, misc + kSymCount,
-                    p->long_rows.p, misc + kLongCount, a_rows, heavy_rows(misc), s);
+                    p->long_rows.p, misc + kLongCount, a_rows, heavy_rows(misc),
+                    shift ? p->sh_on.p + 1 : nullptr, s);
     launch_rowstats_long(op, p->long_rows.p, misc + kLongCount, p->ops.p, p->cls.p,
                          p->counts.p, misc + kSymCount, heavy_rows(misc), p->num_sms, s);
     ph.launches = 2;
@@ -902,7 +905,6 @@ rvsp_status_t symbolic_impl(rvsp_cuda_plan_t p, cudaStream_t s, int32_t a_rows,
       // none of the analysis's passes (each a full grid that would only
       // read the flag and return).  Member rows leave the symbolic classes
       // (census recounted).
-      launch_shift_decide(op, p->sh_probe.p, shift_bar(p), p->sh_on.p, guard, s);
       e = cudaMemcpyAsync(p->h_misc, p->sh_on.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
       if (e == cudaSuccess) e = cudaStreamSynchronize(s);
       if (e != cudaSuccess) return map_cuda(e);
