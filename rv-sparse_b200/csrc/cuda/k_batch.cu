@@ -59,7 +59,10 @@ __device__ __forceinline__ void copy_values(const float *__restrict__ src, int32
   for (int64_t j = t0; j < n; j += int64_t(kCopy) * st) {
     float v[kCopy];
 #pragma unroll
-    for (int u = 0; u < kCopy; ++u) v[u] = j + int64_t(u) * st < n ? __ldg(src + j + int64_t(u) * st) : 0.0f;
+    for (int u = 0; u < kCopy; ++u) {
+      const int64_t at = j + int64_t(u) * st;
+      v[u] = at < n ? __ldg(src + at) : 0.0f;
+    }
 #pragma unroll
     for (int u = 0; u < kCopy; ++u)
       if (j + int64_t(u) * st < n) dst[j + int64_t(u) * st] = v[u];

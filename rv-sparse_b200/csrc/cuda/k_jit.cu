@@ -648,7 +648,8 @@ record_kernel(const int4 *__restrict__ tiles, int32_t nchunks,
     rec[4 + 2 * gid] = glo;
     rec[5 + 2 * gid] = ghi;
   }
-  // this lane's row: the B row starts of its A nonzeros, as offsets
+  // this lane's row: the B row starts of its A nonzeros, as offsets (nine at a
+  // time: a 27-point row takes three rounds, a 5- to 9-point one one)
   constexpr int kAhead = 9;
   for (int j0 = 0; j0 < na; j0 += kAhead) {
     int32_t r[kAhead];

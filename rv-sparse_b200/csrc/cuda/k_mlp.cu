@@ -309,8 +309,8 @@ learned_plan_kernel(Operands op, float b_mean_len, const float *__restrict__ par
 // stripe pass and need no slab slot, else they are B8192 and DENSE rows.
 __global__ void __launch_bounds__(kThreads)
 learned_heavy_kernel(int32_t n, HeavyRows *__restrict__ heavy, int32_t b_rows, int32_t b_cols,
-                     bool always, bool repeats, uint8_t *__restrict__ cls, int32_t *__restrict__ cap,
-                     int32_t *__restrict__ class_count) {
+                     bool always, bool repeats, uint8_t *__restrict__ cls,
+                     int32_t *__restrict__ cap, int32_t *__restrict__ class_count) {
   const HeavyRows h = *heavy;
   if (h.rows == 0) return;
   const bool pay = always || stripes_pay(h, b_rows, b_cols, repeats);

@@ -574,6 +574,8 @@ shift_bresolve_kernel(const int32_t *__restrict__ on, int32_t b_rows,
 // rows of one class lie side by side, so a gather of the warp reads
 // consecutive words.  (Gathering the staged columns in their order, 32
 // positions of about one row at a time, touched some ten sectors a load.)
+// Nine: a row of a 27-point stencil takes three rounds, one of a 5-, 7- or
+// 9-point stencil one.
 constexpr int kClassAhead = 9;
 template <typename P, typename F>
 __device__ __forceinline__ void visit_classes(P m, int32_t len,
@@ -991,7 +993,8 @@ void launch_shift_patterns(const int32_t *on, const Operands &op, const int32_t 
                            int32_t *class_count, int num_sms, cudaStream_t s) {
   const int32_t n = op.a_rows;
   shift_fill32_kernel<<<grid_fill(size_t(n)), kThreads, 0, s>>>(on, share, size_t(n), 0);
-  shift_share_kernel<<<grid_threads((int64_t(n) + kShareSteps - 1) / kShareSteps), kThreads, 0, s>>>(on, n, rcls, share);
+  shift_share_kernel<<<grid_threads((int64_t(n) + kShareSteps - 1) / kShareSteps), kThreads, 0,
+                       s>>>(on, n, rcls, share);
   shift_pat_kernel<<<grid_threads(n), kThreads, 0, s>>>(on, n, rcls, share, min_share, op.a_rp,
                                                         ops, pat_of, pat_canon, pat_cap, npat,
                                                         cap_pat);

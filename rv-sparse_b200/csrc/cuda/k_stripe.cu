@@ -53,9 +53,12 @@
 // Numeric-only repeat at 2^15: 2.6 -> 0.92.  Measured and left: 5 warps (one
 // reading ahead) 3.70 against 3.58, 6 to 9 blocks an SM by launch bounds 3.7
 // to 4.4 (spills), accumulators of 2048 and 8192 slots, 8 or 2 steps in flight
-// and items of 8 K to 128 K products each within 5%.  B wider than
-// kStripeMaxCols keeps the block kernels: a row's bitmap no longer fits shared
-// memory beside its prefix.
+// and items of 8 K to 128 K products each within 5%.  Which products take
+// these kernels: stripe_rule.cuh.  B wider than kStripeMaxCols (2^17) keeps the
+// block kernels: stripe_bounds_kernel is one block that holds four bitmap words
+// a thread, 2^17 columns in all, and kMaxStripes (96) is what B of that width
+// may need, 32 by shares and 64 by words.  (The count's shared memory would hold
+// more: a row's bitmap and prefix take 17 KB at 2^17, 135 KB at 2^20.)
 #include <climits>
 
 #include "device_common.cuh"
@@ -558,7 +561,8 @@ stripe_items_kernel(const int32_t *__restrict__ rows, int32_t nrows,
     }
     if (!pass) {
       // places for all of the warp's items of either kind by one atomic each
-      const int mine = n, bigs = warp_incl_scan(big ? mine : 0), rest = warp_incl_scan(big ? 0 : mine);
+      const int mine = n;
+      const int bigs = warp_incl_scan(big ? mine : 0), rest = warp_incl_scan(big ? 0 : mine);
       int base = 0, base_rest = 0;
       if (lane_id() == 31) {
         if (bigs) base = atomicAdd(&cnt[0], bigs);
@@ -1001,9 +1005,8 @@ void launch_stripe_items(const StripeShape &g, const int32_t *rows, int32_t nrow
                          int32_t *cnt, cudaStream_t s) {
   if (nrows <= 0) return;
   cudaMemsetAsync(cnt, 0, 2 * sizeof(int32_t), s);
-  stripe_items_kernel<<<(nrows + kItemRows - 1) / kItemRows, kItemRows, 0, s>>>(rows, nrows, ops, hslot, soff,
-                                                          g.ns_max, bound, share, items, cap,
-                                                          cnt);
+  stripe_items_kernel<<<(nrows + kItemRows - 1) / kItemRows, kItemRows, 0, s>>>(
+      rows, nrows, ops, hslot, soff, g.ns_max, bound, share, items, cap, cnt);
 }
 
 void launch_stripe_columns(const StripeShape &g, const int32_t *rows, int32_t nrows,

@@ -160,11 +160,11 @@ __device__ __forceinline__ void raise(int32_t *word, int32_t v) {
 }
 
 // Warp per chunk of 32 consecutive rows (see the file comment): tiles[chunk] =
-// (first row, lane mask, pattern, 0), pattern -1 without a tile; per pattern its tiles (pcount), its longest A segment
-// (pseg) and its largest union spans (spans[pattern * 32 * kJitMaxGroup +
-// j * kJitMaxGroup + g - 1]: end of the last B value minus first B value that
-// a tile's rows read for A nonzeros j .. j + g - 1).  counts: tiles,
-// leftovers, three maxima.  The builder is bound by load latency, so a lane
+// (first row, lane mask, pattern, 0), pattern -1 without a tile; per pattern its
+// tiles (pcount), its longest A segment (pseg) and its largest union spans
+// (spans[pattern * 32 * kJitMaxGroup + j * kJitMaxGroup + g - 1]: end of the
+// last B value minus first B value that a tile's rows read for A nonzeros j ..
+// j + g - 1).  counts: tiles, leftovers, three maxima.  The builder is bound by load latency, so a lane
 // takes an A nonzero: with kShifted every row of a pattern is the canonical
 // row moved, the B row of A nonzero j is row + offs[j], and as B's row
 // pointers ascend a tile's range is its first row's start and its last row's
@@ -541,8 +541,8 @@ void launch_tile_build(int32_t n, bool shifted, const int32_t *pid_of_row, const
   const int64_t grid = (steps + per_block - 1) / per_block;
   auto kern = shifted ? tile_build_kernel<true> : tile_build_kernel<false>;
   kern<<<static_cast<unsigned>(grid), kBuildWarps * 32, 0, s>>>(
-      n, static_cast<int32_t>(per_block), pid_of_row, desc, lens, offs, a_rp, a_col, b_rp, c_rp, tiles, pcount, pseg, spans,
-      lo_rows, lo_ids, counts);
+      n, static_cast<int32_t>(per_block), pid_of_row, desc, lens, offs, a_rp, a_col, b_rp, c_rp,
+      tiles, pcount, pseg, spans, lo_rows, lo_ids, counts);
 }
 
 size_t tile_smem_per_warp(int32_t stage_need, int32_t a_seg, int32_t max_out,

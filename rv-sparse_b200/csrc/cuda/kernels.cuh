@@ -414,10 +414,10 @@ void launch_tile_tab(int32_t npat, const int32_t *pat_canon, const int32_t *pste
 // Tiles of the n rows (pid_of_row: pattern of each table row, -1 for the
 // others; shifted: a pattern's rows are its canonical row moved), one per
 // chunk of 32 rows: tiles[chunk] = (first row, lane mask, pattern or -1, 0);
-// the table rows no tile takes go to lo_rows / lo_ids.  counts[0] tiles, [1] leftovers, [2..4] the stage floats, A segment
-// entries and C row the tile kernel must hold; per pattern its tiles, its
-// longest A segment and its union spans (32 * kJitMaxGroup; see k_tile.cu).
-// counts, pcount, pseg and spans are zeroed by the caller.
+// the table rows no tile takes go to lo_rows / lo_ids.  counts[0] tiles, [1]
+// leftovers, [2..4] the stage floats, A segment entries and C row the tile
+// kernel must hold; per pattern its tiles, its longest A segment and its union
+// spans (32 * kJitMaxGroup; see k_tile.cu).  counts, pcount, pseg and spans are zeroed by the caller.
 void launch_tile_build(int32_t n, bool shifted, const int32_t *pid_of_row, const int4 *desc,
                        const uint16_t *lens, const int32_t *offs, const int32_t *a_rp,
                        const int32_t *a_col, const int32_t *b_rp, const int32_t *c_rp,

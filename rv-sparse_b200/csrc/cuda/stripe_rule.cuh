@@ -23,8 +23,8 @@
 //
 // A batch is made to be repeated: 48 products of 256 to 65536 rows repeat in 1.41
 // ms with stripes and 1.56 without, though their starts alone (0.5 M rows of B)
-// cost a product more than it gains.  Where neither holds: 100 rows of 1000 entries, B rows of 8, 10,000 columns,
-// product 0.22 / 0.33, repeat 0.07 / 0.11.
+// cost a product more than it gains.  Where neither holds: 100 rows of 1000
+// entries, B rows of 8, 10,000 columns, product 0.22 / 0.33, repeat 0.07 / 0.11.
 #pragma once
 
 #include <cmath>
